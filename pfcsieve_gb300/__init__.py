@@ -123,6 +123,7 @@ def lib():
             "pfc_ctx_set_graphs": (ctypes.c_int, [vp, ctypes.c_int]),
             "pfc_ctx_set_split": (ctypes.c_int, [vp, ctypes.c_int]),
             "pfc_ctx_set_setup_tc": (ctypes.c_int, [vp, ctypes.c_int]),
+            "pfc_ctx_set_walk_tc": (ctypes.c_int, [vp, ctypes.c_int]),
             "pfc_ctx_set_walk_variant": (ctypes.c_int, [vp, ctypes.c_int, ctypes.c_int, ctypes.c_int]),
             "pfc_ctx_walk_variant": (ctypes.c_int, [vp, ctypes.c_int, ctypes.c_int, P(ctypes.c_int),
                                                     P(ctypes.c_int), P(ctypes.c_int)]),
@@ -206,6 +207,11 @@ class Context:
         below 2^64/3, programs above the word thresholds; default on)."""
         _ck(lib().pfc_ctx_set_setup_tc(self.h, int(bool(on))), "pfc_ctx_set_setup_tc")
         self.setup_tc = bool(on)
+
+    def set_walk_tc(self, on):
+        """Decide the walk's tests on the tensor cores (candidates below 2^64/3; default on, where it pays; 2:
+        wherever it can)."""
+        _ck(lib().pfc_ctx_set_walk_tc(self.h, int(on)), "pfc_ctx_set_walk_tc")
 
     def set_walk_variant(self, cls, fused, variant):
         _ck(lib().pfc_ctx_set_walk_variant(self.h, cls, int(fused), variant), "pfc_ctx_set_walk_variant")

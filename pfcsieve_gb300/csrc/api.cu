@@ -54,6 +54,7 @@ struct pfc_job {
     DArr<uint32_t> qlist;
     DArr<uint32_t> cmult;       // compositorial multipliers of the current chunk
     DArr<uint32_t> ramp;        // the combined search's factorial multipliers (n) of the chunk
+    DArr<uint8_t> words[2];     // the tensor-core walk's tables of the current chunk, per stream
     std::vector<uint32_t> h_qlist;
 
     DevClass<uint32_t> c32;
@@ -86,9 +87,9 @@ struct pfc_job {
     // the post-generation part of a segment captured as a CUDA graph, replayed
     // while the key (buffers, launch shapes, kernel choices) is unchanged
     struct GraphKey {
-        const void *p32, *p64, *hits, *cmult, *ramp, *split32, *split64;
+        const void *p32, *p64, *hits, *cmult, *ramp, *split32, *split64, *words[2];
         uint64_t cap32, cap64, hitcap;
-        int lazy, use32, use64, var[3][2], setup_tc;
+        int lazy, use32, use64, var[3][2], setup_tc, walk_tc;
         uint32_t split_n, split_start[kMaxSplit + 1];
     };
     cudaGraphExec_t graph = nullptr;
@@ -149,6 +150,8 @@ extern "C" int pfc_ctx_create(int device, uint64_t mem_budget, pfc_ctx **out) {
     c->split = !(sp && sp[0] == '0');
     const char *tc = getenv("PFCSIEVE_SETUP_TC");
     c->setup_tc = !(tc && tc[0] == '0');
+    const char *wt = getenv("PFCSIEVE_WALK_TC");
+    c->walk_tc = !(wt && wt[0] == '0');
     cudaError_t e = cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking);
     if (e == cudaSuccess) {
         cudaMemPoolProps props = {};
@@ -231,6 +234,7 @@ static int job_release(pfc_job *j) {
     j->qlist.release(c);
     j->cmult.release(c);
     j->ramp.release(c);
+    for (auto &w : j->words) w.release(c);
     j->c32.release(c);
     j->c64.release(c);
     j->hits.release(c);
@@ -636,6 +640,7 @@ static bool tc_setup32_applies(const pfc_job *j) {
 
 static int enqueue_setup(pfc_job *j) {
     pfc_ctx *c = j->ctx;
+    CK(cudaMemsetAsync(&j->stats.p->tc_err, 0, sizeof(uint32_t), c->st));   // of this segment's tensor-core kernels
     SetupArgs<WideWord> s32;
     s32.mode = j->mode;
     s32.a = j->a32.view;
@@ -660,7 +665,6 @@ static int enqueue_setup(pfc_job *j) {
             SetupArgs<WideWord> stc = s32;
             stc.a = j->tc_view[0];
             stc.b = j->tc_view[1];
-            CK(cudaMemsetAsync(&j->stats.p->tc_err, 0, sizeof(uint32_t), c->st));
             c->launches += launch_setup32_tc(j->c32.view(counts_ptr(j)), stc, ta, tb, &j->stats.p->tc_err, c->st);
         } else {
             c->launches += launch_setup32(j->c32.view(counts_ptr(j)), s32, c->st);
@@ -675,7 +679,6 @@ static int enqueue_setup(pfc_job *j) {
             SetupArgs<WideWord> stc = sw;
             stc.a = j->tc_view[0];
             stc.b = j->tc_view[1];
-            if (!tc_setup32_applies(j)) CK(cudaMemsetAsync(&j->stats.p->tc_err, 0, sizeof(uint32_t), c->st));
             c->launches += launch_setup64w_tc(j->c64.view(counts_ptr(j) + 1), stc, ta, tb, &j->stats.p->tc_err, c->st);
         } else if (j->seg_hi <= kLazyEnd) {
             c->launches += launch_setup64w(j->c64.view(counts_ptr(j) + 1), sw, c->st);
@@ -705,6 +708,104 @@ static HitBuf hitbuf(pfc_job *j) {
     return h;
 }
 
+// ------------------------------------------------------ tensor-core walks
+
+// Which walk, and when it is split.  Times of one walk launch in microseconds,
+// fitted to GB300 (factorial searches at p = 1e9 and 2^61, 2,000 to 300,000
+// candidates x 500 to 10,000 n; the fits are within 15%):
+//   tensor cores: CTAs of 128 candidates, one per SM, so whole waves of them,
+//     each with a fixed part (the candidates' planes, filling and draining the
+//     pipeline, about 1,500 steps' worth) and a part per step; a launch more
+//     for the word table;
+//   per-step kernels: a rate per candidate-step, and below about one chain per
+//     thread the latency of a step.
+// Measured, ms, tensor cores / per-step:
+//   class 32, 19,000 candidates:  500 n .029 / .026, 1,000 .031 / .038, 10,000 .088 / .169
+//            300,000 candidates: 2,000 n .354 / .286, 3,000 .454 / .423, 10,000 1.16 / 1.37
+//   class 64, 19,000 candidates:  500 n .034 / .030, 1,000 .037 / .046, 10,000 .116 / .282
+//            300,000 candidates: 1,000 n .338 / .296, 2,000 .490 / .563, 10,000 1.58 / 2.70
+struct WalkTimes {
+    double fixed, step;            // per wave of the tensor-core walk: fixed part, per step
+    double lat, rate0, rate;       // per-step kernels, per step: latency; base and part per candidate
+};
+constexpr double kTcLaunch = 12.0, kWalkLaunch = 13.0;
+constexpr WalkTimes kTimes32 = {9.7, 6.3e-3, 25.3e-3, 12e-3, 4.1e-7}, kTimes64 = {13.2, 8.8e-3, 31e-3, 20e-3, 8.2e-7};
+
+// candidates that a class's buffer is expected to hold (est_cands)
+static double held(uint64_t cap) { return (double)cap / 1.25; }
+
+// `steps` over all chains of a candidate, cut into S sub-ranges
+static double walk_tc_us(const pfc_job *j, const WalkTimes &t, uint64_t cap, double steps, uint32_t S = 1) {
+    const double waves = std::ceil(std::ceil(held(cap) / 128.0) * S / j->ctx->sms);
+    return kTcLaunch + waves * (t.fixed + t.step * steps / S);
+}
+static double walk_us(const pfc_job *j, const WalkTimes &t, uint64_t cap, double steps) {
+    return kWalkLaunch + steps * std::max(t.lat, t.rate0 + t.rate * held(cap) * 152.0 / j->ctx->sms);
+}
+
+// Longest chunk of the tensor-core walk: its tables (two of 100 to 181 bytes a
+// step in the combined search) stay within a sixteenth of the memory budget.
+static uint32_t max_words(const pfc_job *j) {
+    return (uint32_t)std::min<uint64_t>(j->ctx->budget / 16 / 384, kMaxChunk);
+}
+
+// Smallest primes the tensor-core walk takes.  Towards small p a growing part
+// of the blocks holds a hit or a multiple of p and is replayed; at 2^16 that
+// does not show yet (2,700 candidates x 20,000 n: 0.15 ms, per-step 0.62), and
+// few searches start below.
+constexpr uint64_t kTcMinP = 1u << 16;
+
+static bool walk_tc_pays(const pfc_job *j, const WalkTimes &t, uint64_t cap, uint32_t steps) {
+    const int on = j->ctx->walk_tc;
+    if (!on || j->seg_lo < kTcMinP || steps > max_words(j)) return false;
+    const double all = (double)steps * (j->mode == (PFC_FACTORIAL | PFC_COMPOSITORIAL) ? 2 : 1);
+    return on > 1 || walk_tc_us(j, t, cap, all) < walk_us(j, t, cap, all);
+}
+static bool walk_tc32_applies(const pfc_job *j, uint32_t steps) {
+    return j->use32 && j->c32.p.p && walk_tc_pays(j, kTimes32, j->c32.cap, steps);
+}
+static bool walk_tc64_applies(const pfc_job *j, uint32_t steps) {
+    return j->use64 && j->c64.p.p && j->seg_hi <= kLazyWalkEnd && walk_tc_pays(j, kTimes64, j->c64.cap, steps);
+}
+
+// the largest multiplier of steps below `hi`
+static uint32_t top_mult(const pfc_job *j, uint32_t hi) {
+    return j->mode == PFC_PRIMORIAL ? j->h_qlist[hi - 1] : hi - 1;
+}
+
+// The word tables of chunks of up to `steps` steps (allocated before any
+// capture).  Where the budget has no room left the walk takes the per-step
+// kernels, which need none.
+static void ensure_words(pfc_job *j, uint32_t steps) {
+    if (iter_end(j) == iter_begin(j) || !(walk_tc32_applies(j, steps) || walk_tc64_applies(j, steps))) return;
+    const size_t need = walk_tc_words_bytes(top_mult(j, iter_end(j)), steps);
+    for (int k = 0; k < (j->mode == (PFC_FACTORIAL | PFC_COMPOSITORIAL) ? 2 : 1); ++k)
+        if (j->words[k].n < need && j->words[k].alloc(j->ctx, need) != cudaSuccess) {
+            cudaGetLastError();
+            for (auto &w : j->words) w.release(j->ctx);
+            return;
+        }
+}
+static bool words_fit(const pfc_job *j, uint32_t top, uint32_t steps) {
+    const size_t need = walk_tc_words_bytes(top, steps);
+    return j->words[0].n >= need && (j->mode != (PFC_FACTORIAL | PFC_COMPOSITORIAL) || j->words[1].n >= need);
+}
+
+// chunk length so one launch covers about `budget` candidate-steps
+static uint32_t chunk_len(uint64_t count, double budget) {
+    double L = budget / (double)std::max<uint64_t>(count, 1);
+    L = std::max(16.0, std::min(L, 2147483648.0));
+    return ((uint32_t)L + 15u) & ~15u;
+}
+
+// steps of one walk launch: about 1.5e11 candidate-steps (class-64 steps weigh
+// 3), so that no launch runs for more than a fraction of a second, and at most
+// kMaxChunk (the multiplier tables) or what the tensor-core walk's tables hold
+static uint32_t chunk_steps(const pfc_job *j, uint64_t n32, uint64_t n64) {
+    const uint32_t L = std::min(chunk_len(n32 + 3 * n64, 1.5e11), kMaxChunk), w = std::min(L, max_words(j) & ~15u);
+    return w >= 16 && (walk_tc32_applies(j, w) || walk_tc64_applies(j, w)) ? w : L;
+}
+
 // the walks of one chunk [lo, hi) (n values, or prime indices for n#):
 // factorial over n, compositorial over its multiplier table, primorial over
 // the prime list; each for both size classes
@@ -723,13 +824,41 @@ static int enqueue_iter_range(pfc_job *j, uint32_t lo, uint32_t hi, bool split =
         sp64.s0 = j->split64.p;
         sp64.s1 = j->split64.p ? j->split64.p + (size_t)(j->split_n - 1) * j->c64.cap : nullptr;
     }
+    ensure_words(j, hi - lo);
+    const bool words = words_fit(j, top_mult(j, hi), hi - lo);
+    const bool tc32 = words && walk_tc32_applies(j, hi - lo), tc64 = words && walk_tc64_applies(j, hi - lo);
     auto walk = [&](const WalkArgs &w) {
         const int fused = w.mult2 != nullptr;
         const bool lazy = j->seg_hi <= kLazyWalkEnd;
-        if (j->use32)
+        if (tc32 || tc64) {
+            const uint32_t top = top_mult(j, hi);
+            WalkTcArgs t{};
+            t.nstreams = fused ? 2 : 1;
+            t.lo = lo;
+            t.hi = hi;
+            t.base = w.base;
+            // the factorial's multipliers are n itself (the fused walk's
+            // table of them is for the per-step kernels)
+            t.mult[0] = fused ? nullptr : w.mult;
+            t.mult[1] = w.mult2;
+            t.type[0] = w.type;
+            t.type[1] = w.type2;
+            t.second[1] = 1;
+            for (uint32_t s = 0; s < t.nstreams; ++s) {
+                t.words[s] = j->words[s].p;
+                c->launches += launch_walk_words(t.mult[s], t.base, lo, hi, top, j->words[s].p, c->st);
+            }
+            if (tc32)
+                c->launches += launch_walk_tc32(j->c32.view(counts_ptr(j)), t, top, h, split ? &sp32 : nullptr,
+                                                &j->stats.p->tc_err, c->st);
+            if (tc64)
+                c->launches += launch_walk_tc64(j->c64.view(counts_ptr(j) + 1), t, top, h, split ? &sp64 : nullptr,
+                                                &j->stats.p->tc_err, c->st);
+        }
+        if (j->use32 && !tc32)
             c->launches += launch_walk32(j->c32.view(counts_ptr(j)), w, h, c->st, c->walk_var[0][fused],
                                          split ? &sp32 : nullptr);
-        if (j->use64)
+        if (j->use64 && !tc64)
             c->launches += launch_walk64(j->c64.view(counts_ptr(j) + 1), w, h, c->st, lazy,
                                          c->walk_var[lazy ? 1 : 2][fused], split ? &sp64 : nullptr);
     };
@@ -750,10 +879,10 @@ static int enqueue_iter_range(pfc_job *j, uint32_t lo, uint32_t hi, bool split =
     }
     if (j->mode & PFC_COMPOSITORIAL) {
         // multiplier tables of the chunk: compositorial (n or 1) and, for the
-        // fused walk, factorial (n; the plain factorial walk forms n itself,
-        // shared by its two candidates, and gains nothing from a table)
+        // per-step fused walk, factorial (n; the plain factorial walk forms n
+        // itself, shared by its two candidates, and gains nothing from a table)
         const size_t need = ((size_t)(hi - lo) + 15) & ~(size_t)15;
-        const bool comp = true, fact = (j->mode & PFC_FACTORIAL) != 0;
+        const bool comp = true, fact = (j->mode & PFC_FACTORIAL) && ((j->use32 && !tc32) || (j->use64 && !tc64));
         if (comp && j->cmult.n < need) CK(j->cmult.alloc(c, std::max<size_t>(need, 4096)));
         if (fact && j->ramp.n < need) CK(j->ramp.alloc(c, std::max<size_t>(need, 4096)));
         c->launches += launch_cmult(comp ? j->cmult.p : nullptr, fact ? j->ramp.p : nullptr, j->primebits.p,
@@ -777,13 +906,6 @@ static int enqueue_iter_range(pfc_job *j, uint32_t lo, uint32_t hi, bool split =
     return PFC_OK;
 }
 
-// chunk length so one launch covers about `budget` candidate-steps
-static uint32_t chunk_len(uint64_t count, double budget) {
-    double L = budget / (double)std::max<uint64_t>(count, 1);
-    L = std::max(16.0, std::min(L, 2147483648.0));
-    return ((uint32_t)L + 15u) & ~15u;
-}
-
 // ------------------------------------------------------------ split walks
 //
 // A segment with few candidates leaves most of the GPU idle in its walk: each
@@ -795,11 +917,13 @@ static uint32_t chunk_len(uint64_t count, double budget) {
 // primorial of the primes below the boundary's prime), evaluated by the setup
 // kernel, and one launch walks every (candidate, sub-range) pair.  S fills
 // about two waves of resident CTAs; boundaries whose programs would cost more
-// than a sixth of the walk (large nmin) disable the split.  Results are the
+// than a sixth of the walk (large nmin) disable the split.  The tensor-core
+// walk takes the S of the least modelled time.  Results are the
 // same as the plain walk's: every n is tested once, hits carry their own n,
 // the last sub-range leaves the final residue and nnext counts every step.
 
 constexpr uint32_t kMinSplitLen = 2048;   // shortest sub-range worth a setup program
+constexpr uint32_t kMinSplitLenTc = 1024;   // (the tensor-core walk's: bounds the plans compared)
 
 template <class W>
 static uint64_t prog_cost(const HostProg<W> &a, const HostProg<W> &b) {
@@ -819,16 +943,50 @@ static int split_prepare(pfc_job *j) {
     const uint32_t lo = iter_begin(j), hi = iter_end(j), len = hi - lo;
     const uint64_t n32 = (j->use32 && j->c32.p.p) ? j->c32.cap : 0;
     const uint64_t n64 = (j->use64 && j->c64.p.p) ? j->c64.cap : 0;
-    const uint32_t L = std::min(chunk_len(n32 + 3 * n64, 1.5e11), kMaxChunk);
+    const uint32_t L = chunk_steps(j, n32, n64);
     if (!c->split || len > L || n32 + n64 == 0) return PFC_OK;
     const bool fused = j->mode == (PFC_FACTORIAL | PFC_COMPOSITORIAL);
-    const uint64_t chains = (n32 + n64) * (fused ? 2 : 1);
-    const uint64_t target = (uint64_t)c->sms * 3 * 256 * 2 * 2;   // two waves of CTAs, two chains a thread
-    uint32_t S = (uint32_t)std::min<uint64_t>({(uint64_t)kMaxSplit, target / chains, len / kMinSplitLen});
+    const uint64_t walk = (uint64_t)len * (fused ? 2 : 1);
+    const bool tc32 = walk_tc32_applies(j, len), tc64 = walk_tc64_applies(j, len), tc = tc32 || tc64;
+    // The tensor-core walk's time with S sub-ranges whose boundaries' programs
+    // cost `sum` and at most `most` steps: their launch takes about 18 us, a
+    // step of theirs about as long as one of the walk's, over a wave of
+    // candidates (1.7 times as long in class 64, whose words cost more).
+    auto tc_us = [&](uint32_t S, double sum, double most) {
+        double us = S > 1 ? 18.0 : 0.0;
+        const double wave = 128.0 * c->sms;
+        if (tc32) us += walk_tc_us(j, kTimes32, n32, (double)walk, S) + kTimes32.step * std::max(most, sum * held(n32) / wave);
+        if (tc64) us += walk_tc_us(j, kTimes64, n64, (double)walk, S) + kTimes64.step * std::max(most, sum * 1.7 * held(n64) / wave);
+        return us;
+    };
+    auto value_at = [&](uint32_t k) { return j->mode == PFC_PRIMORIAL ? j->h_qlist[k] : k; };
+    uint32_t S;
+    if (tc) {
+        // by the model, with a program for b estimated at the 2 b bits of b!'s
+        // odd parts in 896-bit words of 15 steps
+        S = 1;
+        double best = tc_us(1, 0, 0);
+        for (uint32_t s = 2; s <= (uint32_t)kMaxSplit && len / s >= kMinSplitLenTc; ++s) {
+            double sum = 0, most = 0;
+            for (uint32_t k = 1; k < s; ++k) {
+                const double cost = value_at(lo + (uint32_t)((uint64_t)len * k / s)) / 30.0;
+                sum += cost;
+                most = std::max(most, cost);
+            }
+            const double us = tc_us(s, sum, most);
+            if (us < best) {
+                best = us;
+                S = s;
+            }
+        }
+    } else {
+        const uint64_t chains = (n32 + n64) * (fused ? 2 : 1);
+        const uint64_t target = (uint64_t)c->sms * 3 * 256 * 2 * 2;   // two waves of CTAs, two chains a thread
+        S = (uint32_t)std::min<uint64_t>({(uint64_t)kMaxSplit, target / chains, len / kMinSplitLen});
+    }
     if (S < 2) return PFC_OK;
     const bool lazy = j->seg_hi <= kLazyEnd;
     const bool wide = n32 > 0 || (n64 > 0 && lazy), narrow = n64 > 0 && !lazy;
-    const uint64_t walk = (uint64_t)len * (fused ? 2 : 1);
 
     // a lower bound on a boundary's program cost, before anything is built:
     // every program multiplies at least the primes up to (b-1)/2, whose
@@ -840,14 +998,15 @@ static int split_prepare(pfc_job *j) {
     };
     for (; S >= 2; --S) {
         uint32_t start[kMaxSplit + 1];
-        const uint32_t step = ((len / S) + 15u) & ~15u;
+        const uint32_t align = tc ? walk_tc_align(top_mult(j, hi)) : 16u;
+        const uint32_t step = (len / S + align - 1) / align * align;
         for (uint32_t k = 0; k < S; ++k) start[k] = lo + k * step;
         start[S] = hi;
         if (start[S - 1] >= hi) continue;
         double floor_cost = 0;
         for (uint32_t k = 1; k < S; ++k)
-            floor_cost += cost_floor(j->mode == PFC_PRIMORIAL ? j->h_qlist[start[k]] : start[k]);
-        if (floor_cost * 6 > (double)walk) continue;
+            floor_cost += cost_floor(value_at(start[k]));
+        if (!tc && floor_cost * 6 > (double)walk) continue;
         const bool same = j->split_wide == wide && j->split_narrow == narrow &&
                           j->split_wa.size() + j->split_na.size() > 0 &&
                           std::max(j->split_wa.size(), j->split_na.size()) == S - 1 &&
@@ -856,14 +1015,17 @@ static int split_prepare(pfc_job *j) {
             // the value before each boundary's first multiplier; the
             // boundaries' programs come from the context's cache
             std::vector<std::shared_ptr<const ProgSet>> ps(S);
-            uint64_t cost = 0;
+            uint64_t cost = 0, most = 0;
             for (uint32_t k = 1; k < S; ++k) {
-                const uint32_t startN = (j->mode == PFC_PRIMORIAL ? j->h_qlist[start[k]] : start[k]) - 1;
+                const uint32_t startN = value_at(start[k]) - 1;
                 ps[k] = ctx_progs(c, j->mode, startN, wide, narrow);
                 if (!ps[k]) return PFC_ERR_ARG;
-                cost += wide ? prog_cost(ps[k]->wa, ps[k]->wb) : prog_cost(ps[k]->na, ps[k]->nb);
+                const uint64_t one = wide ? prog_cost(ps[k]->wa, ps[k]->wb) : prog_cost(ps[k]->na, ps[k]->nb);
+                cost += one;
+                most = std::max(most, one);
             }
-            if (cost * 6 > walk) continue;   // boundaries too dear: fewer sub-ranges or none
+            // boundaries too dear: fewer sub-ranges or none
+            if (tc ? tc_us(S, (double)cost, (double)most) >= tc_us(1, 0, 0) : cost * 6 > walk) continue;
             for (auto &pg : j->split_wa) pg.release(c);
             for (auto &pg : j->split_wb) pg.release(c);
             for (auto &pg : j->split_na) pg.release(c);
@@ -937,7 +1099,7 @@ static int enqueue_iter_chunked(pfc_job *j, uint32_t lo, uint32_t hi, uint64_t n
         if (rc) return rc;
         return enqueue_iter_range(j, lo, hi, true);
     }
-    const uint32_t L = std::min(chunk_len(n32 + 3 * n64, 1.5e11), kMaxChunk);
+    const uint32_t L = chunk_steps(j, n32, n64);
     while (lo < hi) {
         const uint32_t e = (uint32_t)std::min<uint64_t>((uint64_t)lo + L, hi);
         int rc = enqueue_iter_range(j, lo, e);
@@ -1061,7 +1223,7 @@ static int segment_body_graph(pfc_job *j) {
     // a buffer the body would otherwise allocate while it is being captured
     if (j->mode & PFC_COMPOSITORIAL) {
         const uint64_t n32 = j->c32.p.p ? j->c32.cap : 0, n64 = j->c64.p.p ? j->c64.cap : 0;
-        const size_t L = std::min(chunk_len(n32 + 3 * n64, 1.5e11), kMaxChunk);
+        const size_t L = chunk_steps(j, n32, n64);
         const size_t need = (((size_t)std::min<uint64_t>(L, iter_end(j) - iter_begin(j))) + 15) & ~(size_t)15;
         if ((j->mode & PFC_COMPOSITORIAL) && j->cmult.n < need) CK(j->cmult.alloc(c, std::max<size_t>(need, 4096)));
         if ((j->mode & PFC_FACTORIAL) && j->ramp.n < need) CK(j->ramp.alloc(c, std::max<size_t>(need, 4096)));
@@ -1069,6 +1231,11 @@ static int segment_body_graph(pfc_job *j) {
     if (tc_setup_applies(j) || tc_setup32_applies(j)) {
         const int rc = tc_prepare(j);
         if (rc) return rc;
+    }
+    {
+        const uint64_t n32 = j->c32.p.p ? j->c32.cap : 0, n64 = j->c64.p.p ? j->c64.cap : 0;
+        const uint32_t L = chunk_steps(j, n32, n64);
+        ensure_words(j, std::min(L, iter_end(j) - iter_begin(j)));
     }
     pfc_job::GraphKey k{};
     k.p32 = j->c32.p.p;
@@ -1087,6 +1254,8 @@ static int segment_body_graph(pfc_job *j) {
     k.split64 = j->split64.p;
     k.split_n = j->split_n;
     k.setup_tc = c->setup_tc;
+    k.walk_tc = j->seg_lo < kTcMinP ? 0 : c->walk_tc;
+    for (int i = 0; i < 2; ++i) k.words[i] = j->words[i].p;
     if (j->split_n > 1) memcpy(k.split_start, j->split_start, sizeof(k.split_start));
     if (!j->graph || memcmp(&k, &j->gkey, sizeof(k)) != 0) {
         if (j->graph) cudaGraphExecDestroy(j->graph);
@@ -1445,6 +1614,8 @@ static int tune_one(pfc_ctx *c, int cls, int fused, char *report, size_t cap, si
     rc = pfc_gen_candidates(j, lo, hi);
     if (!rc) rc = pfc_setup(j);
     const int saved = c->walk_var[cls][fused];
+    const int walk_tc = c->walk_tc;
+    c->walk_tc = 0;   // the variants are the per-step kernels'
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (!rc && (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess)) rc = PFC_ERR_CUDA;
     uint32_t n = nmin;
@@ -1478,6 +1649,7 @@ static int tune_one(pfc_ctx *c, int cls, int fused, char *report, size_t cap, si
         }
     }
     c->walk_var[cls][fused] = pick;
+    c->walk_tc = walk_tc;
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     pfc_job_destroy(j);
@@ -1506,6 +1678,12 @@ extern "C" int pfc_ctx_set_graphs(pfc_ctx *c, int on) {
 extern "C" int pfc_ctx_set_split(pfc_ctx *c, int on) {
     if (!c) return PFC_ERR_ARG;
     c->split = on != 0;
+    return PFC_OK;
+}
+
+extern "C" int pfc_ctx_set_walk_tc(pfc_ctx *c, int on) {
+    if (!c) return PFC_ERR_ARG;
+    c->walk_tc = on < 0 ? 0 : on > 2 ? 2 : on;
     return PFC_OK;
 }
 

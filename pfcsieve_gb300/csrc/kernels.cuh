@@ -184,6 +184,28 @@ int launch_walk32(const ClassBuf<uint32_t> &c, const WalkArgs &a, const HitBuf &
 // lazy: every candidate is below 2^64/3 (the walk then takes lazy one-word steps)
 int launch_walk64(const ClassBuf<uint64_t> &c, const WalkArgs &a, const HitBuf &h, cudaStream_t st, bool lazy,
                   int variant, const SplitArgs<uint64_t> *sp = nullptr);
+// The walk with its tests on the tensor cores (walk_tc.cu): one or two streams
+// (the two chains of the combined search) of steps [lo, hi) over every
+// candidate, from the tables of words that launch_walk_words laid out for them
+// (`top`: the largest multiplier of the tables, which sets the words' shape).
+struct WalkTcArgs {
+    const unsigned char *words[2];
+    const uint32_t *mult[2];   // multipliers of step k at mult[k - base], or k itself (null)
+    int32_t type[2];           // factor type of a stream's hits
+    uint32_t second[2];        // 1: the stream walks the residue s1
+    uint32_t nstreams;
+    uint32_t lo, hi, base;
+    uint32_t nb, shift11, shift22;   // set by the launch: steps per block, 2^11, 2^22
+};
+uint32_t walk_tc_align(uint32_t top);   // sub-ranges of a split walk start at multiples of this from lo
+size_t walk_tc_words_bytes(uint32_t top, uint32_t steps);
+int launch_walk_words(const uint32_t *mult, uint32_t base, uint32_t lo, uint32_t hi, uint32_t top, unsigned char *out,
+                      cudaStream_t st);
+// a wait that gives up sets bit 2 of *err
+int launch_walk_tc32(const ClassBuf<uint32_t> &c, const WalkTcArgs &a, uint32_t top, const HitBuf &h,
+                     const SplitArgs<uint32_t> *sp, uint32_t *err, cudaStream_t st);
+int launch_walk_tc64(const ClassBuf<uint64_t> &c, const WalkTcArgs &a, uint32_t top, const HitBuf &h,
+                     const SplitArgs<uint64_t> *sp, uint32_t *err, cudaStream_t st);
 // size class 0: p < 2^31, 1: lazy class 64 (p < 2^64/3), 2: other class 64
 int walk_variant_count(int cls, bool fused);
 int walk_variant_shape(int cls, bool fused, int variant, int *nc, int *b);

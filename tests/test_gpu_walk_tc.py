@@ -1,0 +1,73 @@
+"""The tensor-core walk (csrc/walk_tc.cu) against the oracle and the per-step kernels, at the edges of its
+tiles: candidate counts around a CTA's 128, n lengths around a block, a tile and a supertile, the word
+shapes, both size classes, every mode, several launches of one walk, split walks.  Integers: equal, no
+tolerance."""
+import numpy as np
+import pytest
+
+pfc = pytest.importorskip("pfcsieve_gb300")
+
+from oracle import oracle as o  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+def segment(mode, nmin, nmax, lo, hi, on, cuts=(), split=False):
+    with pfc.Context(0) as ctx:
+        ctx.set_walk_tc(2 * on)   # (2: whatever the size)
+        ctx.set_split(split)
+        with pfc.Job(ctx, mode, nmin, nmax, lo, hi) as job:
+            job.gen(lo, hi)
+            job.setup()
+            at = [nmin, *cuts, nmax]
+            for a, b in zip(at, at[1:]):
+                job.iterate(a, b)
+            job.check()
+            p, s0, s1 = job.segment_state()
+            order = np.argsort(p)
+            return p[order], s0[order], s1[order], job.totals(), o.sort_factors(job.drain_hits())
+
+
+def same(a, b):
+    for x, y in zip(a, b):
+        assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("mode", [1, 2, 4, 5])
+@pytest.mark.parametrize("p", [2**16, 2**31 - 20000, 2**62, 2**64 // 3 - 100000])
+def test_walk_matches_the_oracle(mode, p):
+    nmin, nmax = 101, 9000 + p % 7
+    hi = p + 50003
+    got = segment(mode, nmin, nmax, p, hi, True)
+    cands = o.candidates(p, hi)
+    assert np.array_equal(got[0], cands)
+    hits, _, terms = o.sieve(mode, nmin, nmax, cands, want_terms=True)
+    assert np.array_equal(got[1], terms[:, 0])
+    if mode == 5:
+        assert np.array_equal(got[2], terms[:, 2])
+    assert np.array_equal(got[4], hits)
+
+
+@pytest.mark.parametrize("nmin,length", [(n, k) for n in (201000, 202001, 12899000)
+                                         for k in (1, 15, 17, 64, 255, 257, 1025, 4097)] + [(2**31 - 6000, 2049)])
+def test_lengths_and_word_shapes(nmin, length):
+    for p in (1500000000, 2**45):
+        args = (1, nmin, nmin + length, p, p + 200000)
+        same(segment(*args, True), segment(*args, False))
+
+
+@pytest.mark.parametrize("mode,p,span,cuts,split", [
+    (5, 10**9, 40, (), False), (2, 2**40, 2700, (), False), (5, 10**9, 2800, (), True), (1, 2**40, 60000, (), True),
+    (5, 10**8, 150000, (517, 1541, 9000, 20001), False), (2, 2**50, 150000, (517, 1541, 9000, 20001), False),
+    (4, 2**31 - 70000, 150000, (), True), (5, 2**31 - 70000, 150000, (), True),
+])
+def test_candidate_counts_and_ranges(mode, p, span, cuts, split):
+    args = (mode, 500, 30000, p, p + span)
+    same(segment(*args, True, cuts=cuts, split=split), segment(*args, False))
+
+
+@pytest.mark.parametrize("mode", [1, 2, 4, 5])
+def test_many_hits(mode):
+    """p not far above n: hits in every block, and candidates that n passes (their residue is 0 from there)."""
+    args = (mode, 101, 90000, 2**16, 160000)
+    same(segment(*args, True), segment(*args, False))
