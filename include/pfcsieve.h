@@ -123,14 +123,14 @@ int pfc_ctx_set_split(pfc_ctx *ctx, int on);
  * the integer-pipe fold.  Results are identical. */
 int pfc_ctx_set_setup_tc(pfc_ctx *ctx, int on);
 
-/* Tensor-core walk (default on): candidates below 2^64/3 walk the n range in
- * blocks of 16 steps whose tests are decided from the block's integer products
- * in one exact contraction on the tensor cores, shared by all candidates; the
- * few that pass are replayed step by step.  Short n ranges, segments that
- * start below 2^16, and every walk when off (`on` = 0, or PFCSIEVE_WALK_TC=0
- * in the environment when the context is created), take the per-step kernels;
- * `on` = 2 takes short ranges too.  Results are identical.  No counterpart in the reference, which multiplies
- * each residue by each n (kernels/iterate.cl:59-198). */
+/* Tensor-core walk (default on): candidates walk the n range in blocks of 16
+ * steps whose tests are decided from the block's integer products in one exact
+ * contraction on the tensor cores, shared by all candidates; the few that pass
+ * are replayed step by step.  Short n ranges, segments that start below 2^16,
+ * and every walk when off (`on` = 0, or PFCSIEVE_WALK_TC=0 in the environment
+ * when the context is created), take the per-step kernels; `on` = 2 takes
+ * short ranges too.  Results are identical.  No counterpart in the reference,
+ * which multiplies each residue by each n (kernels/iterate.cl:59-198). */
 int pfc_ctx_set_walk_tc(pfc_ctx *ctx, int on);
 
 /* Number of kernels this context has launched so far. */

@@ -209,8 +209,7 @@ class Context:
         self.setup_tc = bool(on)
 
     def set_walk_tc(self, on):
-        """Decide the walk's tests on the tensor cores (candidates below 2^64/3; default on, where it pays; 2:
-        wherever it can)."""
+        """Decide the walk's tests on the tensor cores (default on, where it pays; 2: wherever it can)."""
         _ck(lib().pfc_ctx_set_walk_tc(self.h, int(on)), "pfc_ctx_set_walk_tc")
 
     def set_walk_variant(self, cls, fused, variant):

@@ -711,8 +711,8 @@ static HitBuf hitbuf(pfc_job *j) {
 // ------------------------------------------------------ tensor-core walks
 
 // Which walk, and when it is split.  Times of one walk launch in microseconds,
-// fitted to GB300 (factorial searches at p = 1e9 and 2^61, 2,000 to 300,000
-// candidates x 500 to 10,000 n; the fits are within 15%):
+// fitted to GB300 (factorial searches at p = 1e9, 2^61 and 3 2^62, 2,000 to
+// 300,000 candidates x 200 to 10,000 n; the fits are within 15%):
 //   tensor cores: CTAs of 128 candidates, one per SM, so whole waves of them,
 //     each with a fixed part (the candidates' planes, filling and draining the
 //     pipeline, about 1,500 steps' worth) and a part per step; a launch more
@@ -724,12 +724,15 @@ static HitBuf hitbuf(pfc_job *j) {
 //            300,000 candidates: 2,000 n .354 / .286, 3,000 .454 / .423, 10,000 1.16 / 1.37
 //   class 64, 19,000 candidates:  500 n .034 / .030, 1,000 .037 / .046, 10,000 .116 / .282
 //            300,000 candidates: 1,000 n .338 / .296, 2,000 .490 / .563, 10,000 1.58 / 2.70
+//   from 2^64/3, 19,000 candidates: 200 n .031 / .025, 500 .033 / .042, 10,000 .125 / .481
+//            300,000 candidates: 500 n .287 / .287, 1,000 .363 / .547, 10,000 1.75 / 5.28
 struct WalkTimes {
     double fixed, step;            // per wave of the tensor-core walk: fixed part, per step
     double lat, rate0, rate;       // per-step kernels, per step: latency; base and part per candidate
 };
 constexpr double kTcLaunch = 12.0, kWalkLaunch = 13.0;
-constexpr WalkTimes kTimes32 = {9.7, 6.3e-3, 25.3e-3, 12e-3, 4.1e-7}, kTimes64 = {13.2, 8.8e-3, 31e-3, 20e-3, 8.2e-7};
+constexpr WalkTimes kTimes32 = {9.7, 6.3e-3, 25.3e-3, 12e-3, 4.1e-7}, kTimes64 = {13.2, 8.8e-3, 31e-3, 20e-3, 8.2e-7},
+                    kTimesTop = {12.3, 9.6e-3, 58e-3, 8e-3, 1.73e-6};   // (class 64 from 2^64/3)
 
 // candidates that a class's buffer is expected to hold (est_cands)
 static double held(uint64_t cap) { return (double)cap / 1.25; }
@@ -765,7 +768,9 @@ static bool walk_tc32_applies(const pfc_job *j, uint32_t steps) {
     return j->use32 && j->c32.p.p && walk_tc_pays(j, kTimes32, j->c32.cap, steps);
 }
 static bool walk_tc64_applies(const pfc_job *j, uint32_t steps) {
-    return j->use64 && j->c64.p.p && j->seg_hi <= kLazyWalkEnd && walk_tc_pays(j, kTimes64, j->c64.cap, steps);
+    if (!j->use64 || !j->c64.p.p) return false;
+    if (j->seg_hi <= kLazyWalkEnd) return walk_tc_pays(j, kTimes64, j->c64.cap, steps);
+    return j->seg_lo >> 62 && walk_tc_pays(j, kTimesTop, j->c64.cap, steps);   // (its A takes the residue's top word)
 }
 
 // the largest multiplier of steps below `hi`
@@ -853,7 +858,7 @@ static int enqueue_iter_range(pfc_job *j, uint32_t lo, uint32_t hi, bool split =
                                                 &j->stats.p->tc_err, c->st);
             if (tc64)
                 c->launches += launch_walk_tc64(j->c64.view(counts_ptr(j) + 1), t, top, h, split ? &sp64 : nullptr,
-                                                &j->stats.p->tc_err, c->st);
+                                                &j->stats.p->tc_err, c->st, lazy);
         }
         if (j->use32 && !tc32)
             c->launches += launch_walk32(j->c32.view(counts_ptr(j)), w, h, c->st, c->walk_var[0][fused],
@@ -946,6 +951,8 @@ static int split_prepare(pfc_job *j) {
     const uint32_t L = chunk_steps(j, n32, n64);
     if (!c->split || len > L || n32 + n64 == 0) return PFC_OK;
     const bool fused = j->mode == (PFC_FACTORIAL | PFC_COMPOSITORIAL);
+    const bool lazy = j->seg_hi <= kLazyEnd;
+    const bool wide = n32 > 0 || (n64 > 0 && lazy), narrow = n64 > 0 && !lazy;
     const uint64_t walk = (uint64_t)len * (fused ? 2 : 1);
     const bool tc32 = walk_tc32_applies(j, len), tc64 = walk_tc64_applies(j, len), tc = tc32 || tc64;
     // The tensor-core walk's time with S sub-ranges whose boundaries' programs
@@ -955,21 +962,28 @@ static int split_prepare(pfc_job *j) {
     auto tc_us = [&](uint32_t S, double sum, double most) {
         double us = S > 1 ? 18.0 : 0.0;
         const double wave = 128.0 * c->sms;
+        const WalkTimes &t64 = j->seg_hi <= kLazyWalkEnd ? kTimes64 : kTimesTop;
         if (tc32) us += walk_tc_us(j, kTimes32, n32, (double)walk, S) + kTimes32.step * std::max(most, sum * held(n32) / wave);
-        if (tc64) us += walk_tc_us(j, kTimes64, n64, (double)walk, S) + kTimes64.step * std::max(most, sum * 1.7 * held(n64) / wave);
+        if (tc64) us += walk_tc_us(j, t64, n64, (double)walk, S) + t64.step * std::max(most, sum * 1.7 * held(n64) / wave);
         return us;
     };
     auto value_at = [&](uint32_t k) { return j->mode == PFC_PRIMORIAL ? j->h_qlist[k] : k; };
-    uint32_t S;
+    const uint64_t chains = (n32 + n64) * (fused ? 2 : 1);
+    const uint64_t target = (uint64_t)c->sms * 3 * 256 * 2 * 2;   // two waves of CTAs, two chains a thread
+    uint32_t S = (uint32_t)std::min<uint64_t>({(uint64_t)kMaxSplit, target / chains, len / kMinSplitLen});
+    // From 2^64/3 up to a wave of candidates splits wherever the per-step walk
+    // would (13,500 candidates x 19,900 n: 0.27 ms split, 0.22 plain, since
+    // the boundaries' programs there take 64-bit words).
+    const bool keep = tc && narrow && S > 1 && held(n64) <= 128.0 * c->sms;
     if (tc) {
         // by the model, with a program for b estimated at the 2 b bits of b!'s
-        // odd parts in 896-bit words of 15 steps
+        // odd parts in 896-bit words of 15 steps, or 64-bit words of 2
         S = 1;
-        double best = tc_us(1, 0, 0);
+        double best = keep ? 1e300 : tc_us(1, 0, 0);
         for (uint32_t s = 2; s <= (uint32_t)kMaxSplit && len / s >= kMinSplitLenTc; ++s) {
             double sum = 0, most = 0;
             for (uint32_t k = 1; k < s; ++k) {
-                const double cost = value_at(lo + (uint32_t)((uint64_t)len * k / s)) / 30.0;
+                const double cost = value_at(lo + (uint32_t)((uint64_t)len * k / s)) / (narrow && !wide ? 16.0 : 30.0);
                 sum += cost;
                 most = std::max(most, cost);
             }
@@ -979,14 +993,8 @@ static int split_prepare(pfc_job *j) {
                 S = s;
             }
         }
-    } else {
-        const uint64_t chains = (n32 + n64) * (fused ? 2 : 1);
-        const uint64_t target = (uint64_t)c->sms * 3 * 256 * 2 * 2;   // two waves of CTAs, two chains a thread
-        S = (uint32_t)std::min<uint64_t>({(uint64_t)kMaxSplit, target / chains, len / kMinSplitLen});
     }
     if (S < 2) return PFC_OK;
-    const bool lazy = j->seg_hi <= kLazyEnd;
-    const bool wide = n32 > 0 || (n64 > 0 && lazy), narrow = n64 > 0 && !lazy;
 
     // a lower bound on a boundary's program cost, before anything is built:
     // every program multiplies at least the primes up to (b-1)/2, whose
@@ -1025,7 +1033,7 @@ static int split_prepare(pfc_job *j) {
                 most = std::max(most, one);
             }
             // boundaries too dear: fewer sub-ranges or none
-            if (tc ? tc_us(S, (double)cost, (double)most) >= tc_us(1, 0, 0) : cost * 6 > walk) continue;
+            if (tc && !keep ? tc_us(S, (double)cost, (double)most) >= tc_us(1, 0, 0) : cost * 6 > walk) continue;
             for (auto &pg : j->split_wa) pg.release(c);
             for (auto &pg : j->split_wb) pg.release(c);
             for (auto &pg : j->split_na) pg.release(c);
@@ -1254,7 +1262,7 @@ static int segment_body_graph(pfc_job *j) {
     k.split64 = j->split64.p;
     k.split_n = j->split_n;
     k.setup_tc = c->setup_tc;
-    k.walk_tc = j->seg_lo < kTcMinP ? 0 : c->walk_tc;
+    k.walk_tc = 2 * c->walk_tc + (j->seg_lo >= kTcMinP) + 8 * (int)(j->seg_lo >> 62);
     for (int i = 0; i < 2; ++i) k.words[i] = j->words[i].p;
     if (j->split_n > 1) memcpy(k.split_start, j->split_start, sizeof(k.split_start));
     if (!j->graph || memcmp(&k, &j->gkey, sizeof(k)) != 0) {

@@ -34,7 +34,7 @@ struct pfc_ctx {
     int walk_var[3][2] = {{0, 0}, {0, 0}, {0, 0}};   // walk variant per size class and kind (fused)
     bool graphs = true;   // pfc_segment replays each job's segment body as a CUDA graph
     bool split = true;    // small candidate sets walk their n range in sub-ranges (split walks)
-    int walk_tc = 1;      // walks below 2^64/3 test their steps on the tensor cores (1: where that pays, 2: wherever it can)
+    int walk_tc = 1;      // walks test their steps on the tensor cores (1: where that pays, 2: wherever it can)
     bool setup_tc = true; // lazy class-64 setup folds its table words on the tensor cores
     // prime flags of [0, vbits_top] kept for pfc_verify_factors_device (one
     // bit per integer), rebuilt only when a call needs a larger range

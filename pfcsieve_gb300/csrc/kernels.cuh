@@ -205,7 +205,7 @@ int launch_walk_words(const uint32_t *mult, uint32_t base, uint32_t lo, uint32_t
 int launch_walk_tc32(const ClassBuf<uint32_t> &c, const WalkTcArgs &a, uint32_t top, const HitBuf &h,
                      const SplitArgs<uint32_t> *sp, uint32_t *err, cudaStream_t st);
 int launch_walk_tc64(const ClassBuf<uint64_t> &c, const WalkTcArgs &a, uint32_t top, const HitBuf &h,
-                     const SplitArgs<uint64_t> *sp, uint32_t *err, cudaStream_t st);
+                     const SplitArgs<uint64_t> *sp, uint32_t *err, cudaStream_t st, bool lazy);
 // size class 0: p < 2^31, 1: lazy class 64 (p < 2^64/3), 2: other class 64
 int walk_variant_count(int cls, bool fused);
 int walk_variant_shape(int cls, bool fused, int variant, int *nc, int *b);

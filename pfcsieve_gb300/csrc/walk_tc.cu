@@ -1,5 +1,6 @@
 // walk_tc.cu -- the walk over n with its per-step test on the tensor cores
-// (tcgen05), for class 32 and class 64 below 2^64/3.
+// (tcgen05), for the three size classes (class 32; class 64 below 2^64/3 and
+// from there).
 //
 // walk.cuh multiplies every candidate's residue by every n.  Here the n range
 // is cut into blocks of nb multipliers (16, or 12 for n that do not fit the
@@ -59,7 +60,8 @@
 // and packed minima).  Cycles per 32 candidates and step on an SM's quarter,
 // 4.8e5 (class 32) and 1.2e5 candidates, per-step kernels to this one: class
 // 32 17.7 to 13.4 (words of 47 digits), 19.6 to 14.4 (63); class 64 35.9 to
-// 18.2 (63), 38.3 to 19.3 (47).  At that rate 68% of the issue slots are used,
+// 18.2 (63), 38.3 to 19.3 (47), from 2^64/3 (3.0e5 candidates) 69.5 to 20.3.  At
+// that rate 68% of the issue slots are used,
 // the ALU 58% of the time, the tensor cores 30 to 36%.  A CTA's fixed part,
 // about 1,500 steps long, is planes (7 to 14 thousand cycles), the first
 // products' way through the roles (5 thousand), and the last replays.
@@ -69,6 +71,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "walk.cuh"
 
@@ -118,7 +121,7 @@ struct ChainClass<Cls32> {
     using W = uint32_t;
     using M = Mont32;
     using U = int32_t;                         // a block product, reduced
-    using Pair = uint2;
+    using Q = uint32_t;                        // p^-1, as reduce and prod take it
     static constexpr int kPlanes = 3;
     static constexpr bool kInTmem = true;      // 3 planes of K / 2 columns
     static constexpr int kBlocksE = 16;        // blocks per MMA of the residues, in
@@ -128,7 +131,7 @@ struct ChainClass<Cls32> {
     static constexpr uint32_t kIdle = 0x7FFFFFFFu;
     static constexpr float kScale = 4194304.0f;   // 2^22: |r| < p
     static constexpr int kShift = 6;
-    __device__ static __forceinline__ uint32_t qv(const M &m) { return m.pinv; }
+    __device__ static __forceinline__ Q qv(const M &m) { return m.pinv; }
     // 2^bits w_0, w_0 = 2^64 (u = T 2^-32 = W 2^32, r u 2^-32 = r W), from the
     // next power of R
     __device__ static __forceinline__ W power(const M &m, uint32_t bits) {
@@ -163,7 +166,7 @@ struct ChainClass<Cls64L> {
     using W = uint64_t;
     using M = Mont64;
     using U = uint64_t;
-    using Pair = ulonglong2;
+    using Q = uint32_t;
     static constexpr int kPlanes = 6;
     // 6 planes do not fit in TMEM; with them in shared memory an MMA takes 41
     // cycles for 16 or for 32 blocks (the planes' read), so 32, in one buffer
@@ -175,7 +178,7 @@ struct ChainClass<Cls64L> {
     static constexpr uint64_t kIdle = 0x1FFFFFFFFFFFFFFFull;
     static constexpr float kScale = 2097152.0f;   // 2^21: r < 2p
     static constexpr int kShift = 5;
-    __device__ static __forceinline__ uint32_t qv(const M &m) { return m.q32; }
+    __device__ static __forceinline__ Q qv(const M &m) { return m.q32; }
     __device__ static __forceinline__ W two32(W p) { return p > (1ull << 32) ? (1ull << 32) : (1ull << 32) - p; }
     // 2^bits w_0, w_0 = 2^96 (u = T 2^-32 = W 2^64, r u 2^-64 = r W), from the
     // next power of R down by lazy rounds of 2^-32, in [0, 2p) as are the w_b
@@ -206,6 +209,44 @@ struct ChainClass<Cls64L> {
     __device__ static __forceinline__ float value(W r, uint32_t sh) {
         return (float)__funnelshift_rc((uint32_t)r, (uint32_t)(r >> 32), sh);
     }
+};
+
+// class 64 from 2^64/3: residues in [0, p), R = 2^64
+template <>
+struct ChainClass<Cls64> {
+    using W = uint64_t;
+    using M = Mont64;
+    using U = uint64_t;
+    using Q = uint64_t;
+    using L = ChainClass<Cls64L>;
+    static constexpr int kPlanes = 6;
+    static constexpr bool kInTmem = false;
+    static constexpr int kBlocksE = L::kBlocksE, kBufsE = L::kBufsE;
+    static constexpr int kReduceGroups = L::kReduceGroups, kReplayWarps = L::kReplayWarps;
+    static constexpr int kUnit = L::kUnit, kUUnits = L::kUUnits, kRUnits = L::kRUnits;
+    static constexpr uint64_t kIdle = L::kIdle;
+    static constexpr float kScale = 4194304.0f;   // 2^22: r < p
+    static constexpr int kShift = 6;
+    __device__ static __forceinline__ Q qv(const M &m) { return m.pinv; }
+    __device__ static __forceinline__ W power(const M &m, uint32_t bits) {
+        const uint32_t k = (bits + 96 + 63) / 64;
+        return m.mul(m.mont_R_pow(k - 1), 1ull << (bits + 160 - 64 * k));
+    }
+    __device__ static __forceinline__ W div64(const M &m, W x) { return m.mul(x, 1ull << 58); }
+    __device__ static __forceinline__ W c32(const M &m) { return m.to_mont(1ull << 32); }
+    __device__ static __forceinline__ W step32(const M &m, W x, W c96) { return m.mul(x, c96); }
+    // T = L + 2^32 H: u = (T + m p) / 2^32 with m = -T p^-1 is a carry of m p
+    // (at most p) and T's high part (below 2^46), less p where that passes p
+    __device__ static __forceinline__ W reduce(const uint32_t (&b)[6], W p, Q q, uint2 sh) {
+        const uint64_t L = gather(b[0], b[1], b[2], sh), H = gather(b[3], b[4], b[5], sh);
+        const uint32_t m = 0u - (uint32_t)L * (uint32_t)q;
+        const uint64_t c = (uint64_t)m * (uint32_t)p + (uint32_t)L, t = H + (L >> 32);
+        const uint64_t u = (uint64_t)m * (uint32_t)(p >> 32) + (c >> 32) + t;
+        return u < t || u >= p ? u - p : u;
+    }
+    __device__ static __forceinline__ W prod(W r, W u, W p, Q q) { return redc64(r, u, p, q); }
+    __device__ static __forceinline__ uint32_t shift(W) { return 32; }
+    __device__ static __forceinline__ float value(W r, uint32_t) { return (float)(uint32_t)(r >> 32); }
 };
 
 // Warp roles, in groups of four warps (a thread per candidate): testers
@@ -253,7 +294,7 @@ struct Lay {
     static constexpr uint32_t kOffQs = kOffQk + kBatches * 32 * 4;                        // written: round + 1
     static constexpr uint32_t kOffP = kOffQs + kBatches * 32 * 4;                         // candidates' p, then q
     static constexpr uint32_t kOffPq = kOffP + kCands * sizeof(W);
-    static constexpr uint32_t kOffBar = kOffPq + kCands * 4;
+    static constexpr uint32_t kOffBar = kOffPq + kCands * sizeof(typename C::Q);
     static constexpr uint32_t kBars = kFStages + kWStages + 2 * kBufs + 2 * C::kRUnits + 2 * kBufsE + 2 * C::kUUnits + kBufs + 1;
     static constexpr uint32_t kOffMisc = kOffBar + kBars * 8;   // failed, TMEM address, suspects, testers done, [batch] rounds replayed
     static constexpr uint32_t kSmem = kOffMisc + 16 + kBatches * 4;
@@ -401,18 +442,17 @@ __device__ __forceinline__ constexpr uint32_t idesc_n(uint32_t n) {
 // steps before, which hit at n = p - 1 and p - 2.  Such a block is a suspect:
 // 0 = +-0.)
 template <class T>
-__device__ __forceinline__ void replay_suspect(bool act, typename T::W p, uint32_t q, typename T::W r, uint32_t k,
+__device__ __forceinline__ void replay_suspect(bool act, typename T::W p, typename ChainClass<T>::Q q, typename T::W r, uint32_t k,
                                                uint32_t len, const uint32_t *mult, int32_t type, const HitBuf &h) {
     using W = typename T::W;
     typename T::M m;
     m.p = p;
-    W t;
-    if constexpr (sizeof(W) == 4) {
-        m.pinv = q;
-        t = 1;
-    } else {
+    W t = 1;
+    if constexpr (std::is_same<T, Cls64L>::value) {
         m.q32 = q;
-        t = ChainClass<Cls64L>::two32(p);
+        t = ChainClass<T>::two32(p);
+    } else {
+        m.pinv = q;
     }
     uint32_t mul[16];
 #pragma unroll
@@ -573,7 +613,7 @@ __global__ void __launch_bounds__(Role<T>::kThreads, 1)
     const uint32_t fail = smem_u32(misc);
     uint32_t *taddr_slot = misc + 1, *suspects = misc + 2, *testers_done = misc + 3, *replayed = misc + 4;
     W *cand_p = reinterpret_cast<W *>(sm + L::kOffP);
-    uint32_t *cand_q = reinterpret_cast<uint32_t *>(sm + L::kOffPq);
+    auto *cand_q = reinterpret_cast<typename C::Q *>(sm + L::kOffPq);
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(taddr_slot))
@@ -852,7 +892,8 @@ __global__ void __launch_bounds__(Role<T>::kThreads, 1)
     } else if (warp < Role<T>::kChain) {
         // --------------------------------------------------------- reducers
         const W p = m.p;
-        const uint32_t q = C::qv(m), grp = (warp - Role<T>::kReduce) / 4;
+        const typename C::Q q = C::qv(m);
+        const uint32_t grp = (warp - Role<T>::kReduce) / 4;
         const uint2 shifts = make_uint2(a.shift11, a.shift22);
         typename C::U *us = reinterpret_cast<typename C::U *>(sm + L::kOffU) + cl;
         constexpr int kBlocksUnit = C::kUnit * kBlocksTile;
@@ -911,7 +952,7 @@ __global__ void __launch_bounds__(Role<T>::kThreads, 1)
     } else if (warp < Role<T>::kTestMma) {
         // ------------------------------------------------------------ chain
         const W p = m.p;
-        const uint32_t q = C::qv(m);
+        const typename C::Q q = C::qv(m);
         const typename C::U *us = reinterpret_cast<const typename C::U *>(sm + L::kOffU) + cl;
         W *rs = reinterpret_cast<W *>(sm + L::kOffR) + cl;
         constexpr int kBlocksUnit = C::kUnit * kBlocksTile;
@@ -1140,8 +1181,8 @@ int launch_walk_tc32(const ClassBuf<uint32_t> &c, const WalkTcArgs &a, uint32_t 
     return launch_tc<Cls32>(c, a, top, h, sp, err, st);
 }
 int launch_walk_tc64(const ClassBuf<uint64_t> &c, const WalkTcArgs &a, uint32_t top, const HitBuf &h,
-                     const SplitArgs<uint64_t> *sp, uint32_t *err, cudaStream_t st) {
-    return launch_tc<Cls64L>(c, a, top, h, sp, err, st);
+                     const SplitArgs<uint64_t> *sp, uint32_t *err, cudaStream_t st, bool lazy) {
+    return lazy ? launch_tc<Cls64L>(c, a, top, h, sp, err, st) : launch_tc<Cls64>(c, a, top, h, sp, err, st);
 }
 
 }  // namespace pfc

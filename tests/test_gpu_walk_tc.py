@@ -34,7 +34,7 @@ def same(a, b):
 
 
 @pytest.mark.parametrize("mode", [1, 2, 4, 5])
-@pytest.mark.parametrize("p", [2**16, 2**31 - 20000, 2**62, 2**64 // 3 - 100000])
+@pytest.mark.parametrize("p", [2**16, 2**31 - 20000, 2**62, 2**64 // 3 - 100000, 2**64 // 3, 2**64 - 60000])
 def test_walk_matches_the_oracle(mode, p):
     nmin, nmax = 101, 9000 + p % 7
     hi = p + 50003
@@ -51,7 +51,7 @@ def test_walk_matches_the_oracle(mode, p):
 @pytest.mark.parametrize("nmin,length", [(n, k) for n in (201000, 202001, 12899000)
                                          for k in (1, 15, 17, 64, 255, 257, 1025, 4097)] + [(2**31 - 6000, 2049)])
 def test_lengths_and_word_shapes(nmin, length):
-    for p in (1500000000, 2**45):
+    for p in (1500000000, 2**45, 2**63 + 2**61):
         args = (1, nmin, nmin + length, p, p + 200000)
         same(segment(*args, True), segment(*args, False))
 
@@ -59,6 +59,7 @@ def test_lengths_and_word_shapes(nmin, length):
 @pytest.mark.parametrize("mode,p,span,cuts,split", [
     (5, 10**9, 40, (), False), (2, 2**40, 2700, (), False), (5, 10**9, 2800, (), True), (1, 2**40, 60000, (), True),
     (5, 10**8, 150000, (517, 1541, 9000, 20001), False), (2, 2**50, 150000, (517, 1541, 9000, 20001), False),
+    (5, 2**64 - 60000, 59999, (517, 1541, 9000, 20001), False), (2, 2**64 // 3 - 30000, 60000, (), True),
     (4, 2**31 - 70000, 150000, (), True), (5, 2**31 - 70000, 150000, (), True),
 ])
 def test_candidate_counts_and_ranges(mode, p, span, cuts, split):
