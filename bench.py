@@ -487,7 +487,7 @@ def hit_order(f):
 # programs below these sizes (896-bit words, both programs of a search) keep the
 # integer-pipe setup when the tensor-core setup is on: kTcMinWords32 and
 # kTcMinWords64 of pfcsieve_gb300/csrc/kernels.cuh
-TC_MIN_WORDS = {32: 448, 64: 480}
+TC_MIN_WORDS = {32: 240, 64: 216}
 
 
 def mixed_roofline(jobs, outcomes, seconds, peaks, tc_s=0.0, setup_tc=True):

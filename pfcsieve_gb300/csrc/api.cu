@@ -388,10 +388,20 @@ uint64_t host_prog(const HostMont &m, const HostProg<W> &pg, uint64_t acc) {
 uint64_t host_tc_prog(const HostMont &m, const HostProg<WideWord> &pg, uint64_t acc) {
     TcProg tp;
     if (!build_tc_prog(pg, tp)) return ~0ull;
-    return host_run(m, tp.groups, tp.final_sq, tp.corr, acc, [&](uint32_t i) {
-        const uint32_t s = tp.src[i] & 0x7FFFFFFFu;
-        const uint64_t z = host_word(m, pg.words[s]);
-        return (tp.src[i] & 0x80000000u) ? m.mul(z, host_word(m, pg.words[s + 1])) : z;
+    // a group's words: its lanes of every tile
+    std::vector<uint32_t> groups, src;
+    for (size_t g = 0; g + 2 < tp.groups.size(); g += 3) {
+        groups.push_back((uint32_t)src.size());
+        for (size_t t = 0; t < tp.src.size(); t += kTcLanes)
+            src.insert(src.end(), tp.src.begin() + t + tp.groups[g], tp.src.begin() + t + tp.groups[g + 1]);
+        groups.push_back((uint32_t)src.size());
+        groups.push_back(tp.groups[g + 2]);
+    }
+    return host_run(m, groups, tp.final_sq, tp.corr, acc, [&](uint32_t i) {
+        if (src[i] == kTcOne) return 1 % m.p;
+        const uint32_t s = src[i] & 0x7FFFFFFFu, own = (uint32_t)pg.words.size();
+        auto word = [&](uint32_t k) { return host_word(m, k < own ? pg.words[k] : tp.extra[k - own]); };
+        return (src[i] & 0x80000000u) ? m.mul(word(s), word(s + 1)) : word(s);
     });
 }
 }  // namespace
@@ -487,11 +497,11 @@ extern "C" int pfc_job_create(pfc_ctx *c, unsigned mode, uint32_t nmin, uint32_t
         }
     }
 
-    cudaError_t e = j->a32.upload(c, a32);
+    cudaError_t e = j->a32.upload(c, a32, j->tcp[0].extra);
     if (e == cudaSuccess) e = j->a64.upload(c, a64);
-    if (e == cudaSuccess) e = j->aw.upload(c, aw);
-    if (e == cudaSuccess) e = j->bw.upload(c, bw);
-    if (e == cudaSuccess) e = j->b32.upload(c, b32);
+    if (e == cudaSuccess) e = j->aw.upload(c, aw, j->tcp[0].extra);
+    if (e == cudaSuccess) e = j->bw.upload(c, bw, j->tcp[1].extra);
+    if (e == cudaSuccess) e = j->b32.upload(c, b32, j->tcp[1].extra);
     if (e == cudaSuccess) e = j->b64.upload(c, b64);
     if (e == cudaSuccess && (mode & PFC_COMPOSITORIAL)) e = j->primebits.upload(c, prime_bitmap(nmin, nmax, primes));
     if (e == cudaSuccess && mode == PFC_PRIMORIAL) {

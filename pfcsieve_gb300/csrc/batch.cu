@@ -407,6 +407,7 @@ struct BatchJob {
     // first program then the second's; tc_nw counts the 896-bit words of the
     // first program, tc_pw the paired words of each)
     std::vector<uint32_t> tcsrc, tcgroups;
+    uint32_t tc_second = 0;   // first word of the second program
     uint32_t tc_ng[2] = {0, 0}, tc_fsq[2] = {0, 0}, tc_nw[2] = {0, 0}, tc_pw[2] = {0, 0}, tc_ntiles[2] = {0, 0};
     uint64_t tc_corr[2] = {0, 0};
     uint64_t c32a = 0, c32b = 0, c64a = 0, c64b = 0;
@@ -508,13 +509,15 @@ static void prepare_job(BatchJob *j, const std::vector<uint32_t> &cache) {
     j->c64a = wide ? aw.corr : a64.corr;
     if (wide) {
         const HostProg<WideWord> *pr[2] = {&aw, &bw};
-        j->tc = true;
+        j->tc = true;   // (a second program is one group and has no extra words)
         for (int k = 0; k < (fc ? 2 : 1); ++k) {
             TcProg tp;
-            if (!build_tc_prog(*pr[k], tp)) {
+            if (!build_tc_prog(*pr[k], tp) || (k && !tp.extra.empty())) {
                 j->tc = false;
                 break;
             }
+            j->wordsw.insert(j->wordsw.end(), tp.extra.begin(), tp.extra.end());
+            if (k == 0) j->tc_second = (uint32_t)j->wordsw.size();
             j->tcsrc.insert(j->tcsrc.end(), tp.src.begin(), tp.src.end());
             j->tcgroups.insert(j->tcgroups.end(), tp.groups.begin(), tp.groups.end());
             j->tc_ng[k] = (uint32_t)(tp.groups.size() / 3);
@@ -571,9 +574,9 @@ static void free_vec(std::vector<W> &v) {
 using namespace pfc;
 
 // a tensor-core setup tile of one candidate block (128 paired words x 32
-// candidates, about 9,000 SM cycles) in the budget's units: multiplies at
-// 64 per SM cycle
-constexpr double kTcTileCost = 9000.0 * 64.0;
+// candidates, about 3,000 SM cycles) in the budget's units, multiplies at 64
+// per SM cycle, and the block's fixed part in tiles
+constexpr double kTcTileCost = 3000.0 * 64.0, kTcFixedTiles = 6.0;
 // share of a latency-policy iteration's budget given to setup chunks
 constexpr double kTcChunkShare = 0.5;
 
@@ -738,7 +741,7 @@ int upload_job(pfc_batch *b, BatchJob *j) {
     }
     if (tc) {
         c->launches += launch_tc_pack(j->d_wordsw.p, j->d_tcsrc.p, j->tc_pw[0], j->tc_ntiles[0], j->d_tct.p, c->st);
-        c->launches += launch_tc_pack(j->d_wordsw.p + j->tc_nw[0], j->d_tcsrc.p + j->tc_pw[0], j->tc_pw[1],
+        c->launches += launch_tc_pack(j->d_wordsw.p + j->tc_second, j->d_tcsrc.p + j->tc_pw[0], j->tc_pw[1],
                                       j->tc_ntiles[1], j->d_tct.p + (size_t)j->tc_ntiles[0] * tb, c->st);
         CK(cudaGetLastError());
     }
@@ -882,7 +885,7 @@ int admit_prepared(pfc_batch *b) {
                 // small programs keep their setup windows (kernels.cuh kTcMinWords*)
                 if (!n || words < (cls ? kTcMinWords64 : kTcMinWords32)) continue;
                 j->tc_blocks[cls] = cls ? tc_setup_blocks(n) : tc_setup_blocks32(n);
-                j->tc_block_cost[cls] = kTcTileCost * ((double)j->tc_ntiles[0] + j->tc_ntiles[1]);
+                j->tc_block_cost[cls] = kTcTileCost * ((double)j->tc_ntiles[0] + j->tc_ntiles[1] + kTcFixedTiles);
                 (cls ? j->pos64 : j->pos32) = cls ? j->nsetup64 : j->nsetup32;
                 j->tc_wait[cls] = true;
                 if (b->policy == PFC_BATCH_LATENCY) {

@@ -114,8 +114,16 @@ struct DevProg {
     DArr<W> words;
     DArr<uint32_t> groups;
     Prog<W> view{};
-    cudaError_t upload(pfc_ctx *c, const HostProg<W> &h) {
-        cudaError_t e = words.upload(c, h.words);
+    // (extra: words behind the program's own, of its tensor-core form)
+    cudaError_t upload(pfc_ctx *c, const HostProg<W> &h, const std::vector<W> &extra = {}) {
+        cudaError_t e;
+        if (extra.empty()) {
+            e = words.upload(c, h.words);
+        } else {
+            std::vector<W> all(h.words);
+            all.insert(all.end(), extra.begin(), extra.end());
+            e = words.upload(c, all);
+        }
         if (e == cudaSuccess) e = groups.upload(c, h.groups);
         view.words = words.p;
         view.groups = groups.p;

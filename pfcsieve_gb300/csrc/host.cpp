@@ -169,20 +169,99 @@ static bool finish_prog(HostProg<W> &p) {
     return true;
 }
 
+// a *= b if the product fits a word
+static bool join(WideWord &a, const WideWord &b) {
+    constexpr uint64_t mask = (1ull << kWideRadixBits) - 1u;
+    auto size = [](const WideWord &w) {
+        int k = kWideLimbs;
+        while (k > 1 && !w.limb[k - 1]) --k;
+        return k;
+    };
+    const int na = size(a), nb = size(b);
+    if (na + nb > kWideLimbs + 1) return false;
+    uint64_t v[kWideLimbs + 1] = {};   // columns: at most 32 products below 2^56
+    for (int i = 0; i < na; ++i)
+        for (int k = 0; k < nb; ++k) v[i + k] += (uint64_t)a.limb[i] * b.limb[k];
+    WideWord out{};
+    uint64_t carry = 0;
+    for (int i = 0; i < kWideLimbs; ++i) {
+        carry += v[i];
+        out.limb[i] = (uint32_t)(carry & mask);
+        carry >>= kWideRadixBits;
+    }
+    if (carry + v[kWideLimbs]) return false;
+    a = out;
+    return true;
+}
+
 bool build_tc_prog(const HostProg<WideWord> &p, TcProg &out) {
     out = TcProg();
-    HostProg<uint64_t> shape;   // the groups of the paired words, for the drift correction
-    for (size_t g = 0; g + 2 < p.groups.size(); g += 3) {
-        const uint32_t b = p.groups[g], e = p.groups[g + 1];
-        const uint32_t first = (uint32_t)out.src.size();
-        for (uint32_t w = b; w < e; w += 2) out.src.push_back(w + 1 < e ? (w | 0x80000000u) : w);
-        shape.groups.push_back(first);
-        shape.groups.push_back((uint32_t)out.src.size());
-        shape.groups.push_back(p.groups[g + 2]);
+    const size_t ng = p.groups.size() / 3;
+    if (!ng) {
+        HostProg<uint64_t> none;
+        none.final_sq = p.final_sq;
+        if (!finish_prog(none)) return false;
+        out.final_sq = none.final_sq;
+        out.corr = none.corr;
+        return true;
+    }
+    // the tiles that paired words of `n[g]` a group fill, whole lanes to a group
+    auto tiles = [](const std::vector<size_t> &n) {
+        size_t all = 0;
+        for (size_t k : n) all += k;
+        for (size_t t = std::max<size_t>(1, (all + kTcLanes - 1) / kTcLanes);; ++t) {
+            size_t lanes = 0;
+            for (size_t k : n) lanes += (k + t - 1) / t;
+            if (lanes <= kTcLanes) return t;
+        }
+    };
+    // merge the first groups as deep as that takes the fewest tiles
+    std::vector<WideWord> first(p.words.begin() + p.groups[0], p.words.begin() + p.groups[1]), best = first;
+    size_t depth = 1, nt = 0;
+    for (size_t g = 1;; ++g) {   // `first` holds groups 0 .. g - 1
+        std::vector<size_t> n{(first.size() + 1) / 2};
+        for (size_t k = g; k < ng; ++k) n.push_back((p.groups[3 * k + 1] - p.groups[3 * k] + 1) / 2);
+        if (n.size() <= kTcLanes) {
+            const size_t t = tiles(n);
+            if (!nt || t <= nt) {
+                nt = t;
+                depth = g;
+                best = first;
+            }
+        }
+        if (g == ng || p.groups[3 * g + 2] > 8 || (first.size() << p.groups[3 * g + 2]) > kTcFirstWords) break;
+        std::vector<WideWord> joined;
+        auto add = [&](const WideWord &w) {
+            if (joined.empty() || !join(joined.back(), w)) joined.push_back(w);
+        };
+        for (const WideWord &w : first)
+            for (uint32_t k = 0; k < 1u << p.groups[3 * g + 2]; ++k) add(w);
+        for (uint32_t k = p.groups[3 * g]; k < p.groups[3 * g + 1]; ++k) add(p.words[k]);
+        first.swap(joined);
+    }
+    if (!nt) return false;
+    if (depth > 1) out.extra = best;
+    // lay the groups out, tile by tile within a group's lanes
+    out.src.assign(nt * kTcLanes, kTcOne);
+    HostProg<uint64_t> shape;   // for the drift correction: every lane multiplies nt words
+    size_t lane = 0;
+    for (size_t g = depth - 1; g < ng; ++g) {
+        const bool extra = g + 1 == depth && depth > 1;
+        const uint32_t w0 = extra ? (uint32_t)p.words.size() : p.groups[3 * g];
+        const uint32_t w1 = extra ? w0 + (uint32_t)best.size() : p.groups[3 * g + 1];
+        const size_t n = (w1 - w0 + 1) / 2, own = g + 1 == ng ? kTcLanes - lane : (n + nt - 1) / nt;
+        for (size_t i = 0; i < n; ++i) {
+            const uint32_t w = w0 + 2 * (uint32_t)i;
+            out.src[i / own * kTcLanes + lane + i % own] = w + 1 < w1 ? (w | 0x80000000u) : w;
+        }
+        // (a merged first group, or the first, has its own squarings before it)
+        const uint32_t sq = p.groups[3 * (g + 1 == depth ? 0 : g) + 2];
+        for (size_t v : {lane, lane + own, (size_t)sq}) out.groups.push_back((uint32_t)v);
+        for (size_t v : {lane * nt, (lane + own) * nt, (size_t)sq}) shape.groups.push_back((uint32_t)v);
+        lane += own;
     }
     shape.final_sq = p.final_sq;
     if (!finish_prog(shape)) return false;
-    out.groups = shape.groups;
     out.final_sq = shape.final_sq;
     out.corr = shape.corr;
     return true;

@@ -35,11 +35,24 @@ struct HostProg {
 
 // The tensor-core form of a 896-bit program: within each group, consecutive
 // pairs of words are multiplied into one 1792-bit word (a group's odd last
-// word stays alone), so the device multiplies half as many words into its
-// accumulator.  src[i]: index of the first 896-bit word of word i, with bit 31
-// set when the next word is multiplied in too.  groups, final_sq and corr are
-// those of this word count (each word lowers the power of R by one).
+// word stays alone), so the device multiplies half as many words.  The words
+// are laid out in tiles of kTcLanes, each group in lanes of its own through all
+// tiles, so that a lane's running product belongs to one group and the
+// squarings between the groups are due only once, on the products of the lanes
+// (on running products they would cost most of a tile each).  src[i]: lane i %
+// kTcLanes of tile i / kTcLanes, the index of its first 896-bit word, with bit
+// 31 set when the next word is multiplied in too, or kTcOne.  The first groups
+// (few words each) are merged where that takes no more tiles: a group's words
+// join the words of the groups before it repeated 2^squarings times,
+// multiplied together where the product fits 896 bits.  Those words are
+// `extra`, numbered from the program's last word on.  groups: {first lane, end
+// lane, squarings before}; corr is that of this word count (every lane of
+// every tile lowers the power of R by one).
+constexpr size_t kTcLanes = 128;
+constexpr size_t kTcFirstWords = 2048;   // bounds the merged words tried
+constexpr uint32_t kTcOne = 0x7FFFFFFFu;
 struct TcProg {
+    std::vector<WideWord> extra;
     std::vector<uint32_t> src;
     std::vector<uint32_t> groups;
     uint32_t final_sq = 0;

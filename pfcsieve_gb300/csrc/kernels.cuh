@@ -157,15 +157,15 @@ int launch_setup64w_tc(const ClassBuf<uint64_t> &c, const SetupArgs<WideWord> &a
 // class 32 on the same tiles (the class-32 and lazy class-64 programs are the same)
 uint32_t tc_setup_blocks32(uint32_t cands);
 // Smallest programs (896-bit words, both programs of the search) set up on the
-// tensor cores: below them the kernel's fixed cost per CTA (the 224 position
-// residues, TMEM, the first tile's copy and products, the final tree, tens of
-// thousands of cycles) outweighs what it saves per word.  Measured on GB300
+// tensor cores: below them the kernel's fixed cost per CTA (the position
+// residues' planes, TMEM, the first tile's copy and products, the final tree,
+// about 18,000 cycles) outweighs what it saves per word.  Measured on GB300
 // (factorial searches, 4e6-wide p ranges), integer pipe against tensor cores:
-// class 32 at 235 words 0.22 / 0.33 ms, at 460 words 0.41 / 0.40 ms; class 64
-// at 460 words 0.79 / 0.80 ms, at 687 words 1.16 / 0.92 ms, at 20,330 words
-// 33.4 / 8.0 ms.
-constexpr uint64_t kTcMinWords32 = 448;
-constexpr uint64_t kTcMinWords64 = 480;
+// class 32 at 214 words 0.203 / 0.226 ms, at 304 0.280 / 0.246, at 2,265 1.95 /
+// 0.45; class 64 at 145 words 0.28 / 0.39 ms, at 214 0.396 / 0.394, at 304
+// 0.54 / 0.44, at 2,265 3.77 / 0.79.
+constexpr uint64_t kTcMinWords32 = 240;
+constexpr uint64_t kTcMinWords64 = 216;
 int launch_setup32_tc(const ClassBuf<uint32_t> &c, const SetupArgs<WideWord> &a, const TcTiles &ta,
                       const TcTiles &tb, uint32_t *err, cudaStream_t st, uint32_t block0 = 0, uint32_t nblocks = 0);
 // start residues of a split walk: boundary k's into s0/s1 + (k-1) * c.cap

@@ -11,162 +11,108 @@
 // tensor cores in fp16 with fp32 accumulation and stays exact:
 //   * the words are 1792-bit: each is the product of a pair of the program's
 //     896-bit words (host.hpp TcProg), so half as many words reach the
-//     CUDA cores; a word is its 224 bytes z_b (0..255, exact in fp16);
-//   * a candidate's 64-bit residues w_b are split into 8 byte planes
-//     W_a[b] = byte a of w_b (0..255);
-//   * the bytes are summed in two halves of 112, each into its own fp32
-//     accumulator: D_{a,h}[word, cand] = 2^23 + sum_{b in half h} z_b W_a[b].
-//     The first MMA of each half writes 2048 * 4096 = 2^23 into every sum, and
-//     a half's sum is at most 112 * 255 * 255 < 2^23, so every partial sum is
-//     an integer in [2^23, 2^24), exact in fp32, and the fp32 bits of D are
-//     0x4B000000 + the integer sum;
-//   * T = sum_a (D_{a,0} + D_{a,1} - 2^24) 2^(8a) < 2^79 is assembled on the
-//     CUDA cores.
-// The programs are first laid out as fp16 byte tiles of 128 words (A operand,
-// M = 128, K = 224, the shared-memory image; tc_pack_kernel multiplies the
-// word pairs, once per job).  One CTA of 512 threads owns 32 candidates:
-// their byte planes stay in shared memory as the MMA's B operand, K-major,
-// one 8-row core group per candidate (row = plane), so that one MMA with
-// N = 256 covers the 32 candidates x 8 planes and a candidate's 8 sums of a
-// half are adjacent TMEM columns (two halves x 256 columns, word = TMEM lane;
-// per half a bias MMA and seven MMAs of K = 16, 16 per tile).  Per tile t:
-//   1. each thread reads one word's sums for a share of the candidates
-//      (tcgen05.ld, 4 candidates x 8 planes per load and half; the four warps
-//      of a lane quadrant split the candidates), assembles T and reduces it
-//      by one Montgomery round, u = (T + m p) / 2^32 with m = -T p^-1 mod 2^32,
-//      so u = T 2^-32 = Z (mod p) and u < 2^48 + p, stored in shared memory;
-//      meanwhile tile t+1 arrives by one bulk copy (cp.async.bulk);
-//   2. the products of tile t+1 are issued; they run while
-//   3. fifteen threads of each candidate (one per warp but the first, whose
-//      thread 0 issued the products) multiply a fifteenth of the tile's u
-//      into their running products, two independent chains per thread (two
-//      lazy rounds per product; a product lowers the power of R by one, as a
-//      word on the integer pipe does).  At a group start that carries
-//      squarings (Horner over exponent bits) every thread squares each of its
-//      running products (squaring distributes over their Montgomery product);
-//      at the end of a program they are combined into the accumulator (a tree
-//      over the threads of the candidate).
-// Class 32 (p < 2^31) runs the same kernel with 4 byte planes, 64 candidates
-// per CTA (N = 64 x 4 = 256 again), T < 2^47 reduced by one 32-bit round and
-// one Montgomery product (R = 2^32) per word.  The result equals
+//     CUDA cores; a word is 225 balanced base-256 digits z_b (-128..127, the
+//     last one a carry of 0 or 1);
+//   * a candidate's residues w_b are balanced base-256 digits too, in 8 planes
+//     W_a[b];
+//   * digits of either sign keep a whole word's sums in one accumulator:
+//     S_a[word, cand] = sum_b z_b W_a[b] has |S_a| <= 225 * 128 * 128 < 2^22
+//     and rides on a bias of 1.5 * 2^23 (digit 225: 4096 in every word, 3072
+//     in every plane), so every partial sum is an integer in [2^23, 2^24),
+//     exact in fp32, and the accumulator's bits are 0x4B400000 + S_a;
+//   * on the CUDA cores neighbouring planes combine as t_j = S_2j + 256 S_2j+1
+//     + 0x8B400000 straight from those bits, which is positive and below 2^32,
+//     so T' = sum_j t_j 2^(16j) needs no corrections: digit 226, 1 in every
+//     word, carries minus the constant's residue mod p, and T' = Z 2^32 (mod p).
+// The programs are first laid out as fp16 tiles of 128 words (A operand, M =
+// 128, K = 240, the shared-memory image in three parts of K = 80;
+// tc_pack_kernel multiplies the word pairs, once per job).  One CTA owns 32
+// candidates: their planes stay in shared memory as the MMA's B operand,
+// K-major, one 8-row core group per candidate (row = plane), so that one MMA
+// with N = 256 covers the 32 candidates x 8 planes and a candidate's 8 sums are
+// adjacent TMEM columns (word = TMEM lane).  Two such buffers of 256 columns.
+// A warp copies the tiles' parts (cp.async.bulk) as the MMAs release them, a
+// warp issues the MMAs, 15 of K = 16 per tile, and 16 warps take the sums of
+// the other buffer: a thread owns one word (TMEM lane) and a quarter of the
+// candidates, and keeps a running product for each of those in registers:
+// it reduces T' by one Montgomery round, u = (T' + m p) / 2^32 with m = -T' p^-1
+// mod 2^32, so u = Z (mod p) up to a power of R and u < 2^48 + p, and multiplies
+// it in (two lazy rounds; a product lowers the power of R by one, as a word on
+// the integer pipe does).  A lane's words all belong to one group of the
+// program, so the squarings between the groups (Horner over exponent bits) wait
+// until the program's end, where the lanes' products are multiplied over a tree
+// through shared memory.  So a tile needs no barrier among the threads.
+// Class 32 (p < 2^31) runs the same kernel with 4 planes, 64 candidates per CTA
+// (N = 64 x 4 = 256 again), T' < 2^48 reduced by one 32-bit round and one
+// Montgomery product (R = 2^32) per word.  The result equals
 // setup_kernel<Cls64L>'s or setup_kernel<Cls32>'s: the same product of the
 // same words in the same Horner order, exact arithmetic, canonical residues
-// at the end.  Every wait is bounded; after a timeout the kernel sets bit 1 of
-// `flags`, frees its TMEM and stores nothing.
+// at the end.  Every wait is bounded; after one that gave up the kernel sets
+// bit 1 of `flags`, frees its TMEM and stores nothing.
 #include <cuda_runtime.h>
 
 #include <cstdint>
 
+#include "host.hpp"
+#include "tcgen05.cuh"
 #include "walk.cuh"
 
 namespace pfc {
 namespace {
 
-constexpr int kTcThreads = 512;
-constexpr int kTcGroups = kTcThreads / 128;   // warp groups (each covers the 128 TMEM lanes)
-constexpr int kTcWords = 128;                 // words per tile: MMA M, TMEM lanes
-constexpr int kTcN = 256;                     // MMA N: candidates x byte planes
-constexpr int kTcBytes = 224;                 // bytes of a 1792-bit word: MMA K
-constexpr int kTcHalfBytes = kTcBytes / 2;    // bytes summed into one accumulator
-constexpr int kTcChains = 2;                  // independent product chains per thread
-constexpr uint32_t kRowGroup = (kTcBytes / 8) * 128;              // 3584 B between 8-row core groups
-constexpr uint32_t kBiasRowGroup = 2 * 128;                       // bias tiles: K = 16
-constexpr uint32_t kATile = (kTcWords / 8) * kRowGroup;           // 57,344 B
-constexpr uint32_t kBTile = (kTcN / 8) * kRowGroup;               // 114,688 B: rows = candidate x plane
-constexpr uint32_t kUStride = kTcWords + 1;   // words per candidate row; odd: column reads hit distinct banks
+constexpr int kTcWorkers = 512;               // threads that take the sums
+constexpr int kTcThreads = kTcWorkers + 64;   // and the warps of the MMAs and of the copies
+constexpr uint32_t kTcWords = kTcLanes;       // words per tile: MMA M, TMEM lanes
+constexpr uint32_t kTcN = 256;                // MMA N: candidates x planes
+constexpr uint32_t kTcDigits = 225;           // digits of a 1792-bit word, with its carry
+constexpr uint32_t kTcK = 240;                // MMA K: digits, bias, offset, zeros
+constexpr uint32_t kStages = 3;               // parts of a tile
+constexpr uint32_t kStageK = kTcK / kStages;
+constexpr uint32_t kStageGroup = (kStageK / 8) * 128;             // bytes between 8-row core groups of a part
+// and of the planes: 16 bytes more than they take, so that the threads that
+// write the same plane of neighbouring candidates hit distinct banks
+constexpr uint32_t kRowGroup = (kTcK / 8) * 128 + 16;
+constexpr uint32_t kStageBytes = (kTcWords / 8) * kStageGroup;    // 20,480
+constexpr uint32_t kATile = kStages * kStageBytes;                // 61,440
+constexpr uint32_t kBTile = (kTcN / 8) * kRowGroup;               // 123,392: rows = candidate x plane
 constexpr uint32_t kOffA = 0;
 constexpr uint32_t kOffB = kOffA + kATile;
-constexpr uint32_t kOffABias = kOffB + kBTile;                                // 128 x 16, column 0 = 2048
-constexpr uint32_t kOffBBias = kOffABias + (kTcWords / 8) * kBiasRowGroup;    // 256 x 16, column 0 = 4096
-constexpr uint32_t kOffU = kOffBBias + (kTcN / 8) * kBiasRowGroup;            // reduced words [cands][kUStride]
-static_assert(kOffB % 16 == 0 && kOffABias % 16 == 0 && kOffBBias % 16 == 0 && kOffU % 16 == 0,
-              "setup_tc alignment");
-static_assert(kATile % 16 == 0, "bulk copies move multiples of 16 bytes");
-static_assert(kTcHalfBytes % 16 == 0, "setup_tc shape");
-constexpr uint32_t kTmemCols = 2 * kTcN;      // 2 halves x 256 (column = 256 h + planes c + plane)
-constexpr long kWaitLimit = 1L << 26;         // mbarrier polls before giving up
-constexpr uint32_t kBiasBits = 0x4B000000u;   // fp32 bits of 2^23
-
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-// shared-memory matrix descriptor: K-major, no swizzle; core matrices of
-// 8 rows x 16 bytes, K-adjacent cores 128 B apart (leading byte offset),
-// 8-row groups `sbo` apart (stride byte offset), descriptor version 1
-__device__ __forceinline__ uint64_t mdesc(uint32_t addr, uint32_t sbo) {
-    return (uint64_t)((addr & 0x3FFFF) >> 4) | ((uint64_t)(128u >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) |
-           (1ull << 46);
-}
+constexpr uint32_t kOffU = kOffB + kBTile;
+static_assert(kTcDigits + 2 <= kTcK && kStageK % 16 == 0, "setup_tc shape");
+static_assert(kStageBytes % 128 == 0 && kBTile % 128 == 0, "setup_tc alignment");
+constexpr uint32_t kTBias = 0x8B400000u;      // 257 * 0x4B400000 mod 2^32, in every t_j
 
 // byte offset of the core-matrix row holding elements (r, 8 k8 .. 8 k8 + 7)
-__device__ __forceinline__ uint32_t tile_off(uint32_t r, uint32_t k8, uint32_t rowgroup = kRowGroup) {
+__device__ __forceinline__ uint32_t tile_off(uint32_t r, uint32_t k8, uint32_t rowgroup) {
     return (r / 8) * rowgroup + k8 * 128 + (r % 8) * 16;
 }
 
-// two bytes (bits 0-7 and 8-15 of x, or 16-23 and 24-31 with hi) -> two
-// fp16 0..255: the fp16 of 1024 + v is 0x6400 | v (v < 1024), less 1024
+// two bytes (bits 0-7 and 8-15 of x, or 16-23 and 24-31 with hi) -> two fp16
+// v - 128: the fp16 of 1024 + v is 0x6400 | v (v < 1024), less 1152
 template <bool HI>
 __device__ __forceinline__ uint32_t f16x2_of_bytes(uint32_t x) {
-    const uint32_t y = __byte_perm(x, 0x64u, HI ? 0x4342u : 0x4140u);
-    uint32_t r;
-    asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(y), "r"(0x64006400u));
-    return r;
+    return sub_f16x2(__byte_perm(x, 0x64u, HI ? 0x4342u : 0x4140u), 0x64806480u);
 }
 
-// eight bytes -> eight fp16 (16 bytes, one core-matrix row)
+// eight bytes -> eight fp16 v - 128 (16 bytes, one core-matrix row)
 __device__ __forceinline__ uint4 f16x8(uint64_t bytes8) {
     const uint32_t lo = (uint32_t)bytes8, hi = (uint32_t)(bytes8 >> 32);
     return make_uint4(f16x2_of_bytes<false>(lo), f16x2_of_bytes<true>(lo), f16x2_of_bytes<false>(hi),
                       f16x2_of_bytes<true>(hi));
 }
 
-__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
-    for (long it = 0; it < kWaitLimit; ++it) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(mbar), "r"(parity)
-            : "memory");
-        if (ok) return true;
-    }
-    return false;
+// bytes 0..3 of four words each, transposed
+__device__ __forceinline__ void transpose4(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t (&out)[4]) {
+    const uint32_t t0 = __byte_perm(a, b, 0x5140), t1 = __byte_perm(c, d, 0x5140);
+    const uint32_t t2 = __byte_perm(a, b, 0x7362), t3 = __byte_perm(c, d, 0x7362);
+    out[0] = __byte_perm(t0, t1, 0x5410);
+    out[1] = __byte_perm(t0, t1, 0x7632);
+    out[2] = __byte_perm(t2, t3, 0x5410);
+    out[3] = __byte_perm(t2, t3, 0x7632);
 }
 
-// 32 columns of this thread's TMEM lane from column `col`
-__device__ __forceinline__ void ld32(uint32_t taddr, uint32_t col, uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr + col)
-        : "memory");
-}
-
-__device__ __forceinline__ void sync_tc() {
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-
-__device__ __forceinline__ uint64_t mulw2(uint64_t s, uint64_t u, uint64_t p, uint32_t q) {
-    const uint32_t w[2] = {(uint32_t)u, (uint32_t)(u >> 32)};
-    return mul_wide_word<2>(s, w, p, q);
-}
-
-// the program's word range [first, end)
-__device__ __forceinline__ void prog_range(const Prog<WideWord> &pg, uint32_t &first, uint32_t &end) {
-    first = end = 0;
-    if (pg.ngroups) {
-        first = __ldg(pg.groups);
-        end = __ldg(pg.groups + 3 * (pg.ngroups - 1) + 1);
-    }
-}
-
-// What differs between the size classes: the residue type, its byte planes,
-// the reduction of T and the product of a reduced word into a running value.
+// What differs between the size classes: the residue type, its planes, the
+// reduction of T' and the product of a reduced word into a running value.
 template <class T>
 struct TcClass;
 
@@ -177,21 +123,46 @@ struct TcClass<Cls64L> {
     using M = Mont64;
     static constexpr int kPlanes = 8;
     static constexpr uint64_t kIdle = 0x1FFFFFFFFFFFFFFFull;   // an idle slot works on 2^61 - 1
-    __device__ static __forceinline__ uint32_t qv(const M &m) { return m.q32; }   // -p^-1 mod 2^32
-    __device__ static __forceinline__ W two32(const M &m) {   // 2^32 mod p
-        return m.p > (1ull << 32) ? (1ull << 32) : (1ull << 32) - m.p;
+    struct __align__(16) Cand {
+        W p;
+        uint32_t q, pad;   // -p^-1 mod 2^32
+    };
+    __device__ static __forceinline__ Cand cand(const M &m) { return {m.p, m.q32, 0u}; }
+    // 2^bits mod p, from the next power of R down by rounds of 2^-32
+    __device__ static __forceinline__ W power(const M &m, uint32_t bits) {
+        const uint32_t k = (bits + 63) / 64, down = 64 * k - bits;
+        W x = m.mont_R_pow(k - 1);
+        if (down >= 32) x = redc64l(x, 1u, m.p, m.q32);
+        if (down % 32) x = redc64l(x, 1u << (32 - down % 32), m.p, m.q32);
+        return x >= m.p ? x - m.p : x;
     }
-    // T = L + 2^32 H < 2^79: u = (T + m p) / 2^32 with m = -T p^-1 mod 2^32,
-    // so u = T 2^-32 (mod p) and u < 2^48 + p; tw0 + lo(m p0) = 2^32 [tw0 != 0]
-    __device__ static __forceinline__ W reduce(uint64_t L, uint64_t H, W p, uint32_t q) {
+    __device__ static __forceinline__ W div256(const M &m, W x) {
+        x = redc64l(x, 1u << 24, m.p, m.q32);
+        return x >= m.p ? x - m.p : x;
+    }
+    // kTBias (1 + 2^16) (1 + 2^32) mod p
+    __device__ static __forceinline__ W bias(const M &m) {
+        const W g = m.to_mont((W)kTBias * 65537u);
+        return addmod64(m.mul(g, 1u), m.mul(g, 1ull << 32), m.p);
+    }
+    // byte pl of w's balanced digits, plus 128 (w below 2^64/3 needs no sign)
+    __device__ static __forceinline__ W digits(W w, W) { return w + 0x8080808080808080ull; }
+    // T' = L + 2^32 H < 2^80: u = (T' + m p) / 2^32 with m = -T' p^-1 mod 2^32,
+    // so u = T' 2^-32 (mod p) and u < 2^48 + p; t0 + lo(m p0) = 2^32 [t0 != 0]
+    __device__ static __forceinline__ W reduce(const uint32_t (&t)[4], const Cand &c) {
+        const uint64_t L = (uint64_t)t[0] + ((uint64_t)t[1] << 16), H = (uint64_t)t[2] + ((uint64_t)t[3] << 16);
         const uint32_t tw0 = (uint32_t)L;
         const uint64_t Mh = (L >> 32) + H;
-        const uint32_t mm = tw0 * q;
-        const uint64_t lo = (uint64_t)mm * (uint32_t)p;
-        return Mh + (uint64_t)mm * (uint32_t)(p >> 32) + (lo >> 32) + (tw0 != 0 ? 1u : 0u);
+        const uint32_t mm = tw0 * c.q;
+        const uint64_t lo = (uint64_t)mm * (uint32_t)c.p;
+        return Mh + (uint64_t)mm * (uint32_t)(c.p >> 32) + (lo >> 32) + (tw0 != 0 ? 1u : 0u);
     }
-    __device__ static __forceinline__ W prod(const M &m, W s, W u) { return mulw2(s, u, m.p, m.q32); }
-    __device__ static __forceinline__ W sq(const M &m, W s) { return Cls64L::sq(m, s); }
+    // two lazy rounds, s < 2p: below (3p + 2p u_hi + 2^32 p) / 2^32, which is
+    // below 2p for u < 2^48 + p and p < 2^64/3
+    __device__ static __forceinline__ W prod(W s, W u, const Cand &c) {
+        return cios_round(redc64l(s, (uint32_t)u, c.p, c.q), s, (uint32_t)(u >> 32), c.p, c.q);
+    }
+    __device__ static __forceinline__ W canon(W s, const Cand &c) { return s >= c.p ? s - c.p : s; }
 };
 
 // class 32: canonical residues, R = 2^32
@@ -201,65 +172,89 @@ struct TcClass<Cls32> {
     using M = Mont32;
     static constexpr int kPlanes = 4;
     static constexpr uint32_t kIdle = 0x7FFFFFFFu;   // an idle slot works on 2^31 - 1
-    __device__ static __forceinline__ uint32_t qv(const M &m) { return m.pinv; }   // p^-1 mod 2^32
-    __device__ static __forceinline__ W two32(const M &m) { return m.one; }
-    // T = L < 2^48: with m = lo(T) p^-1 mod 2^32, T - m p = 0 (mod 2^32), so
-    // u = hi(T) - hi(m p) exactly, in (-p, 2^17), plus p when negative:
-    // u = T 2^-32 (mod p), u < 2^31
-    __device__ static __forceinline__ W reduce(uint64_t L, uint64_t, W p, uint32_t pinv) {
-        const uint32_t m1 = (uint32_t)L * pinv;
-        const int64_t u = (int64_t)(L >> 32) - (int64_t)(((uint64_t)m1 * p) >> 32);
-        return (W)(u < 0 ? u + p : u);
+    struct __align__(8) Cand {
+        W p;
+        uint32_t q;   // p^-1 mod 2^32
+    };
+    __device__ static __forceinline__ Cand cand(const M &m) { return {m.p, m.pinv}; }
+    __device__ static __forceinline__ W power(const M &m, uint32_t bits) {
+        const uint32_t k = (bits + 31) / 32, down = 32 * k - bits;
+        const W x = m.mont_R_pow(k - 1);
+        return down ? m.mul(x, 1u << (32 - down)) : x;
+    }
+    __device__ static __forceinline__ W div256(const M &m, W x) { return m.mul(x, 1u << 24); }
+    // kTBias (1 + 2^16) mod p
+    __device__ static __forceinline__ W bias(const M &m) { return (W)((uint64_t)kTBias * 65537u % m.p); }
+    // (four digits hold -0x80808080 .. 0x7F7F7F7F)
+    __device__ static __forceinline__ W digits(W w, W p) { return (w > 0x7F7F7F7Fu ? w - p : w) + 0x80808080u; }
+    // T' < 2^48: with m = lo(T') p^-1 mod 2^32, T' - m p = 0 (mod 2^32), so
+    // u = hi(T') - hi(m p) exactly, in (-p, 2^16), plus p when negative:
+    // u = T' 2^-32 (mod p), u < 2^31
+    __device__ static __forceinline__ W reduce(const uint32_t (&t)[2], const Cand &c) {
+        const uint64_t L = (uint64_t)t[0] + ((uint64_t)t[1] << 16);
+        const uint32_t m1 = (uint32_t)L * c.q;
+        const int32_t u = (int32_t)(uint32_t)(L >> 32) - (int32_t)(((uint64_t)m1 * c.p) >> 32);
+        return (W)(u < 0 ? u + (int32_t)c.p : u);
     }
     // s < p and u < 2^31: s u < p 2^32, one canonical round
-    __device__ static __forceinline__ W prod(const M &m, W s, W u) { return m.mul(s, u); }
-    __device__ static __forceinline__ W sq(const M &m, W s) { return m.mul(s, s); }
+    __device__ static __forceinline__ W prod(W s, W u, const Cand &c) { return redc32(s, u, c.p, c.q); }
+    __device__ static __forceinline__ W canon(W s, const Cand &) { return s; }
 };
 
 template <class T>
 struct TcLayout {
-    using W = typename TcClass<T>::W;
-    static constexpr int kPlanes = TcClass<T>::kPlanes;
+    using C = TcClass<T>;
+    using W = typename C::W;
+    static constexpr int kPlanes = C::kPlanes;
     static constexpr int kCands = kTcN / kPlanes;              // candidates per CTA
-    static constexpr int kParts = kTcThreads / kCands;         // threads per candidate in the products
-    static constexpr uint32_t kOffPart = kOffU + kCands * kUStride * sizeof(W);   // running products [parts][cands]
-    static constexpr uint32_t kOffCand = kOffPart + kParts * kCands * sizeof(W);  // p (W) and q (u32) per candidate
-    static constexpr uint32_t kOffCorr = (kOffCand + kCands * 12 + 7) & ~7u;      // Mont(R^corr) [2 programs][cands]
-    static constexpr uint32_t kOffMisc = (kOffCorr + 2 * kCands * sizeof(W) + 15) & ~15u;   // 2 mbarriers, TMEM address, flag
-    // parts that build byte planes; the first one after them computes the
-    // programs' power-of-R corrections meanwhile
-    static constexpr uint32_t kChunk = (kTcBytes / 8 + kParts - 1) / kParts;
-    static constexpr uint32_t kBusy = (kTcBytes / 8 + kChunk - 1) / kChunk;
-    static_assert(kBusy < (uint32_t)kParts, "a part left for the corrections");
-    static constexpr uint32_t kSmemBytes = kOffMisc + 64;
+    static constexpr int kOwn = kCands / 4;                    // running products per thread
+    static constexpr int kParts = kTcWorkers / kCands;         // threads per candidate in the planes
+    // the lanes' products [cands][kUStride], partial products [parts][cands], p and q, Mont(1), Mont(R^corr)
+    // of both programs, the squarings before each lane, all up to it
+    static constexpr uint32_t kUStride = kTcWords + 1;   // odd: column reads hit distinct banks
+    static constexpr uint32_t kOffPart = kOffU + kCands * kUStride * sizeof(W);
+    static constexpr uint32_t kOffCand = kOffPart + kParts * kCands * sizeof(W);
+    static constexpr uint32_t kOffOne = kOffCand + kCands * sizeof(typename C::Cand);
+    static constexpr uint32_t kOffCorr = kOffOne + kCands * sizeof(W);
+    static constexpr uint32_t kOffSq = kOffCorr + 2 * kCands * sizeof(W);
+    static constexpr uint32_t kOffBar = kOffSq + 2 * (kTcWords + 1) * 4 + 8;
+    static constexpr uint32_t kBars = 2 * kStages + 4 + 1;
+    static constexpr uint32_t kOffMisc = kOffBar + 8 * kBars;   // failed, TMEM address
+    static constexpr uint32_t kSmemBytes = kOffMisc + 16;
+    static constexpr uint32_t kGroupsK = (kTcDigits + 7) / 8;   // groups of 8 elements with digits
+    static constexpr uint32_t kChunk = (kGroupsK + kParts - 1) / kParts;
     static_assert(kSmemBytes <= 227 * 1024, "setup_tc shared memory");
-    static_assert(kCands % 32 == 0 && (kParts & (kParts - 1)) == 0,
-                  "a part of the products is whole warps: part 0 holds the warp that issues the MMAs");
+    static_assert(kOffBar % 8 == 0 && kOffCand % 16 == 0, "setup_tc alignment");
+    static_assert(kOwn * kPlanes == 64, "two loads of 32 columns a tile");
 };
 
 }  // namespace
 
 // One thread per word slot of a tile: the 1792-bit word (the product of a
-// pair of 896-bit words, or one alone; zero past the end) as 224 fp16 bytes
-// in the tile's shared-memory image.  The product is formed column by column
-// in radix 2^28 (a column sums at most 32 products of 28-bit limbs, below
-// 2^61 with its carry) and written eight bytes at a time.
+// pair of 896-bit words, one alone, or 1) as fp16 digits in
+// the tile's shared-memory image.  The product is formed column by column in
+// radix 2^28 (a column sums at most 32 products of 28-bit limbs, below 2^61
+// with its carry) and written eight digits at a time (adding 128 to every
+// byte makes the bytes of the sum the balanced digits plus 128).
 __global__ void tc_pack_kernel(const WideWord *words, const uint32_t *src, uint32_t nw, uint32_t ntiles, uint4 *out) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ntiles * kTcWords) return;
     const uint32_t tile = i / kTcWords, slot = i % kTcWords;
     uint32_t x[kWideLimbs], y[kWideLimbs];
-    const bool have = i < nw;
-    const uint32_t s = have ? __ldg(src + i) : 0u;
-    const bool pair = have && (s >> 31);
+    const uint32_t s = i < nw ? __ldg(src + i) : kTcOne;
+    const bool have = s != kTcOne, pair = have && (s >> 31);
     const uint32_t w = s & 0x7FFFFFFFu;
 #pragma unroll
     for (int k = 0; k < kWideLimbs; ++k) {
-        x[k] = have ? words[w].limb[k] : 0u;
+        x[k] = have ? words[w].limb[k] : (k == 0 ? 1u : 0u);
         y[k] = pair ? words[w + 1].limb[k] : (k == 0 ? 1u : 0u);
     }
     unsigned char *tb = reinterpret_cast<unsigned char *>(out) + (size_t)tile * kATile;
-    uint64_t carry = 0, bits = 0;
+    auto row = [&](uint32_t k8) {
+        constexpr uint32_t per = kStageK / 8;
+        return reinterpret_cast<uint4 *>(tb + (k8 / per) * kStageBytes + tile_off(slot, k8 % per, kStageGroup));
+    };
+    uint64_t carry = 0, bits = 0, up = 0;
     int nbits = 0;
     uint32_t k8 = 0;
     for (int c = 0; c < 2 * kWideLimbs; ++c) {
@@ -271,7 +266,9 @@ __global__ void tc_pack_kernel(const WideWord *words, const uint32_t *src, uint3
         // 28 new bits above the nbits (< 64) already gathered
         bits |= limb << nbits;
         if (nbits + kWideRadixBits >= 64) {   // 64 bits complete
-            *reinterpret_cast<uint4 *>(tb + tile_off(slot, k8++)) = f16x8(bits);
+            const uint64_t sum = bits + 0x8080808080808080ull + up;
+            up = sum < bits ? 1u : 0u;
+            *row(k8++) = f16x8(sum);
             const int used = 64 - nbits;      // bits of this limb in the completed group
             bits = used < kWideRadixBits ? limb >> used : 0;
             nbits = kWideRadixBits - used;
@@ -279,329 +276,276 @@ __global__ void tc_pack_kernel(const WideWord *words, const uint32_t *src, uint3
             nbits += kWideRadixBits;
         }
     }
+    // the last carry, the bias's 4096, the offset's 1
+    *row(k8++) = make_uint4((up ? 0x3C00u : 0u) | 0x6C000000u, 0x3C00u, 0u, 0u);
+    *row(k8) = make_uint4(0u, 0u, 0u, 0u);
 }
 
+// What bounds it: the CUDA cores' multiply pipe, which the ten (class 32:
+// three) wide multiplies per word and candidate keep busy 79% of the time; the
+// tensor cores, 15 MMAs of 128 cycles a tile, are at 65 to 74%.  A tile takes
+// about 2,950 cycles (class 64, 20,330 words x 144,000 candidates: 3.96 ms;
+// unsigned bytes in two accumulators a plane, one buffer of sums and barriers
+// around each tile took 8.01 ms), 2,600 in class 32 (1.69 ms, before 3.59);
+// a CTA's fixed part, planes, first tile and the final tree, about 18,000.
 template <class T>
 __global__ void __launch_bounds__(kTcThreads, 1)
     setup_tc_kernel(ClassBuf<typename TcClass<T>::W> c, SetupArgs<WideWord> a, TcTiles ta, TcTiles tb,
-                    uint32_t *flags, uint32_t block0) {
+                    uint32_t *flags, uint32_t block0, uint32_t radix) {
     using C = TcClass<T>;
     using Lay = TcLayout<T>;
     using W = typename C::W;
-    constexpr int kCands = Lay::kCands, kParts = Lay::kParts, kPlanes = Lay::kPlanes;
+    using Cand = typename C::Cand;
+    constexpr int kCands = Lay::kCands, kParts = Lay::kParts, kPlanes = Lay::kPlanes, kOwn = Lay::kOwn;
     extern __shared__ __align__(1024) unsigned char sm[];
-    const uint32_t tid = threadIdx.x, warp = tid / 32;
+    const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     const uint32_t cnt = min(*c.count, c.cap);
     const uint32_t c0 = (blockIdx.x + block0) * kCands;
     if (c0 >= cnt) return;   // whole CTA idle
 
     W *U = reinterpret_cast<W *>(sm + kOffU);
     W *part = reinterpret_cast<W *>(sm + Lay::kOffPart);
-    W *cand_p = reinterpret_cast<W *>(sm + Lay::kOffCand);
-    uint32_t *cand_q = reinterpret_cast<uint32_t *>(sm + Lay::kOffCand + kCands * 8);
-    uint64_t *mbar_mma = reinterpret_cast<uint64_t *>(sm + Lay::kOffMisc);
-    uint64_t *mbar_load = reinterpret_cast<uint64_t *>(sm + Lay::kOffMisc + 8);
-    uint32_t *taddr_slot = reinterpret_cast<uint32_t *>(sm + Lay::kOffMisc + 16);
-    uint32_t *timeout = reinterpret_cast<uint32_t *>(sm + Lay::kOffMisc + 20);
+    Cand *cands = reinterpret_cast<Cand *>(sm + Lay::kOffCand);
+    W *ones = reinterpret_cast<W *>(sm + Lay::kOffOne);
     W *corr_pow = reinterpret_cast<W *>(sm + Lay::kOffCorr);
+    uint32_t *lane_sq = reinterpret_cast<uint32_t *>(sm + Lay::kOffSq);   // squarings before a lane, of one program
+    uint32_t *all_sq = lane_sq + kTcWords;                                // up to and before it [kTcWords + 1]
+    uint32_t *misc = reinterpret_cast<uint32_t *>(sm + Lay::kOffMisc);
+    volatile uint32_t *failed = misc;
+    const uint32_t fail = smem_u32(misc);
+    uint32_t *taddr_slot = misc + 1;
+    const uint32_t bar = smem_u32(sm + Lay::kOffBar);
+    auto bar_full = [&](uint32_t s) { return bar + 8 * s; };                       // a part of a tile landed
+    auto bar_free = [&](uint32_t s) { return bar + 8 * (kStages + s); };           // and multiplied
+    auto bar_ready = [&](uint32_t b) { return bar + 8 * (2 * kStages + b); };      // a buffer's sums ready
+    auto bar_read = [&](uint32_t b) { return bar + 8 * (2 * kStages + 2 + b); };   // and read
+    const uint32_t bar_end = bar + 8 * (2 * kStages + 4);
 
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(taddr_slot)),
-                     "r"(kTmemCols)
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(taddr_slot))
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar_mma)) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar_load)) : "memory");
-        *timeout = 0;
-    }
-
-    // this thread's candidate and part: kParts threads per candidate (part 0
-    // holds the accumulator)
-    const uint32_t cl = tid % kCands, prt = tid / kCands;
-    const uint32_t ci = c0 + cl;
-    const bool act = ci < cnt;
-    typename C::M m;
-    m.init(act ? c.p[ci] : (W)C::kIdle);
-    if (prt == 0) {
-        cand_p[cl] = m.p;
-        cand_q[cl] = C::qv(m);
-    }
-
-    // bias tiles: A column 0 = 2048, B column 0 = 4096 (fp16), the rest 0
-    for (uint32_t r = tid; r < kTcWords + kTcN; r += kTcThreads) {
-        const bool isa = r < kTcWords;
-        const uint32_t row = isa ? r : r - kTcWords;
-        unsigned char *base = sm + (isa ? kOffABias : kOffBBias);
-        *reinterpret_cast<uint4 *>(base + tile_off(row, 0, kBiasRowGroup)) =
-            make_uint4(isa ? 0x6800u : 0x6C00u, 0, 0, 0);
-        *reinterpret_cast<uint4 *>(base + tile_off(row, 1, kBiasRowGroup)) = make_uint4(0, 0, 0, 0);
-    }
-
-    // B operand: the candidate's residues w_b = 2^(8b+32) mod p as byte
-    // planes, rows kPlanes c .. kPlanes c + kPlanes - 1 (each part writes its
-    // share of the 28 groups of 8 bytes, starting from 2^32 256^b0 mod p by
-    // square-and-multiply; the plane order is rotated by the candidate so
-    // that a warp's stores spread over the banks)
-    {
-        constexpr uint32_t kChunk = Lay::kChunk;
-        const uint32_t k8a = min(prt * kChunk, (uint32_t)(kTcBytes / 8)),
-                       k8b = min(k8a + kChunk, (uint32_t)(kTcBytes / 8));
-        const W c256 = m.to_mont(256);
-        W x = C::two32(m);
-        {
-            W pw = m.one, base = c256;
-            for (uint32_t e = 8 * k8a; e; e >>= 1) {
-                if (e & 1) pw = m.mul(pw, base);
-                base = m.mul(base, base);
-            }
-            x = m.mul(x, pw);
+        for (uint32_t s = 0; s < 2 * kStages; ++s) mbar_init(bar + 8 * s, 1);
+        for (uint32_t b = 0; b < 2; ++b) {
+            mbar_init(bar_ready(b), 1);
+            mbar_init(bar_read(b), kTcWorkers / 32);
         }
-        for (uint32_t k8 = k8a; k8 < k8b; ++k8) {
+        mbar_init(bar_end, 1);
+        *failed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tbase = *taddr_slot;
+    const int nprog = a.mode == (PFC_FACTORIAL | PFC_COMPOSITORIAL) ? 2 : 1;
+    const uint32_t ntiles = ta.ntiles + (nprog == 2 ? tb.ntiles : 0u);
+
+    // a part of tile t (none after a wait that gave up: a copy may then still
+    // be pending on its barrier)
+    auto load = [&](uint32_t t, uint32_t s) {
+        const unsigned char *src = reinterpret_cast<const unsigned char *>(t < ta.ntiles ? ta.tiles : tb.tiles) +
+                                   (size_t)(t < ta.ntiles ? t : t - ta.ntiles) * kATile + s * kStageBytes;
+        if (elect() && !*failed) copy_in(smem_u32(sm + kOffA) + s * kStageBytes, src, kStageBytes, bar_full(s));
+        __syncwarp();
+    };
+
+    // this thread's candidate while the planes are built, kParts threads each
+    const uint32_t cl = tid % kCands, prt = tid / kCands, ci = c0 + cl;
+    const bool act = tid < (uint32_t)kTcWorkers && ci < cnt;
+    typename C::M m;
+    if (tid < (uint32_t)kTcWorkers) {
+        m.init(act ? c.p[ci] : (W)C::kIdle);
+        if (prt == 0) {
+            cands[cl] = C::cand(m);
+            ones[cl] = m.one;
+        }
+        // w_b = 2^(8b+32) mod p as planes, rows kPlanes c .. kPlanes c + kPlanes
+        // - 1: each part writes its share of the groups of 8 digits, from the
+        // last digit down, w_b = w_(b+1) / 256
+        const uint32_t k8a = min(prt * Lay::kChunk, Lay::kGroupsK), k8b = min(k8a + Lay::kChunk, Lay::kGroupsK);
+        W x = k8a < k8b ? C::power(m, 8 * min(8 * k8b - 1, kTcDigits - 1) + 32) : 0;
+        unsigned char *rows = sm + kOffB;
+        for (uint32_t k8 = k8b; k8-- > k8a;) {
+            const bool tail = k8 == kTcDigits / 8;   // one digit, the bias, the offset
             W w[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                w[j] = x;
-                x = m.mul(x, c256);
+            for (int j = 7; j >= 0; --j) {
+                w[j] = C::digits(x, m.p);
+                if (!tail || j == 0) x = C::div256(m, x);
+            }
+            if (tail) {
+#pragma unroll
+                for (int j = 1; j < 8; ++j) w[j] = C::digits(0, m.p);
+                const W off = C::bias(m);
+                w[2] = C::digits(off ? m.p - off : 0, m.p);
             }
 #pragma unroll
-            for (int r = 0; r < kPlanes; ++r) {
-                const int pl = (r + (int)cl) % kPlanes;
-                uint64_t bytes = 0;
+            for (int h = 0; h < kPlanes / 4; ++h) {
+                uint32_t lo[4], hi[4];
+                transpose4((uint32_t)(w[0] >> (32 * h)), (uint32_t)(w[1] >> (32 * h)), (uint32_t)(w[2] >> (32 * h)),
+                           (uint32_t)(w[3] >> (32 * h)), lo);
+                transpose4((uint32_t)(w[4] >> (32 * h)), (uint32_t)(w[5] >> (32 * h)), (uint32_t)(w[6] >> (32 * h)),
+                           (uint32_t)(w[7] >> (32 * h)), hi);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) bytes |= (uint64_t)((w[j] >> (8 * pl)) & 0xFFu) << (8 * j);
-                *reinterpret_cast<uint4 *>(sm + kOffB + tile_off(kPlanes * cl + pl, k8)) = f16x8(bytes);
+                for (int r = 0; r < 4; ++r) {
+                    uint4 v = f16x8(lo[r] | ((uint64_t)hi[r] << 32));
+                    if (tail) v.x = (v.x & 0xFFFFu) | 0x6A000000u;   // 3072
+                    *reinterpret_cast<uint4 *>(rows + tile_off(kPlanes * cl + 4 * h + r, k8, kRowGroup)) = v;
+                }
             }
         }
+        if (prt == (uint32_t)kParts - 1) {   // (the shortest share)
+#pragma unroll
+            for (int pl = 0; pl < kPlanes; ++pl)
+                *reinterpret_cast<uint4 *>(rows + tile_off(kPlanes * cl + pl, kTcK / 8 - 1, kRowGroup)) =
+                    make_uint4(0u, 0u, 0u, 0u);
+            // the programs' power-of-R corrections
+            for (int pi = 0; pi < nprog; ++pi) corr_pow[pi * kCands + cl] = m.mont_R_pow((pi == 0 ? a.a : a.b).corr);
+        }
+    } else if (warp == kTcThreads / 32 - 1) {
+        for (uint32_t s = 0; s < kStages && ntiles; ++s) load(0, s);
     }
-
-    // the power-of-R corrections Mont(R^corr) of the programs, on the part(s)
-    // that build no byte planes (read by part 0 at the end of each program)
-    const int nprog0 = a.mode == (PFC_FACTORIAL | PFC_COMPOSITORIAL) ? 2 : 1;
-    for (int pi = 0; pi < nprog0; ++pi)
-        if (prt == Lay::kBusy + ((uint32_t)pi % (kParts - Lay::kBusy)))
-            corr_pow[pi * kCands + cl] = m.mont_R_pow((pi == 0 ? a.a : a.b).corr);
-
-    const uint32_t quad = warp % 4, wgroup = warp / 4;      // TMEM lane quadrant, warp group
-    const uint32_t word = quad * 32 + (tid % 32);           // this thread's word of a tile
-    // f32 <- f16 x f16, both K-major, N = 256, M = 128
-    const uint32_t idesc = (1u << 4) | ((uint32_t)(kTcN >> 3) << 17) | ((uint32_t)(kTcWords >> 4) << 24);
-    const int nprog = a.mode == (PFC_FACTORIAL | PFC_COMPOSITORIAL) ? 2 : 1;
-
-    // tile i of program pi into the A region (one thread), completing on mbar_load
-    auto load_tile = [&](int pi, uint32_t i) {
-        const TcTiles &tt = pi == 0 ? ta : tb;
-        const unsigned char *src = reinterpret_cast<const unsigned char *>(tt.tiles) + (size_t)i * kATile;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(mbar_load)),
-                     "r"(kATile)
-                     : "memory");
-        asm volatile(
-            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                smem_u32(sm + kOffA)),
-            "l"(src), "r"(kATile), "r"(smem_u32(mbar_load))
-            : "memory");
-    };
-    // the tile's products: per half of the bytes, a bias product and seven
-    // K-steps into that half's 256 columns
-    auto issue_mma = [&](uint32_t tbase) {
-        const uint32_t aaddr = smem_u32(sm + kOffA), baddr = smem_u32(sm + kOffB),
-                       abias = smem_u32(sm + kOffABias), bbias = smem_u32(sm + kOffBBias);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t d = tbase + h * kTcN;
-            asm volatile(
-                "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, 0, 0;\n\t"
-                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
-                "l"(mdesc(abias, kBiasRowGroup)), "l"(mdesc(bbias, kBiasRowGroup)), "r"(idesc)
-                : "memory");
-#pragma unroll
-            for (int s = 0; s < kTcHalfBytes / 16; ++s) {
-                const uint32_t off = (uint32_t)(h * (kTcHalfBytes / 16) + s) * 256;
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, 1, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
-                    "l"(mdesc(aaddr + off, kRowGroup)), "l"(mdesc(baddr + off, kRowGroup)), "r"(idesc)
-                    : "memory");
-            }
-        }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                         smem_u32(mbar_mma))
-                     : "memory");
-    };
-    // the tile after tile i of program pi, across programs; false at the end
-    auto next_tile = [&](int &pi, uint32_t &i, bool started) -> bool {
-        for (;;) {
-            if (pi >= nprog) return false;
-            const uint32_t t = started ? i + 1 : 0;
-            if (t < (pi == 0 ? ta : tb).ntiles) {
-                i = t;
-                return true;
-            }
-            ++pi;
-            started = false;
-        }
-    };
-
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    sync_tc();
-    const uint32_t tbase = *taddr_slot;
-    const uint32_t taddr = tbase + ((quad * 32u) << 16);    // this warp's TMEM lanes
+    __syncthreads();
 
-    uint32_t par_mma = 0, par_load = 0;
-    bool failed = false;
-    W s0 = 0, s1 = 0;
-    W P[kTcChains];          // this part's running products (part 0, chain 0: the accumulator)
+    if (warp == kTcWorkers / 32) {
+        // ------------------------------------------------------------- MMAs
+        const uint32_t tb2 = __shfl_sync(kFull, tbase, 0);
+        const uint64_t da = mdesc(smem_u32(sm + kOffA), kStageGroup), db = mdesc(smem_u32(sm + kOffB), kRowGroup);
+        for (uint32_t t = 0; t < ntiles; ++t) {
+            const uint32_t buf = t & 1;
+            if (t >= 2) warp_wait(bar_read(buf), ((t >> 1) - 1) & 1, fail);
+#pragma unroll 1
+            for (uint32_t s = 0; s < kStages; ++s) {
+                warp_wait(bar_full(s), t & 1, fail);
+                fence_after();
+                const uint64_t pa = da + s * (kStageBytes / 16), pb = db + s * (kStageK / 8 * 128 / 16);
+                if (elect()) {
 #pragma unroll
-    for (int k = 0; k < kTcChains; ++k) P[k] = m.one;
-    uint32_t g = 0;          // first group of the current program whose squarings are still due
-    int fin = 0;             // programs finished
-
-    // the threads' products into part 0's accumulator, a tree over the parts
-    // (uniform: every thread calls it)
-    auto combine = [&]() {
-#pragma unroll
-        for (int k = 1; k < kTcChains; ++k) {
-            P[0] = C::prod(m, P[0], P[k]);
-            P[k] = m.one;
-        }
-#pragma unroll
-        for (uint32_t stride = 1; stride < (uint32_t)kParts; stride <<= 1) {
-            part[prt * kCands + cl] = P[0];
-            __syncthreads();
-            if ((prt & (2 * stride - 1)) == 0) P[0] = C::prod(m, P[0], part[(prt + stride) * kCands + cl]);
-            __syncthreads();
-        }
-        if (prt != 0) P[0] = m.one;
-    };
-    // end of program pi: remaining squarings, the power-of-R correction,
-    // result; the combined search's second program (primorial words)
-    // continues from the first's result, so part 0 keeps it
-    auto finish = [&](int pi) {
-        const Prog<WideWord> &pg = pi == 0 ? a.a : a.b;
-        combine();
-        if (prt == 0) {
-            W acc = P[0];
-            for (; g < pg.ngroups; ++g)
-                for (uint32_t k = __ldg(pg.groups + 3 * g + 2); k > 0; --k) acc = C::sq(m, acc);
-            for (uint32_t k = 0; k < pg.final_sq; ++k) acc = C::sq(m, acc);
-            acc = m.mul(acc, corr_pow[pi * kCands + cl]);
-            if (nprog == 2 && pi == 0) s1 = acc;
-            else s0 = acc;
-            P[0] = acc;
-        }
-        g = 0;
-    };
-
-    int cpi = 0;
-    uint32_t ci_t = 0;
-    bool have = next_tile(cpi, ci_t, false);
-    if (have && tid == 0) {
-        load_tile(cpi, ci_t);
-        if (!mbar_wait(smem_u32(mbar_load), par_load)) *timeout = 1;
-        else issue_mma(tbase);
-    }
-    par_load ^= 1;
-    while (have) {
-        if (!mbar_wait(smem_u32(mbar_mma), par_mma)) atomicOr(timeout, 1u);
-        par_mma ^= 1;
-        sync_tc();
-        if (*timeout) {
-            failed = true;
-            break;
-        }
-        int npi = cpi;
-        uint32_t ni_t = ci_t;
-        const bool nhave = next_tile(npi, ni_t, true);
-        if (nhave && tid == 0) load_tile(npi, ni_t);   // the A region is free: the products are done
-        // 1. u = T 2^-32 (mod p) for this thread's word and its warp group's candidates
-        constexpr int kPerLoad = 32 / kPlanes;   // candidates per 32-column load
-        for (uint32_t cc = wgroup * (kCands / kTcGroups); cc < (wgroup + 1) * (kCands / kTcGroups); cc += kPerLoad) {
-            uint32_t v0[32], v1[32];
-            ld32(taddr, kPlanes * cc, v0);
-            ld32(taddr, kTcN + kPlanes * cc, v1);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-            for (int j = 0; j < kPerLoad; ++j) {
-                // plane sums e_a = D_{a,0} + D_{a,1} - 2^24 < 2^24 (the two bias
-                // patterns add to 2 x 0x4B000000 < 2^32)
-                uint32_t e[8];
-#pragma unroll
-                for (int pl = 0; pl < 8; ++pl)
-                    e[pl] = pl < kPlanes ? v0[kPlanes * j + pl] + v1[kPlanes * j + pl] - 2u * kBiasBits : 0u;
-                // T = L + 2^32 H
-                const uint64_t L = (uint64_t)e[0] + ((uint64_t)e[1] << 8) + ((uint64_t)e[2] << 16) +
-                                   ((uint64_t)e[3] << 24);
-                const uint64_t H = (uint64_t)e[4] + ((uint64_t)e[5] << 8) + ((uint64_t)e[6] << 16) +
-                                   ((uint64_t)e[7] << 24);
-                const uint32_t cj = cc + j;
-                U[cj * kUStride + word] = C::reduce(L, H, cand_p[cj], cand_q[cj]);
+                    for (uint32_t k = 0; k < kStageK / 16; ++k)
+                        mma_smem(tb2 + buf * kTcN, pa + k * 16, pb + k * 16, idesc_n(kTcN), s != 0 || k != 0);
+                    commit(bar_free(s));
+                    if (s == kStages - 1) commit(bar_ready(buf));
+                }
+                __syncwarp();
             }
         }
-        // 2. the next tile's products (TMEM is free once every thread's loads
-        //    above are complete; the bulk copy has had step 1 to land)
-        sync_tc();
-        if (nhave && tid == 0) {
-            if (!mbar_wait(smem_u32(mbar_load), par_load)) *timeout = 1;   // seen after the next wait
-            else issue_mma(tbase);
-        }
-        if (nhave) par_load ^= 1;
-        while (fin < cpi) finish(fin++);   // programs without words
-        // 3. the tile's u into the running products, in segments between the
-        //    group starts inside the tile
-        {
-            const Prog<WideWord> &pg = cpi == 0 ? a.a : a.b;
-            uint32_t first, end;
-            prog_range(pg, first, end);
-            const uint32_t t0 = first + ci_t * kTcWords, t1 = min(t0 + kTcWords, end);
-            uint32_t s = t0;
-            for (;;) {
-                uint32_t k = 0;
-                for (; g < pg.ngroups && __ldg(pg.groups + 3 * g) <= s; ++g) k += __ldg(pg.groups + 3 * g + 2);
-                // a group start's squarings, applied by every thread to each of
-                // its running products: the accumulator is their Montgomery
-                // product A = P_0 (x) ... (x) P_{n-1} = (prod P) R^-(n-1), and
-                // squaring each, P (x) P = P^2 R^-1, gives (prod P)^2 R^-(2n-1)
-                // = A (x) A, so no combining is needed until the program ends
-                for (; k > 0; --k) {
+        // every MMA has ended before the CTA does
+        if (elect()) commit(bar_end);
+        __syncwarp();
+        ended(bar_end, 0);
+    } else if (warp > kTcWorkers / 32) {
+        // ----------------------------------------------------------- copies
+        for (uint32_t t = 1; t < ntiles; ++t)
+            for (uint32_t s = 0; s < kStages; ++s) {
+                warp_wait(bar_free(s), (t - 1) & 1, fail);
+                load(t, s);
+            }
+    } else {
+        // ---------------------------------------------------------- workers
+        const uint32_t quad = warp % 4, own = warp / 4 * kOwn;   // TMEM lane quadrant, first candidate
+        const uint32_t taddr = tbase + ((quad * 32u) << 16) + own * kPlanes;
+        W s0 = 0, s1 = 0;
+        uint32_t t = 0;
+        for (int pi = 0; pi < nprog; ++pi) {
+            const Prog<WideWord> &pg = pi == 0 ? a.a : a.b;
+            const uint32_t tend = t + (pi == 0 ? ta.ntiles : tb.ntiles);
+            W P[kOwn];   // the lane's running products, Montgomery form up to a power of R per word
 #pragma unroll
-                    for (int c2 = 0; c2 < kTcChains; ++c2) P[c2] = C::sq(m, P[c2]);
-                }
-                // the words go to parts 1.. : part 0 is warp 0, whose first
-                // thread has just issued the next tile's products (it waits
-                // while the tensor pipe takes them) and holds the accumulator
-                const uint32_t e = g < pg.ngroups ? min(t1, __ldg(pg.groups + 3 * g)) : t1;
-                const uint32_t span = (e - s + kParts - 2) / (kParts - 1);
-                const uint32_t lo = prt ? min(s + span * (prt - 1), e) : e, hi = prt ? min(lo + span, e) : e;
-                const W *row = U + cl * kUStride + (lo - t0);
-                const uint32_t n = hi - lo;
-                uint32_t i = 0;
-                for (; i + kTcChains <= n; i += kTcChains) {
+            for (int k = 0; k < kOwn; ++k) P[k] = ones[own + k];
+            for (; t < tend; ++t) {
+                const uint32_t buf = t & 1;
+                warp_wait(bar_ready(buf), (t >> 1) & 1, fail);
+                fence_after();
+                // 32 sums at a time
 #pragma unroll
-                    for (int k = 0; k < kTcChains; ++k) P[k] = C::prod(m, P[k], row[i + k]);
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t v[32];
+                    ld32(taddr + buf * kTcN + 32 * h, v);
+                    wait_ld();
+                    if (h == 1) {
+                        fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar_read(buf));
+                    }
+#pragma unroll
+                    for (int j = 0; j < 32 / kPlanes; ++j) {
+                        const Cand cd = cands[own + h * (kOwn / 2) + j];
+                        uint32_t tj[kPlanes / 2];
+#pragma unroll
+                        for (int k = 0; k < kPlanes / 2; ++k)   // (radix: 256, kept from becoming a shift)
+                            tj[k] = v[kPlanes * j + 2 * k + 1] * radix + v[kPlanes * j + 2 * k];
+                        W &y = P[h * (kOwn / 2) + j];
+                        y = C::prod(y, C::reduce(tj, cd), cd);
+                    }
                 }
-                for (; i < n; ++i) P[0] = C::prod(m, P[0], row[i]);
-                s = e;
-                if (s >= t1) break;
+            }
+            // the program's end: the lanes' products through shared memory, each
+            // thread those of a share of the lanes of its own candidate, then a
+            // tree over the shares; left of a group start go its squarings
+#pragma unroll
+            for (int k = 0; k < kOwn; ++k) U[(own + k) * Lay::kUStride + quad * 32 + lane] = P[k];
+            if (tid < kTcWords) {
+                uint32_t sq = 0;
+                for (uint32_t g = 0; g < pg.ngroups; ++g)
+                    if (__ldg(pg.groups + 3 * g) == tid) sq += __ldg(pg.groups + 3 * g + 2);
+                lane_sq[tid] = sq;
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(kTcWorkers) : "memory");
+            if (tid <= kTcWords) {
+                uint32_t sq = 0;
+                for (uint32_t k = 0; k < tid; ++k) sq += lane_sq[k];
+                all_sq[tid] = sq;
+            }
+            constexpr uint32_t kShare = kTcWords / kParts;
+            const Cand cd = C::cand(m);
+            auto square = [&](W y, uint32_t n) {
+                for (; n; --n) {
+                    y = C::canon(y, cd);
+                    y = C::prod(y, y, cd);
+                }
+                return y;
+            };
+            const W *row = U + cl * Lay::kUStride + prt * kShare;
+            W acc = row[0];
+            for (uint32_t k = 1; k < kShare; ++k)
+                acc = C::prod(square(acc, lane_sq[prt * kShare + k]), C::canon(row[k], cd), cd);
+            for (uint32_t n = 1; n < (uint32_t)kParts; n <<= 1) {
+                part[prt * kCands + cl] = acc;
+                asm volatile("bar.sync 1, %0;" ::"n"(kTcWorkers) : "memory");
+                if ((prt & (2 * n - 1)) == 0)
+                    acc = C::prod(square(acc, all_sq[(prt + 2 * n) * kShare] - all_sq[(prt + n) * kShare]),
+                                  C::canon(part[(prt + n) * kCands + cl], cd), cd);
+            }
+            if (prt == 0) {
+                // the combined search's second program (primorial words)
+                // continues from the first's result
+                if (pi) acc = C::prod(square(s1, all_sq[kTcWords]), C::canon(acc, cd), cd);
+                acc = C::canon(square(acc, pg.final_sq), cd);
+                acc = m.mul(acc, corr_pow[pi * kCands + cl]);
+                if (nprog == 2 && pi == 0) s1 = acc;
+                else s0 = acc;
             }
         }
-        if (!nhave || npi != cpi) finish(fin++);
-        cpi = npi;
-        ci_t = ni_t;
-        have = nhave;
+        if (tid < (uint32_t)kCands && act && !*failed) {
+            c.s0[ci] = s0;
+            c.s1[ci] = s1;
+            c.nnext[ci] = a.nnext0;
+        }
     }
-    if (!failed)
-        while (fin < nprog) finish(fin++);
-
-    sync_tc();
-    if (failed) {
-        if (tid == 0) atomicOr(flags, 2u);
-    } else if (prt == 0 && act) {
-        c.s0[ci] = s0;
-        c.s1[ci] = s1;
-        c.nnext[ci] = a.nnext0;
-    }
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(kTmemCols) : "memory");
+    __syncwarp();
+    // (copies still in flight after a wait that gave up; else each was waited for)
+    if (*failed)
+        for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+    fence_before();
+    __syncthreads();
+    fence_after();
+    if (tid == 0 && *failed) atomicOr(flags, 2u);
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tbase) : "memory");
 }
 
 size_t tc_tile_bytes() { return kATile; }
@@ -615,8 +559,8 @@ int launch_tc_pack(const WideWord *words, const uint32_t *src, uint32_t nw, uint
     return 1;
 }
 
-// One CTA of 512 threads per 32 (class 64) or 64 (class 32) candidates, one
-// CTA per SM (shared memory); blocks [block0, block0 + nblocks) of the class
+// One CTA per 32 (class 64) or 64 (class 32) candidates, one
+// CTA per SM (shared memory, TMEM); blocks [block0, block0 + nblocks) of the class
 // buffer (nblocks 0: to the end).
 uint32_t tc_setup_blocks(uint32_t cands) { return (cands + TcLayout<Cls64L>::kCands - 1) / TcLayout<Cls64L>::kCands; }
 uint32_t tc_setup_blocks32(uint32_t cands) { return (cands + TcLayout<Cls32>::kCands - 1) / TcLayout<Cls32>::kCands; }
@@ -638,7 +582,7 @@ static int launch_tc(const ClassBuf<typename TcClass<T>::W> &c, const SetupArgs<
             return 0;
         configured[dev] = true;
     }
-    setup_tc_kernel<T><<<nblocks, kTcThreads, TcLayout<T>::kSmemBytes, st>>>(c, a, ta, tb, flags, block0);
+    setup_tc_kernel<T><<<nblocks, kTcThreads, TcLayout<T>::kSmemBytes, st>>>(c, a, ta, tb, flags, block0, 256u);
     return 1;
 }
 
