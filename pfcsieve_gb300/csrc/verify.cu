@@ -146,10 +146,18 @@ int slow_products(pfc_ctx *c, uint64_t lo, uint64_t hi, SlowProducts &out) {
 // type's start value (34!, 101#, 44!/44#) times every k in [35, n] (type 0),
 // times the primes in [103, n] or the composites in [45, n] (the list of the
 // search's mode, as the CPU check builds it) -- must be +1 or -1 modulo p with
-// the hit's sign.  One CTA of 256 threads per hit: each thread multiplies a
-// contiguous sub-range of k as plain multipliers in four chains (one
-// reduction each, the power of R fixed once at the end), and the threads'
-// products are combined by shuffles and through shared memory.
+// the hit's sign.  One CTA of 256 threads per hit, a contiguous share of the
+// range per thread, the threads' products combined by shuffles and through
+// shared memory, the power of R fixed once.  Below 2^31 the arithmetic is
+// 32-bit.
+//
+// What bounds it is the multiply pipe, where a wide multiply takes four times
+// as long as a plain one, so the reductions per k are what counts.  Every k:
+// the products of D consecutive k are a polynomial of degree D in the first,
+// tabulated by finite differences, D modular additions and one product for D
+// of them (D = 4 below 2^31, 8 above).  Composites: above 2^31 two of them in
+// one 64-bit word.  Primes: from the set bits of the flags.  With one 64-bit
+// product per k, 9,221 hits of n up to 200,000 took 2.40 ms, now 0.33 ms.
 // Nothing here uses the sieve's tables or its walk, so the check is
 // independent of the arithmetic it checks.
 
@@ -162,51 +170,143 @@ struct VerifyRec {
     int32_t sign;
 };
 
-__global__ void __launch_bounds__(256) verify_hits_kernel(const VerifyRec *r, uint32_t cnt, const uint32_t *primebits,
-                                                          uint8_t *bad) {
-    __shared__ uint64_t part[8];
-    if (blockIdx.x >= cnt) return;   // whole blocks
-    const VerifyRec h = r[blockIdx.x];
-    const uint32_t t = threadIdx.x;
-    Mont64 m;
-    m.init(h.p);
-    uint64_t a0 = m.one, a1 = m.one, a2 = m.one, a3 = m.one;
-    uint32_t taken = 0;
-    if (h.what != 3 && h.hi >= h.lo) {
-        const uint32_t per = (h.hi - h.lo) / blockDim.x + 1;
-        const uint32_t s = h.lo + t * per;   // <= hi + blockDim.x: no wrap below 2^31 + 256
-        const uint32_t e = s <= h.hi ? min(s + per, h.hi + 1) : s;
-        uint32_t k = s;
-        if (h.what == 0) {
-            for (; k + 3 < e; k += 4) {
-                a0 = redc64(a0, k, m.p, m.pinv);
-                a1 = redc64(a1, k + 1, m.p, m.pinv);
-                a2 = redc64(a2, k + 2, m.p, m.pinv);
-                a3 = redc64(a3, k + 3, m.p, m.pinv);
+// what the two sizes of p differ in: the Montgomery arithmetic (a product by a
+// plain k lowers the power of R by one) and the k per polynomial value
+struct Verify32 {
+    using W = uint32_t;
+    using M = Mont32;
+    static constexpr int D = 4;
+    __device__ static __forceinline__ W sub(W a, W b, W p) {   // a - b mod p: a - b below 0 wraps above a - b + p
+        return min(a - b, a - b + p);
+    }
+    // v k .. (k + D - 1) R^-D
+    __device__ static __forceinline__ W times(const M &m, W v, uint32_t k) {
+#pragma unroll
+        for (int i = 0; i < D; ++i) v = m.mul(v, k + i);
+        return v;
+    }
+    static constexpr uint32_t kUnits = D;   // powers of R that takes off
+};
+struct Verify64 {
+    using W = uint64_t;
+    using M = Mont64;
+    static constexpr int D = 8;
+    __device__ static __forceinline__ W sub(W a, W b, W p) { return a < b ? a - b + p : a - b; }
+    __device__ static __forceinline__ W times(const M &m, W v, uint32_t k) {   // two k, below 2^31, to a word
+#pragma unroll
+        for (int i = 0; i < D; i += 2) v = m.mul(v, (uint64_t)(k + i) * (k + i + 1));
+        return v;
+    }
+    static constexpr uint32_t kUnits = D / 2;
+};
+
+// product of the k in [k, e) (times R^(1 - units)), Montgomery form
+template <class V>
+__device__ typename V::W verify_range(const typename V::M &m, uint32_t k, uint32_t e, uint64_t &units) {
+    using W = typename V::W;
+    constexpr int D = V::D;
+    W acc = m.one;
+    if (e - k >= 8u * D) {
+        // g[j]: j-th difference of f(x) = x .. (x + D - 1) at steps of D, the
+        // odd ones negated so that every update is a subtraction
+        W g[D + 1];
+#pragma unroll
+        for (int j = 0; j <= D; ++j) g[j] = V::times(m, m.one, k + j * D);
+#pragma unroll
+        for (int j = 1; j <= D; ++j)
+#pragma unroll
+            for (int i = D; i >= j; --i) g[i] = V::sub(g[i], g[i - 1], m.p);
+#pragma unroll
+        for (int j = 1; j <= D; j += 2) g[j] = V::sub((W)0, g[j], m.p);
+        const uint32_t n = (e - k) / D;
+        for (uint32_t i = 0; i < n; ++i) {
+            acc = m.mul(acc, g[0]);
+#pragma unroll
+            for (int j = 0; j < D; ++j) g[j] = V::sub(g[j], g[j + 1], m.p);
+        }
+        k += n * D;
+        units += (uint64_t)n * V::kUnits;   // (g is f R^(1 - kUnits), and a product)
+    }
+    units += e - k;
+    for (; k < e; ++k) acc = m.mul(acc, k);
+    return acc;
+}
+
+// the same for the k of words [w, e) of prime flags, primes or composites,
+// within [lo, hi]
+template <class V>
+__device__ typename V::W verify_list(const typename V::M &m, uint32_t w, uint32_t e, uint32_t lo, uint32_t hi,
+                                     bool primes, const uint32_t *bits, uint64_t &units) {
+    using W = typename V::W;
+    W acc[4] = {m.one, m.one, m.one, m.one};
+    for (; w < e; ++w) {
+        const uint32_t base = 32 * w;
+        uint32_t in = primes ? __ldg(bits + w) : ~__ldg(bits + w);
+        if (base < lo) in &= ~0u << (lo - base);
+        if (hi - base < 31) in &= ~0u >> (31 - (hi - base));
+        if (primes) {
+            units += __popc(in);
+            for (; in; in &= in - 1) acc[0] = m.mul(acc[0], base + __ffs(in) - 1);
+        } else {   // 1 in place of a prime
+            constexpr int per = sizeof(W) == 4 ? 1 : 2;
+            units += 32 / per;
+#pragma unroll
+            for (int j = 0; j < 32; j += per) {
+                W k = (in >> j) & 1u ? base + j : 1u;
+                if (per == 2) k *= (in >> (j + 1)) & 1u ? base + j + 1 : 1u;
+                acc[j / per % 4] = m.mul(acc[j / per % 4], k);
             }
-            for (; k < e; ++k) a0 = redc64(a0, k, m.p, m.pinv);
-            taken = e - s;
-        } else {
-            const uint32_t want = h.what == 1 ? 1u : 0u;
-            for (; k < e; ++k)
-                if (((__ldg(primebits + (k >> 5)) >> (k & 31)) & 1u) == want) {
-                    if (taken & 1) a1 = redc64(a1, k, m.p, m.pinv);
-                    else a0 = redc64(a0, k, m.p, m.pinv);
-                    ++taken;
-                }
         }
     }
-    // each reduction by a plain k lowered the power of R by one
-    uint64_t acc = m.mul(m.mul(m.mul(a0, a1), m.mul(a2, a3)), m.mont_R_pow(taken));
-#pragma unroll
-    for (int o = 16; o; o >>= 1) acc = m.mul(acc, __shfl_down_sync(0xffffffffu, acc, o));
-    if ((t & 31) == 0) part[t >> 5] = acc;
-    __syncthreads();
-    if (t == 0) {
-        for (uint32_t i = 1; i < (blockDim.x >> 5); ++i) acc = m.mul(acc, part[i]);
-        const uint64_t v = m.mul(acc, m.to_mont(h.start));
-        bad[blockIdx.x] = h.sign < 0 ? v != m.one : v != m.p - m.one;
+    return m.mul(m.mul(acc[0], acc[1]), m.mul(acc[2], acc[3]));
+}
+
+template <class V>
+__device__ bool verify_hit(const VerifyRec &h, const uint32_t *primebits, typename V::W *part, uint64_t *parts) {
+    using W = typename V::W;
+    const uint32_t t = threadIdx.x;
+    typename V::M m;
+    m.init((W)h.p);
+    W acc = m.one;
+    uint64_t units = 0;
+    if (h.what != 3 && h.hi >= h.lo) {
+        // share t of [lo, hi], or of the words of flags that hold it
+        const uint32_t lo = h.what ? h.lo / 32 : h.lo, hi = h.what ? h.hi / 32 : h.hi;
+        const uint32_t per = (hi - lo) / blockDim.x + 1;
+        const uint32_t s = lo + t * per;   // <= hi + blockDim.x: no wrap below 2^31 + 256
+        const uint32_t e = s <= hi ? min(s + per, hi + 1) : s;
+        if (h.what == 0) acc = verify_range<V>(m, s, e, units);
+        else acc = verify_list<V>(m, s, e, h.lo, h.hi, h.what == 1, primebits, units);
     }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        acc = m.mul(acc, __shfl_down_sync(0xffffffffu, acc, o));
+        units += __shfl_down_sync(0xffffffffu, units, o);
+    }
+    if ((t & 31) == 0) {
+        part[t >> 5] = acc;
+        parts[t >> 5] = units;
+    }
+    __syncthreads();
+    if (t) return false;
+    for (uint32_t i = 1; i < (blockDim.x >> 5); ++i) {
+        acc = m.mul(acc, part[i]);
+        units += parts[i];
+    }
+    // each reduction by a plain word lowered the power of R by one
+    acc = m.mul(acc, m.mont_R_pow(units));
+    const W v = m.mul(acc, m.to_mont((W)h.start));
+    return h.sign < 0 ? v != m.one : v != m.p - m.one;
+}
+
+__global__ void __launch_bounds__(256) verify_hits_kernel(const VerifyRec *r, uint32_t cnt, const uint32_t *primebits,
+                                                          uint8_t *bad) {
+    __shared__ uint64_t part[8], parts[8];
+    if (blockIdx.x >= cnt) return;   // whole blocks
+    const VerifyRec h = r[blockIdx.x];
+    const bool b = h.p >> 31 ? verify_hit<Verify64>(h, primebits, part, parts)
+                             : verify_hit<Verify32>(h, primebits, reinterpret_cast<uint32_t *>(part), parts);
+    if (threadIdx.x == 0) bad[blockIdx.x] = b;
 }
 
 }  // namespace pfc
