@@ -281,8 +281,10 @@ class Job:
         _ck(lib().pfc_sync(self.h), "pfc_sync")
 
     def drain_hits(self):
+        # most drains are a few hits: a first buffer of 64 KB comes from the
+        # heap, where a large one is mapped and its pages cleared on each call
         n = ctypes.c_size_t(0)
-        cap = 1 << 16
+        cap = 1 << 12
         while True:
             buf = np.zeros(cap, dtype=FACTOR_DTYPE)
             rc = lib().pfc_drain_hits(self.h, buf.ctypes.data, cap, ctypes.byref(n))
@@ -299,15 +301,22 @@ class Job:
 
     def run(self, cap=1 << 20):
         """Whole p range; returns the raw hits (unsorted)."""
-        while True:
-            buf = np.zeros(max(cap, 1), dtype=FACTOR_DTYPE)
-            n = ctypes.c_size_t(0)
-            rc = lib().pfc_job_run(self.h, buf.ctypes.data, cap, ctypes.byref(n))
-            if rc == PFC_ERR_HIT_OVERFLOW:
-                raise PFCError(rc, "pfc_job_run: %d hits do not fit %d; rerun with cap=%d"
-                               % (n.value, cap, n.value))
-            _ck(rc, "pfc_job_run")
-            return buf[: n.value]
+        # pfc_job_run's loop with the hits drained per segment: a buffer of
+        # `cap` records, 16 MB, cost 160 us a call in page clearing, more than
+        # half of a search of 8e6 pairs
+        parts, total, lo = [], 0, self.pmin
+        while lo < self.pmax:
+            hi = self.segment_end(lo)
+            self.segment(lo, hi)
+            h = self.drain_hits()
+            total += len(h)
+            if total <= cap:
+                parts.append(h)
+            lo = hi
+        if total > cap:
+            raise PFCError(PFC_ERR_HIT_OVERFLOW, "pfc_job_run: %d hits do not fit %d; rerun with cap=%d"
+                           % (total, cap, total))
+        return parts[0] if len(parts) == 1 else np.concatenate(parts) if parts else np.zeros(0, dtype=FACTOR_DTYPE)
 
     def segment_state(self):
         """(p, s0, s1) of the current segment in the reference's R = 2^64 form."""
