@@ -720,30 +720,6 @@ static HitBuf hitbuf(pfc_job *j) {
 
 // ------------------------------------------------------ tensor-core walks
 
-// Which walk, and when it is split.  Times of one walk launch in microseconds,
-// fitted to GB300 (factorial searches at p = 1e9, 2^61 and 3 2^62, 2,000 to
-// 300,000 candidates x 200 to 10,000 n; the fits are within 15%):
-//   tensor cores: CTAs of 128 candidates, one per SM, so whole waves of them,
-//     each with a fixed part (the candidates' planes, filling and draining the
-//     pipeline, about 1,500 steps' worth) and a part per step; a launch more
-//     for the word table;
-//   per-step kernels: a rate per candidate-step, and below about one chain per
-//     thread the latency of a step.
-// Measured, ms, tensor cores / per-step:
-//   class 32, 19,000 candidates:  500 n .029 / .026, 1,000 .031 / .038, 10,000 .088 / .169
-//            300,000 candidates: 2,000 n .354 / .286, 3,000 .454 / .423, 10,000 1.16 / 1.37
-//   class 64, 19,000 candidates:  500 n .034 / .030, 1,000 .037 / .046, 10,000 .116 / .282
-//            300,000 candidates: 1,000 n .338 / .296, 2,000 .490 / .563, 10,000 1.58 / 2.70
-//   from 2^64/3, 19,000 candidates: 200 n .031 / .025, 500 .033 / .042, 10,000 .125 / .481
-//            300,000 candidates: 500 n .287 / .287, 1,000 .363 / .547, 10,000 1.75 / 5.28
-struct WalkTimes {
-    double fixed, step;            // per wave of the tensor-core walk: fixed part, per step
-    double lat, rate0, rate;       // per-step kernels, per step: latency; base and part per candidate
-};
-constexpr double kTcLaunch = 12.0, kWalkLaunch = 13.0;
-constexpr WalkTimes kTimes32 = {9.7, 6.3e-3, 25.3e-3, 12e-3, 4.1e-7}, kTimes64 = {13.2, 8.8e-3, 31e-3, 20e-3, 8.2e-7},
-                    kTimesTop = {12.3, 9.6e-3, 58e-3, 8e-3, 1.73e-6};   // (class 64 from 2^64/3)
-
 // candidates that a class's buffer is expected to hold (est_cands)
 static double held(uint64_t cap) { return (double)cap / 1.25; }
 
@@ -761,12 +737,6 @@ static double walk_us(const pfc_job *j, const WalkTimes &t, uint64_t cap, double
 static uint32_t max_words(const pfc_job *j) {
     return (uint32_t)std::min<uint64_t>(j->ctx->budget / 16 / 384, kMaxChunk);
 }
-
-// Smallest primes the tensor-core walk takes.  Towards small p a growing part
-// of the blocks holds a hit or a multiple of p and is replayed; at 2^16 that
-// does not show yet (2,700 candidates x 20,000 n: 0.15 ms, per-step 0.62), and
-// few searches start below.
-constexpr uint64_t kTcMinP = 1u << 16;
 
 static bool walk_tc_pays(const pfc_job *j, const WalkTimes &t, uint64_t cap, uint32_t steps) {
     const int on = j->ctx->walk_tc;
@@ -860,8 +830,7 @@ static int enqueue_iter_range(pfc_job *j, uint32_t lo, uint32_t hi, bool split =
             t.type[1] = w.type2;
             t.second[1] = 1;
             for (uint32_t s = 0; s < t.nstreams; ++s) {
-                t.words[s] = j->words[s].p;
-                c->launches += launch_walk_words(t.mult[s], t.base, lo, hi, top, j->words[s].p, c->st);
+                c->launches += launch_walk_words(t.mult[s], t.base, lo, hi, top, j->words[s].p, t, (int)s, c->st);
             }
             if (tc32)
                 c->launches += launch_walk_tc32(j->c32.view(counts_ptr(j)), t, top, h, split ? &sp32 : nullptr,

@@ -14,7 +14,10 @@
 // one launch per class group (class 32, class 64 below 2^64/3, other class 64)
 // and task kind (setup, walk, general) with one CTA per block, on six
 // streams, dispatched by the hardware block scheduler, so jobs of every size
-// and mode share the SMs.
+// and mode share the SMs.  Walk windows long enough for it take the
+// tensor-core walk (walk_tc.cu) instead, one launch per class group and word
+// shape with one CTA per 128 candidates (four drawn mixes of 24 searches: 117,
+// 79, 128 and 77 ms with per-step walks, 108, 65, 93 and 58 so).
 // Between iterations the host admits new jobs as memory and slots allow,
 // drains the hits (tagged with the job slot) and retires finished jobs:
 // requests that arrive while others run join at the next iteration.
@@ -611,6 +614,36 @@ struct pfc_batch {
     uint32_t cache_lim = 0;
     std::vector<Window> w[kLists][kKinds];   // this iteration's windows per launch
     uint64_t ctas[kLists][kKinds] = {};
+    // walk windows on the tensor cores, per class group and word shape: their
+    // word tables, window records (in passes over as much of the windows as
+    // the tables hold), and empty walk windows after them that end timelines
+    struct TcWalk {
+        std::vector<std::pair<double, Window>> plan;   // (cost, window)
+        DArr<uint8_t> tables;
+        DArr<uint32_t> digits;                         // two a window
+        DArr<WalkWordsWin> d_words;
+        DArr<WalkTcWin<uint32_t>> d_w32;
+        DArr<WalkTcWin<uint64_t>> d_w64;
+        DArr<Window> d_fin;
+        std::vector<WalkWordsWin> words;
+        std::vector<WalkTcWin<uint32_t>> w32;
+        std::vector<WalkTcWin<uint64_t>> w64;
+        std::vector<Window> fin;
+        struct Pass {
+            uint32_t words0, words, words_ctas, win0, wins, ctas;
+        };
+        std::vector<Pass> passes;
+        uint64_t fin_ctas = 0;
+        void release(pfc_ctx *c) {
+            tables.release(c);
+            digits.release(c);
+            d_words.release(c);
+            d_w32.release(c);
+            d_w64.release(c);
+            d_fin.release(c);
+        }
+    };
+    TcWalk tcw[kLists][2];
     uint64_t next_id = 1;
     double work_per_iter = 0;            // candidate-steps per iteration (class 64 weighs 3); 0: the policy's
     int policy = PFC_BATCH_THROUGHPUT;
@@ -953,6 +986,124 @@ static uint32_t per_cta(const BatchJob *j, bool cls64, int kind) {
     return j->mode == (PFC_FACTORIAL | PFC_COMPOSITORIAL) ? 256u : 256u * Cls32::NC;
 }
 
+// Whether a walk window of n candidates and `steps` steps (over all chains)
+// takes the tensor-core walk: the SM time of both (kernels.cuh WalkTimes)
+// where other searches fill what a window leaves idle.
+static bool tc_walk_pays(const pfc_batch *b, const BatchJob *j, int l, uint32_t n, double steps) {
+    const int on = b->ctx->walk_tc;
+    if (!on || j->pmin < kTcMinP || (l == 2 && !(j->pmin >> 62))) return false;
+    const WalkTimes &t = l == 0 ? kTimes32 : l == 1 ? kTimes64 : kTimesTop;
+    return on > 1 || walk_tc_ctas(n) * (t.fixed + t.step * steps) < n * 152.0 * t.rate * steps;
+}
+
+// Lay out the windows of one class group and word shape: pieces of them in
+// passes whose tables fit a 48th of the memory budget, one after another on
+// the group's stream.  False where even that has no room left.
+static bool plan_tc_walk(pfc_batch *b, int l, int shape, const std::vector<BatchJob *> &by_slot) {
+    pfc_ctx *c = b->ctx;
+    pfc_batch::TcWalk &g = b->tcw[l][shape];
+    g.words.clear();
+    g.w32.clear();
+    g.w64.clear();
+    g.fin.clear();
+    g.passes.clear();
+    g.fin_ctas = 0;
+    if (g.plan.empty()) return true;
+    std::sort(g.plan.begin(), g.plan.end(), [](const auto &x, const auto &y) { return x.first > y.first; });
+    auto chains = [](const BatchJob *j) { return j->mode == (PFC_FACTORIAL | PFC_COMPOSITORIAL) ? 2u : 1u; };
+    double all = 0;
+    for (const auto &e : g.plan) {
+        const BatchJob *j = by_slot[e.second.slot];
+        all += (double)chains(j) * walk_tc_words_bytes(j->nmax - 1, e.second.hi - e.second.lo);
+    }
+    const uint32_t npass = (uint32_t)std::ceil(all / std::max((double)(c->budget / 48), 1.0));
+    size_t tables = 0;
+    std::vector<uint32_t> piece;
+    for (const auto &e : g.plan) {
+        const BatchJob *j = by_slot[e.second.slot];
+        const uint32_t len = e.second.hi - e.second.lo, align = walk_tc_align(j->nmax - 1);
+        const uint32_t per = (uint32_t)(((uint64_t)(len + npass - 1) / npass + align - 1) / align * align);
+        piece.push_back(per);
+        tables += (size_t)chains(j) * walk_tc_words_bytes(j->nmax - 1, std::min(per, len));
+    }
+    const size_t nw = g.plan.size();
+    cudaError_t e = cudaSuccess;
+    auto room = [&](auto &arr, size_t n) {
+        if (e == cudaSuccess && arr.n < n) e = arr.alloc(c, n + n / 4);
+    };
+    if (tables > c->budget / 16) return false;
+    if (g.tables.n < tables) e = g.tables.alloc(c, tables);
+    room(g.digits, 2 * nw);
+    room(g.d_words, 2 * nw * npass);
+    if (l == 0) room(g.d_w32, nw * npass);
+    else room(g.d_w64, nw * npass);
+    room(g.d_fin, nw);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        g.release(c);
+        return false;
+    }
+    for (uint32_t k = 0; k < npass; ++k) {
+        pfc_batch::TcWalk::Pass ps{(uint32_t)g.words.size(), 0, 0, (uint32_t)(l == 0 ? g.w32.size() : g.w64.size()), 0, 0};
+        size_t at = 0;
+        for (size_t i = 0; i < nw; ++i) {
+            const Window &w = g.plan[i].second;
+            BatchJob *j = by_slot[w.slot];
+            const uint32_t ns = l == 0 ? j->nsetup32 : j->nsetup64, top = j->nmax - 1;
+            const uint32_t base = j->mode == PFC_PRIMORIAL ? 0u : j->nmin;
+            const uint64_t from = (uint64_t)w.lo + (uint64_t)k * piece[i];
+            const size_t bytes = walk_tc_words_bytes(top, std::min(piece[i], w.hi - w.lo));
+            const size_t tab = at;
+            at += chains(j) * bytes;
+            if (from >= w.hi) continue;
+            WalkTcArgs a{};
+            walk_tc_args(a, top);
+            a.nstreams = chains(j);
+            a.lo = base + (uint32_t)(from - ns);
+            a.hi = base + (uint32_t)(std::min<uint64_t>(from + piece[i], w.hi) - ns);
+            a.base = base;
+            const bool prim = j->mode == PFC_PRIMORIAL, comp = j->mode == PFC_COMPOSITORIAL;
+            a.mult[0] = prim ? j->d_qlist.p : comp ? j->d_cmult.p : nullptr;
+            a.mult[1] = j->d_cmult.p;
+            a.type[0] = prim ? PFC_TYPE_PRIMORIAL : comp ? PFC_TYPE_COMPOSITORIAL : PFC_TYPE_FACTORIAL;
+            a.type[1] = PFC_TYPE_COMPOSITORIAL;
+            a.second[1] = 1;
+            for (uint32_t s = 0; s < a.nstreams; ++s) {
+                unsigned char *table = g.tables.p + tab + s * bytes;
+                a.words[s] = table;
+                a.digits[s] = g.digits.p + 2 * i + s;
+                WalkWordsWin ww{};
+                walk_words_win(ww, a.mult[s], base, a.lo, a.hi, top, table, g.digits.p + 2 * i + s);
+                ww.first_cta = ps.words_ctas;
+                ps.words_ctas += walk_words_ctas(top, a.hi - a.lo);
+                g.words.push_back(ww);
+                ++ps.words;
+            }
+            BatchStats *bs = b->stats.p + w.slot;   // device address
+            auto win = [&](auto &list, const auto &buf) {
+                list.push_back({buf, a, &bs->flags, ps.ctas, w.slot});
+            };
+            if (l == 0) win(g.w32, j->c32.view(bs->counts));
+            else win(g.w64, j->c64.view(bs->counts + 1));
+            ps.ctas += walk_tc_ctas(w.ncand);
+            ++ps.wins;
+        }
+        if (ps.wins) g.passes.push_back(ps);
+    }
+    for (const auto &en : g.plan) {
+        const BatchJob *j = by_slot[en.second.slot];
+        const uint32_t tot = l == 0 ? j->tot32 : j->tot64, per = per_cta(j, l != 0, kWalkTask);
+        if (en.second.hi < tot) continue;
+        Window w = en.second;
+        w.lo = w.hi = tot;
+        w.nblocks = (w.ncand + per - 1) / per;
+        w.first_cta = (uint32_t)g.fin_ctas;
+        g.fin_ctas += w.nblocks;
+        g.fin.push_back(w);
+    }
+    return true;
+}
+
 // One window per search and class.  Throughput policy: every search advances
 // a common window of L positions per iteration (all searches progress at the
 // same pace, so the largest ones are never starved and the batch ends as
@@ -1043,7 +1194,11 @@ uint32_t build_tasks(pfc_batch *b) {
     const uint32_t L = ((uint32_t)Ld + 15u) & ~15u;
 
     std::vector<std::pair<double, Window>> lists[pfc_batch::kLists][pfc_batch::kKinds];
+    std::vector<BatchJob *> by_slot(pfc_batch::kSlots, nullptr);
+    for (auto &row : b->tcw)
+        for (auto &g : row) g.plan.clear();
     for (BatchJob *j : b->running) {
+        by_slot[j->slot] = j;
         j->next32 = j->pos32;
         j->next64 = j->pos64;
         for (int cls = 0; cls < 2; ++cls) {
@@ -1069,9 +1224,20 @@ uint32_t build_tasks(pfc_batch *b) {
             w.lo = pos;
             w.hi = hi;
             const int l = cls == 0 ? 0 : (j->pmax <= kLazyEnd ? 1 : 2);
-            lists[l][kind].push_back({cost, w});
+            const double chains = j->mode == (PFC_FACTORIAL | PFC_COMPOSITORIAL) ? 2.0 : 1.0;
+            if (kind == kWalkTask && hi > pos && tc_walk_pays(b, j, l, n, chains * (hi - pos)))
+                b->tcw[l][walk_tc_shape(j->nmax - 1)].plan.push_back({chains * (hi - pos), w});
+            else
+                lists[l][kind].push_back({cost, w});
         }
     }
+    for (int l = 0; l < pfc_batch::kLists; ++l)
+        for (int shape = 0; shape < 2; ++shape)
+            if (!plan_tc_walk(b, l, shape, by_slot)) {   // no room for tables: per-step
+                auto &g = b->tcw[l][shape];
+                lists[l][kWalkTask].insert(lists[l][kWalkTask].end(), g.plan.begin(), g.plan.end());
+                g.plan.clear();
+            }
     for (int l = 0; l < pfc_batch::kLists; ++l)
         for (int k = 0; k < pfc_batch::kKinds; ++k) {
             auto &lst = lists[l][k];
@@ -1099,6 +1265,28 @@ static void launch_list(pfc_batch *b, int l, const JobDev<typename T::W> *jobs, 
     b->ctx->launches++;
 }
 
+// the tensor-core walks of a class group and word shape, and the windows that
+// end timelines after them
+template <class T>
+static void launch_tc_walks(pfc_batch *b, int l, int shape, const JobDev<typename T::W> *jobs, const HitBuf &h) {
+    pfc_batch::TcWalk &g = b->tcw[l][shape];
+    if (g.passes.empty()) return;
+    const int si = (l == 0 ? 0 : 3) + ((l == 2) != (shape == 1) ? 2 : 0);
+    cudaStream_t st = b->st[si];
+    for (const auto &ps : g.passes) {
+        cudaMemsetAsync(g.digits.p, 0, 2 * g.plan.size() * sizeof(uint32_t), st);
+        b->ctx->launches += launch_walk_words_many(g.d_words.p + ps.words0, ps.words, ps.words_ctas, shape, st);
+        if (l == 0) b->ctx->launches += launch_walk_tc32_many(g.d_w32.p + ps.win0, ps.wins, ps.ctas, shape, h, st);
+        else b->ctx->launches += launch_walk_tc64_many(g.d_w64.p + ps.win0, ps.wins, ps.ctas, shape, l == 1, h, st);
+    }
+    if (g.fin_ctas) {
+        batch_kernel<T, kWalkTask><<<(unsigned)g.fin_ctas, task_threads<T, kWalkTask>(), 0, st>>>(
+            g.d_fin.p, (uint32_t)g.fin.size(), jobs, h);
+        b->ctx->launches++;
+    }
+    b->used[si] = true;
+}
+
 bool tc_chunks_pending(const pfc_batch *b) {
     for (const BatchJob *j : b->running)
         for (int k = 0; k < 2; ++k)
@@ -1115,6 +1303,18 @@ int launch_iteration(pfc_batch *b) {
             if (b->wins[l][k].n < n) CK(b->wins[l][k].alloc(c, n + n / 2 + 64));
             CK(cudaMemcpyAsync(b->wins[l][k].p, b->w[l][k].data(), n * sizeof(Window), cudaMemcpyHostToDevice, c->st));
             c->h2d += n * sizeof(Window);
+        }
+    for (auto &row : b->tcw)
+        for (auto &g : row) {
+            auto up = [&](auto &dst, const auto &src) -> cudaError_t {
+                if (src.empty()) return cudaSuccess;
+                c->h2d += src.size() * sizeof(src[0]);
+                return cudaMemcpyAsync(dst.p, src.data(), src.size() * sizeof(src[0]), cudaMemcpyHostToDevice, c->st);
+            };
+            CK(up(g.d_words, g.words));
+            CK(up(g.d_w32, g.w32));
+            CK(up(g.d_w64, g.w64));
+            CK(up(g.d_fin, g.fin));
         }
     // latency policy: chunks of pending tensor-core setups, smallest first,
     // ahead of the iteration's windows on the context stream
@@ -1161,6 +1361,11 @@ int launch_iteration(pfc_batch *b) {
     // setup-only and general lists first: they hold the longest tasks
     launch_list<Cls32, kSetupTask>(b, 0, b->jobs32.p, h);
     launch_list<Cls32, kAnyTask>(b, 0, b->jobs32.p, h);
+    for (int shape = 0; shape < 2; ++shape) {   // whole SMs per CTA: before the per-step walks
+        launch_tc_walks<Cls32>(b, 0, shape, b->jobs32.p, h);
+        launch_tc_walks<Cls64L>(b, 1, shape, b->jobs64.p, h);
+        launch_tc_walks<Cls64>(b, 2, shape, b->jobs64.p, h);
+    }
     launch_list<Cls32, kWalkTask>(b, 0, b->jobs32.p, h);
     launch_list<Cls64L, kSetupTask>(b, 1, b->jobs64.p, h);
     launch_list<Cls64L, kAnyTask>(b, 1, b->jobs64.p, h);
@@ -1179,6 +1384,9 @@ int launch_iteration(pfc_batch *b) {
         n32 += b->ctas[0][k];
         n64 += b->ctas[1][k] + b->ctas[2][k];
     }
+    for (int l = 0; l < pfc_batch::kLists; ++l)
+        for (const auto &g : b->tcw[l])
+            for (const auto &ps : g.passes) (l == 0 ? n32 : n64) += ps.ctas;
     b->tasks += n32 + n64;
     b->t32_n = n32;
     b->t64_n = n64;
@@ -1192,6 +1400,8 @@ int finish_iteration(pfc_batch *b, uint32_t L) {
     pfc_ctx *c = b->ctx;
     CK(cudaStreamSynchronize(c->st));
     ++b->iterations;
+    for (auto &row : b->tcw)   // their room is for new searches until the next iteration
+        for (auto &g : row) g.tables.release(c);
     if (b->ck_pending) {
         float ms = 0;
         CK(cudaEventElapsedTime(&ms, b->ev_ck0, b->ev_ck1));
@@ -1287,8 +1497,8 @@ int retire_finished(pfc_batch *b) {
             j->status = rerun_alone(b, j);
         } else if (j->flags & 1u) {
             j->status = PFC_ERR_VALIDATION;
-        } else if (j->flags & 2u) {
-            j->status = PFC_ERR_CUDA;   // a tensor-core setup wait gave up
+        } else if (j->flags & 6u) {
+            j->status = PFC_ERR_CUDA;   // a tensor-core setup's or walk's wait gave up
         }
     }
     b->running.swap(still);
@@ -1361,6 +1571,8 @@ extern "C" int pfc_batch_destroy(pfc_batch *b) {
     b->jobs64.release(c);
     for (auto &row : b->wins)
         for (auto &d : row) d.release(c);
+    for (auto &row : b->tcw)
+        for (auto &g : row) g.release(c);
     b->hits.release(c);
     b->tags.release(c);
     b->hitcount.release(c);
@@ -1428,6 +1640,8 @@ extern "C" int pfc_batch_step(pfc_batch *b, uint32_t *active, uint32_t *queued) 
         bool work = tc_chunks_pending(b);
         for (auto &row : b->ctas)
             for (uint64_t n : row) work |= n > 0;
+        for (auto &row : b->tcw)
+            for (auto &g : row) work |= !g.passes.empty();
         if (!work && pass == 0) {
             // everything running waits for a tensor-core setup: the call
             // returns after a short pause (searches submitted meanwhile are

@@ -190,22 +190,81 @@ int launch_walk64(const ClassBuf<uint64_t> &c, const WalkArgs &a, const HitBuf &
 // (`top`: the largest multiplier of the tables, which sets the words' shape).
 struct WalkTcArgs {
     const unsigned char *words[2];
+    const uint32_t *digits[2];   // largest sum of |digit| of a table's words
     const uint32_t *mult[2];   // multipliers of step k at mult[k - base], or k itself (null)
     int32_t type[2];           // factor type of a stream's hits
     uint32_t second[2];        // 1: the stream walks the residue s1
     uint32_t nstreams;
     uint32_t lo, hi, base;
-    uint32_t nb, shift11, shift22;   // set by the launch: steps per block, 2^11, 2^22
+    uint32_t nb, shift11, shift22;   // set by walk_tc_args: steps per block, 2^11, 2^22
 };
+void walk_tc_args(WalkTcArgs &a, uint32_t top);
 uint32_t walk_tc_align(uint32_t top);   // sub-ranges of a split walk start at multiples of this from lo
 size_t walk_tc_words_bytes(uint32_t top, uint32_t steps);
+// (the table of steps [lo, hi) into `out`, for the walk's stream `stream`)
 int launch_walk_words(const uint32_t *mult, uint32_t base, uint32_t lo, uint32_t hi, uint32_t top, unsigned char *out,
-                      cudaStream_t st);
+                      WalkTcArgs &a, int stream, cudaStream_t st);
+// The same over windows of many searches, one launch for the tables and one
+// for the walks of a size class and word shape (walk_tc_shape).  Windows are
+// ordered by first_cta; a table has walk_tc_words_bytes, its `digits` start at 0.
+struct WalkWordsWin {
+    const uint32_t *mult;
+    unsigned char *out;
+    uint32_t *digits;
+    uint32_t base, lo, hi, nb, nsuper, first_cta;
+};
+template <class W>
+struct WalkTcWin {
+    ClassBuf<W> c;
+    WalkTcArgs a;
+    uint32_t *err;
+    uint32_t first_cta, tag;
+};
+int walk_tc_shape(uint32_t top);
+uint32_t walk_tc_ctas(uint32_t cands);
+uint32_t walk_words_ctas(uint32_t top, uint32_t steps);
+void walk_words_win(WalkWordsWin &win, const uint32_t *mult, uint32_t base, uint32_t lo, uint32_t hi, uint32_t top,
+                    unsigned char *table, uint32_t *digits);
+int launch_walk_words_many(const WalkWordsWin *wins, uint32_t n, uint32_t ctas, int shape, cudaStream_t st);
+int launch_walk_tc32_many(const WalkTcWin<uint32_t> *wins, uint32_t n, uint32_t ctas, int shape, const HitBuf &h,
+                          cudaStream_t st);
+int launch_walk_tc64_many(const WalkTcWin<uint64_t> *wins, uint32_t n, uint32_t ctas, int shape, bool lazy,
+                          const HitBuf &h, cudaStream_t st);
 // a wait that gives up sets bit 2 of *err
 int launch_walk_tc32(const ClassBuf<uint32_t> &c, const WalkTcArgs &a, uint32_t top, const HitBuf &h,
                      const SplitArgs<uint32_t> *sp, uint32_t *err, cudaStream_t st);
 int launch_walk_tc64(const ClassBuf<uint64_t> &c, const WalkTcArgs &a, uint32_t top, const HitBuf &h,
                      const SplitArgs<uint64_t> *sp, uint32_t *err, cudaStream_t st, bool lazy);
+// Which walk, and when it is split.  Times of one walk launch in microseconds,
+// fitted to GB300 (factorial searches at p = 1e9, 2^61 and 3 2^62, 2,000 to
+// 300,000 candidates x 200 to 10,000 n; the fits are within 15%):
+//   tensor cores: CTAs of 128 candidates, one per SM, so whole waves of them,
+//     each with a fixed part (the candidates' planes, filling and draining the
+//     pipeline, about 1,500 steps' worth) and a part per step; a launch more
+//     for the word table;
+//   per-step kernels: a rate per candidate-step, and below about one chain per
+//     thread the latency of a step.
+// Measured, ms, tensor cores / per-step:
+//   class 32, 19,000 candidates:  500 n .029 / .026, 1,000 .031 / .038, 10,000 .088 / .169
+//            300,000 candidates: 2,000 n .354 / .286, 3,000 .454 / .423, 10,000 1.16 / 1.37
+//   class 64, 19,000 candidates:  500 n .034 / .030, 1,000 .037 / .046, 10,000 .116 / .282
+//            300,000 candidates: 1,000 n .338 / .296, 2,000 .490 / .563, 10,000 1.58 / 2.70
+//   from 2^64/3, 19,000 candidates: 200 n .031 / .025, 500 .033 / .042, 10,000 .125 / .481
+//            300,000 candidates: 500 n .287 / .287, 1,000 .363 / .547, 10,000 1.75 / 5.28
+struct WalkTimes {
+    double fixed, step;            // per wave of the tensor-core walk: fixed part, per step
+    double lat, rate0, rate;       // per-step kernels, per step: latency; base and part per candidate
+};
+constexpr double kTcLaunch = 12.0, kWalkLaunch = 13.0;
+constexpr WalkTimes kTimes32 = {9.7, 6.3e-3, 25.3e-3, 12e-3, 4.1e-7}, kTimes64 = {13.2, 8.8e-3, 31e-3, 20e-3, 8.2e-7},
+                    kTimesTop = {12.3, 9.6e-3, 58e-3, 8e-3, 1.73e-6};   // (class 64 from 2^64/3)
+
+// Smallest primes the tensor-core walk takes.  Towards small p a growing part
+// of the blocks holds a hit or a multiple of p and is replayed; at 2^16 that
+// does not show yet (2,700 candidates x 20,000 n: 0.15 ms, per-step 0.62), and
+// few searches start below.
+constexpr uint64_t kTcMinP = 1u << 16;
+
 // size class 0: p < 2^31, 1: lazy class 64 (p < 2^64/3), 2: other class 64
 int walk_variant_count(int cls, bool fused);
 int walk_variant_shape(int cls, bool fused, int variant, int *nc, int *b);

@@ -27,7 +27,7 @@
 // 2^-16, so the test takes a window of +-half around +-A, half =
 // floor(0.504 / 256 max sum |digit| + 0.045) + 1: every hit passes, and with
 // half 2 or 3 one pair in 6,500 or 4,700 passes by chance.  The maximum is
-// taken over the table's own words (its first 4 bytes).  A lane that saw a
+// taken over the table's own words.  A lane that saw a
 // pass queues (residue at the block's START, block, candidate) in a ring in
 // shared memory, and warps of their own replay the queue with exact
 // arithmetic, one entry per lane, so false passes cost time only.  The offsets
@@ -90,7 +90,7 @@ constexpr int kTesterGroups = 4;               // warp groups, two per buffer, e
 constexpr int kTestBlocks = 2;
 constexpr int kBatches = 16;                   // ring of suspects, in batches of 32
 constexpr uint32_t kBiasE = 0x4B000000u;       // fp32 bits of 2^23, under the residues' sums
-constexpr uint32_t kTableHead = 128;           // a word table begins with its largest sum of |digit| (u32)
+constexpr uint32_t kTableHead = 128;           // a search's word table begins with its largest sum of |digit| (u32)
 
 // digits per word (KD) and MMA depth (K = KD + 1, the bias digit first)
 template <int K>
@@ -365,12 +365,12 @@ __device__ __forceinline__ void replay_suspect(bool act, typename T::W p, typena
 // (balanced digits: the 6-bit digits of N + sum 32 * 64^b, less 32).  One
 // thread per word.
 template <int K>
-__global__ void __launch_bounds__(128) walk_words_kernel(const uint32_t *mult, uint32_t base, uint32_t lo, uint32_t hi,
-                                                         uint32_t nb, uint32_t nsuper, unsigned char *table) {
+__device__ __forceinline__ void walk_words(const WalkWordsWin &win, uint32_t i) {
     using S = WordShape<K>;
     constexpr uint32_t kRows = 17 * kBlocksSuper;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned char *out = table + kTableHead;
+    const uint32_t *mult = win.mult;
+    const uint32_t base = win.base, lo = win.lo, hi = win.hi, nb = win.nb, nsuper = win.nsuper;
+    unsigned char *out = win.out;
     const uint32_t st = min(i / kRows, nsuper - 1), r = i % kRows;   // (past the end: the last supertile's again)
     const bool whole = r < kBlocksSuper;
     const uint32_t row = r - kBlocksSuper;                      // among the 256 test words
@@ -435,12 +435,36 @@ __global__ void __launch_bounds__(128) walk_words_kernel(const uint32_t *mult, u
     }
     if (whole) digits = 0;
     digits = __reduce_max_sync(kFull, digits);
-    if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<uint32_t *>(table), digits);
+    if ((threadIdx.x & 31) == 0) atomicMax(win.digits, digits);
 }
 
+template <int K>
+__global__ void __launch_bounds__(128) walk_words_kernel(WalkWordsWin win) {
+    walk_words<K>(win, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// the last of the windows whose first CTA is not past `cta`
+template <class Win>
+__device__ __forceinline__ uint32_t window_of(const Win *wins, uint32_t n, uint32_t cta) {
+    uint32_t a = 0, b = n;
+    while (b - a > 1) {
+        const uint32_t mid = (a + b) >> 1;
+        if (wins[mid].first_cta <= cta) a = mid;
+        else b = mid;
+    }
+    return a;
+}
+
+template <int K>
+__global__ void __launch_bounds__(128) walk_words_many_kernel(const WalkWordsWin *wins, uint32_t n) {
+    const WalkWordsWin win = wins[window_of(wins, n, blockIdx.x)];
+    walk_words<K>(win, (blockIdx.x - win.first_cta) * blockDim.x + threadIdx.x);
+}
+
+// one CTA: candidates 128 cta .. of c, sub-range `sub` of a split walk (sp, or null)
 template <class T, int K>
-__global__ void __launch_bounds__(Role<T>::kThreads, 1)
-    walk_tc_kernel(ClassBuf<typename T::W> c, WalkTcArgs a, HitBuf h, SplitArgs<typename T::W> sp, uint32_t *err) {
+__device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const WalkTcArgs &a, const HitBuf &h,
+                                        const SplitArgs<typename T::W> *sp, uint32_t *err, uint32_t cta, uint32_t sub) {
     using C = ChainClass<T>;
     using L = Lay<T, K>;
     using S = WordShape<K>;
@@ -448,17 +472,16 @@ __global__ void __launch_bounds__(Role<T>::kThreads, 1)
     extern __shared__ __align__(1024) unsigned char sm[];
     const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     const uint32_t cnt = min(*c.count, c.cap);
-    const uint32_t c0 = blockIdx.x * kCands;
+    const uint32_t c0 = cta * kCands;
     if (c0 >= cnt) return;   // whole CTA idle
 
     uint32_t lo = a.lo, hi = a.hi;
-    const uint32_t sub = blockIdx.y;
-    const bool last = sub + 1 >= sp.n;
+    const bool split = sp && sp->n > 1, last = !split || sub + 1 >= sp->n;
 #pragma unroll
     for (int k = 0; k < kMaxSplit; ++k)
-        if (sp.n > 1 && (uint32_t)k == sub) {
-            lo = sp.start[k];
-            hi = sp.start[k + 1];
+        if (split && (uint32_t)k == sub) {
+            lo = sp->start[k];
+            hi = sp->start[k + 1];
         }
     const uint32_t super0 = (lo - a.lo) / (kBlocksSuper * a.nb);   // sub-ranges start at supertiles
     const uint32_t supers = ((hi - lo + a.nb - 1) / a.nb + kBlocksSuper - 1) / kBlocksSuper;   // of a stream
@@ -467,8 +490,8 @@ __global__ void __launch_bounds__(Role<T>::kThreads, 1)
     const uint32_t nsupers_e = (supers + C::kBlocksE / kBlocksSuper - 1) / (C::kBlocksE / kBlocksSuper);
     // the test's window around +-A in units of 2^-16: the f_b are off by up to
     // 0.504 units of 2^-24 each, A by 0.045 of 2^-16
-    uint32_t digits = *reinterpret_cast<const uint32_t *>(a.words[0]);
-    if (a.nstreams > 1) digits = max(digits, *reinterpret_cast<const uint32_t *>(a.words[1]));
+    uint32_t digits = *a.digits[0];
+    if (a.nstreams > 1) digits = max(digits, *a.digits[1]);
     const uint32_t half = (uint32_t)(digits * (0.504f / 256.0f) + 0.045f) + 1u;
     const uint32_t bar = smem_u32(sm + L::kOffBar);
     constexpr uint32_t kB0 = kFStages + L::kWStages, kB1 = kB0 + 2 * kBufs, kB2 = kB1 + 2 * C::kRUnits,
@@ -533,8 +556,8 @@ __global__ void __launch_bounds__(Role<T>::kThreads, 1)
     // copies of the MMA warps: tile t of test words into a stage of its
     // buffer, supertile(s) g of block words; the first ones start here (none
     // after a wait that gave up: a copy may then still be pending on its barrier)
-    const unsigned char *tab0 = a.words[0] + kTableHead + (size_t)super0 * S::kSuper;
-    const unsigned char *tab1 = a.nstreams > 1 ? a.words[1] + kTableHead + (size_t)super0 * S::kSuper : nullptr;
+    const unsigned char *tab0 = a.words[0] + (size_t)super0 * S::kSuper;
+    const unsigned char *tab1 = a.nstreams > 1 ? a.words[1] + (size_t)super0 * S::kSuper : nullptr;
     constexpr uint32_t kPer = C::kBlocksE / kBlocksSuper;   // supertiles per buffer of residue sums
     const uint32_t nge = nsupers_e * a.nstreams;
     auto load_f = [&](uint32_t t, uint32_t b, uint32_t stage) {
@@ -838,7 +861,7 @@ __global__ void __launch_bounds__(Role<T>::kThreads, 1)
         for (uint32_t s = 0; s < a.nstreams; ++s) {
             const bool second = (s ? a.second[1] : a.second[0]) != 0;
             const W *in = second ? c.s1 : c.s0;
-            if (sub) in = (second ? sp.s1 : sp.s0) + (size_t)(sub - 1) * sp.pitch;
+            if (split && sub) in = (second ? sp->s1 : sp->s0) + (size_t)(sub - 1) * sp->pitch;
             W r = act ? in[ci] : (W)0;
             for (uint32_t ul = 0; ul < units; ++ul, ++un) {
                 warp_wait(bar_u(us0), uph, fail);
@@ -872,7 +895,7 @@ __global__ void __launch_bounds__(Role<T>::kThreads, 1)
             }
             if (act && !*failed) {
                 if (last) (second ? c.s1 : c.s0)[ci] = T::canon(m, r);
-                if (sp.n > 1) atomicAdd(c.nnext + ci, hi - lo);
+                if (split) atomicAdd(c.nnext + ci, hi - lo);
                 else c.nnext[ci] += hi - lo;
             }
         }
@@ -995,6 +1018,24 @@ __global__ void __launch_bounds__(Role<T>::kThreads, 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tbase) : "memory");
 }
 
+template <class T, int K>
+__global__ void __launch_bounds__(Role<T>::kThreads, 1)
+    walk_tc_kernel(ClassBuf<typename T::W> c, WalkTcArgs a, HitBuf h, SplitArgs<typename T::W> sp, uint32_t *err) {
+    walk_tc<T, K>(c, a, h, &sp, err, blockIdx.x, blockIdx.y);
+}
+
+// The walks of many searches in one launch (a batch's iteration): each CTA
+// finds its window and keeps the window's record in shared memory.
+template <class T, int K>
+__global__ void __launch_bounds__(Role<T>::kThreads, 1)
+    walk_tc_many_kernel(const WalkTcWin<typename T::W> *wins, uint32_t n, HitBuf h) {
+    __shared__ WalkTcWin<typename T::W> w;
+    if (threadIdx.x == 0) w = wins[window_of(wins, n, blockIdx.x)];
+    __syncthreads();
+    h.tagval = w.tag;
+    walk_tc<T, K>(w.c, w.a, h, nullptr, w.err, blockIdx.x - w.first_cta, 0);
+}
+
 // ------------------------------------------------------------------ launches
 
 // Words of 47 digits (K = 48) hold the product of 16 multipliers below 2^17.6,
@@ -1010,35 +1051,93 @@ size_t walk_tc_words_bytes(uint32_t top, uint32_t steps) {
     return kTableHead + nsuper * (word_depth(top) == 48 ? WordShape<48>::kSuper : WordShape<64>::kSuper);
 }
 
+static uint32_t supers_of(uint32_t top, uint32_t steps) {
+    const uint32_t per = walk_tc_align(top);
+    return (uint32_t)(((uint64_t)steps + per - 1) / per);
+}
+uint32_t walk_words_ctas(uint32_t top, uint32_t steps) { return (supers_of(top, steps) * 17 * kBlocksSuper + 127) / 128; }
+int walk_tc_shape(uint32_t top) { return word_depth(top) == 48 ? 0 : 1; }
+
+void walk_words_win(WalkWordsWin &win, const uint32_t *mult, uint32_t base, uint32_t lo, uint32_t hi, uint32_t top,
+                    unsigned char *table, uint32_t *digits) {
+    win.mult = mult;
+    win.base = base;
+    win.lo = lo;
+    win.hi = hi;
+    win.nb = walk_tc_block(top);
+    win.nsuper = supers_of(top, hi - lo);
+    win.out = table;
+    win.digits = digits;
+}
+
 int launch_walk_words(const uint32_t *mult, uint32_t base, uint32_t lo, uint32_t hi, uint32_t top, unsigned char *out,
-                      cudaStream_t st) {
+                      WalkTcArgs &a, int stream, cudaStream_t st) {
+    a.words[stream] = out + kTableHead;
+    a.digits[stream] = reinterpret_cast<const uint32_t *>(out);
     if (hi <= lo) return 0;
-    const uint32_t nb = walk_tc_block(top), per = kBlocksSuper * nb, nsuper = (hi - lo + per - 1) / per;
-    const uint32_t rows = nsuper * 17 * kBlocksSuper, blocks = (rows + 127) / 128;
+    WalkWordsWin win{};
+    walk_words_win(win, mult, base, lo, hi, top, out + kTableHead, reinterpret_cast<uint32_t *>(out));
+    const uint32_t blocks = walk_words_ctas(top, hi - lo);
     if (cudaMemsetAsync(out, 0, kTableHead, st) != cudaSuccess) return 0;
-    if (word_depth(top) == 48) walk_words_kernel<48><<<blocks, 128, 0, st>>>(mult, base, lo, hi, nb, nsuper, out);
-    else walk_words_kernel<64><<<blocks, 128, 0, st>>>(mult, base, lo, hi, nb, nsuper, out);
+    if (word_depth(top) == 48) walk_words_kernel<48><<<blocks, 128, 0, st>>>(win);
+    else walk_words_kernel<64><<<blocks, 128, 0, st>>>(win);
+    return 1;
+}
+
+int launch_walk_words_many(const WalkWordsWin *wins, uint32_t n, uint32_t ctas, int shape, cudaStream_t st) {
+    if (!n) return 0;
+    if (shape == 0) walk_words_many_kernel<48><<<ctas, 128, 0, st>>>(wins, n);
+    else walk_words_many_kernel<64><<<ctas, 128, 0, st>>>(wins, n);
+    return 1;
+}
+
+// raises a kernel's dynamic shared memory once per device
+template <class Kernel>
+static bool configure(Kernel kernel, uint32_t smem, bool (&configured)[64]) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    if (!configured[dev] &&
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        return false;
+    return configured[dev] = true;
+}
+
+void walk_tc_args(WalkTcArgs &a, uint32_t top) {
+    a.nb = walk_tc_block(top);
+    a.shift11 = 1u << 11;
+    a.shift22 = 1u << 22;
+}
+
+template <class T, int K>
+static int launch_tc(const ClassBuf<typename T::W> &c, const WalkTcArgs &a, const HitBuf &h,
+                     const SplitArgs<typename T::W> &sp, uint32_t *err, cudaStream_t st) {
+    using L = Lay<T, K>;
+    static bool configured[64] = {false};
+    if (!configure(walk_tc_kernel<T, K>, L::kSmem, configured)) return 0;
+    const dim3 grid((c.cap + kCands - 1) / kCands, sp.n);
+    walk_tc_kernel<T, K><<<grid, Role<T>::kThreads, L::kSmem, st>>>(c, a, h, sp, err);
     return 1;
 }
 
 template <class T, int K>
-static int launch_tc(const ClassBuf<typename T::W> &c, WalkTcArgs a, const HitBuf &h,
-                     const SplitArgs<typename T::W> &sp, uint32_t *err, cudaStream_t st) {
+static int launch_many(const WalkTcWin<typename T::W> *wins, uint32_t n, uint32_t ctas, const HitBuf &h, cudaStream_t st) {
     using L = Lay<T, K>;
     static bool configured[64] = {false};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-    if (!configured[dev]) {
-        if (cudaFuncSetAttribute(walk_tc_kernel<T, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kSmem) !=
-            cudaSuccess)
-            return 0;
-        configured[dev] = true;
-    }
-    a.shift11 = 1u << 11;
-    a.shift22 = 1u << 22;
-    const dim3 grid((c.cap + kCands - 1) / kCands, sp.n);
-    walk_tc_kernel<T, K><<<grid, Role<T>::kThreads, L::kSmem, st>>>(c, a, h, sp, err);
+    if (!n || !configure(walk_tc_many_kernel<T, K>, L::kSmem, configured)) return 0;
+    walk_tc_many_kernel<T, K><<<ctas, Role<T>::kThreads, L::kSmem, st>>>(wins, n, h);
     return 1;
+}
+
+uint32_t walk_tc_ctas(uint32_t cands) { return (cands + kCands - 1) / kCands; }
+
+int launch_walk_tc32_many(const WalkTcWin<uint32_t> *wins, uint32_t n, uint32_t ctas, int shape, const HitBuf &h,
+                          cudaStream_t st) {
+    return shape ? launch_many<Cls32, 64>(wins, n, ctas, h, st) : launch_many<Cls32, 48>(wins, n, ctas, h, st);
+}
+int launch_walk_tc64_many(const WalkTcWin<uint64_t> *wins, uint32_t n, uint32_t ctas, int shape, bool lazy,
+                          const HitBuf &h, cudaStream_t st) {
+    if (lazy) return shape ? launch_many<Cls64L, 64>(wins, n, ctas, h, st) : launch_many<Cls64L, 48>(wins, n, ctas, h, st);
+    return shape ? launch_many<Cls64, 64>(wins, n, ctas, h, st) : launch_many<Cls64, 48>(wins, n, ctas, h, st);
 }
 
 template <class T>
@@ -1047,7 +1146,7 @@ static int launch_tc(const ClassBuf<typename T::W> &c, WalkTcArgs a, uint32_t to
     if (!c.cap || a.hi <= a.lo) return 0;
     SplitArgs<typename T::W> one{};
     one.n = 1;
-    a.nb = walk_tc_block(top);
+    walk_tc_args(a, top);
     if (word_depth(top) == 48) return launch_tc<T, 48>(c, a, h, sp ? *sp : one, err, st);
     return launch_tc<T, 64>(c, a, h, sp ? *sp : one, err, st);
 }

@@ -72,3 +72,30 @@ def test_many_hits(mode):
     """p not far above n: hits in every block, and candidates that n passes (their residue is 0 from there)."""
     args = (mode, 101, 90000, 2**16, 160000)
     same(segment(*args, True), segment(*args, False))
+
+
+@pytest.mark.parametrize("budget,work", [(0, None), (96 << 20, None), (0, 2e8)])
+def test_batches(budget, work):
+    """Windows of many searches in one launch: every mode and class, both word shapes, timelines that end in a
+    window and that go on, and (small budget) tables that take several passes."""
+    searches = [(m, n0, n0 + ln, p, p + span) for m, n0, ln, p, span in (
+        (1, 101, 30000, 10**9, 60000), (5, 500, 20000, 2**31 - 40000, 90000), (2, 300000, 90000, 2**50, 30000),
+        (4, 200000, 9000, 2**62, 130000), (5, 1000, 12000, 3 * 2**62, 50000), (1, 20000, 70000, 2**40, 9000),
+        (4, 101, 300, 10**9, 100000), (2, 101, 200000, 2**64 // 3 + 10**6, 40000))]
+
+    def run(on):
+        with pfc.Context(0, budget=budget) as ctx:
+            ctx.set_walk_tc(2 * on)
+            with pfc.Batch(ctx, work) as batch:
+                ids = [batch.submit(*s) for s in searches]
+                batch.run()
+                out = []
+                for i in ids:
+                    st = batch.status(i)
+                    out.append((st.status, st.term_checksum, st.primecount, st.pairs,
+                                o.sort_factors(batch.hits(i)).tobytes()))
+                return out
+
+    got = run(True)
+    assert got == run(False)
+    assert all(r[0] == 0 for r in got) and any(r[4] for r in got)
