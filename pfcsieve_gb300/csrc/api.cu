@@ -44,6 +44,8 @@ struct pfc_job {
     // fp16 tiles on first use
     TcProg tcp[2];
     uint64_t tc_words = 0;        // 896-bit words of the search's programs (both)
+    bool top_tc = false;          // segments from 2^64/3 on set up on the tensor cores
+    bool narrow = false;          // a64 and b64 are there (ensure_narrow)
     DArr<uint8_t> tct;
     DArr<uint32_t> tc_src, tc_groups;
     Prog<WideWord> tc_view[2] = {};
@@ -471,7 +473,13 @@ extern "C" int pfc_job_create(pfc_ctx *c, unsigned mode, uint32_t nmin, uint32_t
     const bool needw = pmax > kClassSplit && pmin < kLazyEnd;
     const bool need64 = pmax > kLazyEnd;
     // class 32 and class 64 below 2^64/3 share the 896-bit programs
-    const std::shared_ptr<const ProgSet> ps = ctx_progs(c, mode, startN, need32 || needw, need64);
+    // (and from there on too, on the tensor cores; the 64-bit words that the
+    // integer pipe takes there are then built when something asks for them)
+    const bool top = need64 && c->setup_tc && startN >= kTcMinStartTop;
+    std::shared_ptr<const ProgSet> ps = ctx_progs(c, mode, startN, need32 || needw || top, need64 && !top);
+    j->top_tc = ps && top && ps->wa.words.size() + ps->wb.words.size() >= kTcMinWordsTop;
+    j->narrow = need64 && !j->top_tc;
+    if (ps && top && !j->top_tc) ps = ctx_progs(c, mode, startN, need32 || needw, true);
     if (!ps) {
         delete j;
         return PFC_ERR_ARG;
@@ -479,17 +487,18 @@ extern "C" int pfc_job_create(pfc_ctx *c, unsigned mode, uint32_t nmin, uint32_t
     const HostProg<WideWord> empty_w;
     const HostProg<uint64_t> empty_n;
     const HostProg<WideWord> &a32 = need32 ? ps->wa : empty_w, &b32 = need32 ? ps->wb : empty_w;
-    const HostProg<WideWord> &aw = needw ? ps->wa : empty_w, &bw = needw ? ps->wb : empty_w;
-    const HostProg<uint64_t> &a64 = need64 ? ps->na : empty_n, &b64 = need64 ? ps->nb : empty_n;
+    const bool wide = needw || j->top_tc;
+    const HostProg<WideWord> &aw = wide ? ps->wa : empty_w, &bw = wide ? ps->wb : empty_w;
+    const HostProg<uint64_t> &a64 = j->narrow ? ps->na : empty_n, &b64 = j->narrow ? ps->nb : empty_n;
     j->setup_mulmods32 = a32.mulmods() + b32.mulmods();
     j->setup_mulmods64 = need64 ? a64.mulmods() + b64.mulmods() : aw.mulmods() + bw.mulmods();
 
     j->tc_words = ps->wa.words.size() + ps->wb.words.size();
-    if ((needw && j->tc_words >= kTcMinWords64) || (need32 && j->tc_words >= kTcMinWords32)) {
-        // the tensor-core setups of both classes use the paired form
-        const HostProg<WideWord> *wide[2] = {needw ? &aw : &a32, needw ? &bw : &b32};
+    if ((needw && j->tc_words >= kTcMinWords64) || (need32 && j->tc_words >= kTcMinWords32) || j->top_tc) {
+        // the tensor-core setups of all classes use the paired form
+        const HostProg<WideWord> *pg[2] = {wide ? &aw : &a32, wide ? &bw : &b32};
         for (int k = 0; k < 2; ++k) {
-            if (!build_tc_prog(*wide[k], j->tcp[k])) {
+            if (!build_tc_prog(*pg[k], j->tcp[k])) {
                 delete j;
                 return PFC_ERR_ARG;
             }
@@ -642,14 +651,37 @@ static int tc_prepare(pfc_job *j) {
 }
 
 static bool tc_setup_applies(const pfc_job *j) {
-    return j->use64 && j->seg_hi <= kLazyEnd && j->ctx->setup_tc && j->tc_words >= kTcMinWords64;
+    if (!j->use64 || !j->ctx->setup_tc) return false;
+    return j->seg_hi <= kLazyEnd ? j->tc_words >= kTcMinWords64 : j->top_tc;
 }
 static bool tc_setup32_applies(const pfc_job *j) {
     return j->use32 && j->ctx->setup_tc && j->tc_words >= kTcMinWords32;
 }
 
+// The programs in 64-bit words of a search that reaches 2^64/3, where its
+// tensor-core setup had left them out (not during a capture).
+static int ensure_narrow(pfc_job *j) {
+    if (j->narrow || j->pmax <= kLazyEnd) return PFC_OK;
+    pfc_ctx *c = j->ctx;
+    CK(cudaSetDevice(c->device));
+    const std::shared_ptr<const ProgSet> ps = ctx_progs(c, j->mode, j->nmin - 1, false, true);
+    if (!ps) return PFC_ERR_ARG;
+    CK(j->a64.upload(c, ps->na));
+    CK(j->b64.upload(c, ps->nb));
+    j->setup_mulmods64 = ps->na.mulmods() + ps->nb.mulmods();
+    j->narrow = true;
+    return PFC_OK;
+}
+static bool narrow_setup_applies(const pfc_job *j) {
+    return j->use64 && j->seg_hi > kLazyEnd && !tc_setup_applies(j);
+}
+
 static int enqueue_setup(pfc_job *j) {
     pfc_ctx *c = j->ctx;
+    if (narrow_setup_applies(j)) {
+        const int rc = ensure_narrow(j);
+        if (rc) return rc;
+    }
     CK(cudaMemsetAsync(&j->stats.p->tc_err, 0, sizeof(uint32_t), c->st));   // of this segment's tensor-core kernels
     SetupArgs<WideWord> s32;
     s32.mode = j->mode;
@@ -689,7 +721,8 @@ static int enqueue_setup(pfc_job *j) {
             SetupArgs<WideWord> stc = sw;
             stc.a = j->tc_view[0];
             stc.b = j->tc_view[1];
-            c->launches += launch_setup64w_tc(j->c64.view(counts_ptr(j) + 1), stc, ta, tb, &j->stats.p->tc_err, c->st);
+            c->launches += launch_setup64_tc(j->c64.view(counts_ptr(j) + 1), stc, ta, tb, j->seg_hi <= kLazyEnd,
+                                             &j->stats.p->tc_err, c->st);
         } else if (j->seg_hi <= kLazyEnd) {
             c->launches += launch_setup64w(j->c64.view(counts_ptr(j) + 1), sw, c->st);
         } else {
@@ -1219,6 +1252,10 @@ static int segment_body_graph(pfc_job *j) {
         const int rc = tc_prepare(j);
         if (rc) return rc;
     }
+    if (narrow_setup_applies(j)) {
+        const int rc = ensure_narrow(j);
+        if (rc) return rc;
+    }
     {
         const uint64_t n32 = j->c32.p.p ? j->c32.cap : 0, n64 = j->c64.p.p ? j->c64.cap : 0;
         const uint32_t L = chunk_steps(j, n32, n64);
@@ -1436,7 +1473,8 @@ extern "C" int pfc_segment_state(pfc_job *j, uint64_t *p, uint64_t *s0, uint64_t
 extern "C" uint64_t pfc_job_pairs(pfc_job *j) { return j ? j->pairs : 0; }
 
 extern "C" uint64_t pfc_job_setup_mulmods(pfc_job *j, int cls64) {
-    return j ? (cls64 ? j->setup_mulmods64 : j->setup_mulmods32) : 0;
+    if (!j || (cls64 && ensure_narrow(j) != PFC_OK)) return 0;
+    return cls64 ? j->setup_mulmods64 : j->setup_mulmods32;
 }
 
 // ------------------------------------------------------- table self-check
@@ -1497,6 +1535,10 @@ extern "C" int pfc_job_verify_tables(pfc_job *j, uint64_t *table_bytes) {
     pfc_ctx *c = j->ctx;
     CK(cudaSetDevice(c->device));
     CK(cudaStreamSynchronize(c->st));
+    {
+        const int nrc = ensure_narrow(j);
+        if (nrc) return nrc;
+    }
     const uint32_t startN = j->nmin - 1;
     // slow side for the setup programs: k in [2, n0 - 1]
     SlowProducts sp;

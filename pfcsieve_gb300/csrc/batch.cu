@@ -410,6 +410,7 @@ struct BatchJob {
     // first program then the second's; tc_nw counts the 896-bit words of the
     // first program, tc_pw the paired words of each)
     std::vector<uint32_t> tcsrc, tcgroups;
+    bool tc_top = false;      // class 64 reaches 2^64/3 and sets up on the tensor cores
     uint32_t tc_second = 0;   // first word of the second program
     uint32_t tc_ng[2] = {0, 0}, tc_fsq[2] = {0, 0}, tc_nw[2] = {0, 0}, tc_pw[2] = {0, 0}, tc_ntiles[2] = {0, 0};
     uint64_t tc_corr[2] = {0, 0};
@@ -489,19 +490,24 @@ static uint32_t prime_limit(const BatchJob *j) {
 
 // Host tables of one search: the same programs, prime lists and multiplier
 // table pfc_job_create builds (from the batch's shared prime list).
-static void prepare_job(BatchJob *j, const std::vector<uint32_t> &cache) {
+static void prepare_job(BatchJob *j, const std::vector<uint32_t> &cache, bool setup_tc) {
     const uint32_t startN = j->nmin - 1;
     const std::vector<uint32_t> primes(cache.begin(), std::upper_bound(cache.begin(), cache.end(), prime_limit(j)));
     const std::vector<uint32_t> below(primes.begin(), std::upper_bound(primes.begin(), primes.end(), startN));
     const unsigned mode = j->mode;
     const bool fc = mode == (PFC_FACTORIAL | PFC_COMPOSITORIAL);
-    const bool wide = j->pmax <= kLazyEnd;  // class 64 with 896-bit words
     HostProg<WideWord> a32, b32;
     HostProg<uint64_t> a64, b64;
-    HostProg<WideWord> aw, bw;
-    const bool ok = build_progs(mode, startN, primes, below, a32, b32) &&
-                    (wide ? build_progs(mode, startN, primes, below, aw, bw)
-                          : build_progs(mode, startN, primes, below, a64, b64));
+    // class 64 with 896-bit words: below 2^64/3, and from there on with a
+    // program and walk that take the tensor-core setup (decided here)
+    const bool ok32 = build_progs(mode, startN, primes, below, a32, b32);
+    j->tc_top = j->pmax > kLazyEnd && setup_tc && j->nmax > j->nmin &&
+                a32.words.size() + b32.words.size() >= kTcMinWordsTop &&
+                (mode != PFC_PRIMORIAL ||
+                 std::lower_bound(primes.begin(), primes.end(), j->nmin) != std::lower_bound(primes.begin(), primes.end(), j->nmax));
+    const bool wide = j->pmax <= kLazyEnd || j->tc_top;
+    const HostProg<WideWord> none, &aw = wide ? a32 : none, &bw = wide ? b32 : none;
+    const bool ok = ok32 && (wide || build_progs(mode, startN, primes, below, a64, b64));
     if (!ok) {
         j->prep_rc = PFC_ERR_ARG;
         return;
@@ -530,6 +536,10 @@ static void prepare_job(BatchJob *j, const std::vector<uint32_t> &cache) {
             j->tc_pw[k] = (uint32_t)tp.src.size();
             j->tc_ntiles[k] = (j->tc_pw[k] + tc_tile_words() - 1) / tc_tile_words();
         }
+    }
+    if (j->tc_top && !j->tc) {
+        j->prep_rc = PFC_ERR_ARG;
+        return;
     }
     if (fc) {
         // fork: the compositorial residue is complete here
@@ -699,7 +709,7 @@ void prepare_queued(pfc_batch *b) {
         b->cache_lim = want;
     }
 #pragma omp parallel for schedule(dynamic, 1)
-    for (int64_t k = 0; k < (int64_t)todo.size(); ++k) prepare_job(todo[k], b->prime_cache);
+    for (int64_t k = 0; k < (int64_t)todo.size(); ++k) prepare_job(todo[k], b->prime_cache, b->ctx->setup_tc);
     for (BatchJob *j : todo) j->state = kPrepared;
 }
 
@@ -756,8 +766,9 @@ int upload_job(pfc_batch *b, BatchJob *j) {
     if (e == cudaSuccess) e = j->d_words64.upload(c, j->words64);
     if (e == cudaSuccess) e = j->d_wordsw.upload(c, j->wordsw);
     const uint64_t words = (uint64_t)j->tc_nw[0] + j->tc_nw[1];
-    const bool tc = j->tc && c->setup_tc &&
-                    ((j->use64 && words >= kTcMinWords64) || (j->use32 && words >= kTcMinWords32));
+    const bool tc = (j->tc && c->setup_tc &&
+                     ((j->use64 && words >= kTcMinWords64) || (j->use32 && words >= kTcMinWords32))) ||
+                    j->tc_top;
     const size_t tb = tc_tile_bytes(), nt = (size_t)j->tc_ntiles[0] + j->tc_ntiles[1];
     if (e == cudaSuccess && tc) e = j->d_tcgroups.upload(c, j->tcgroups);
     if (e == cudaSuccess && tc) e = j->d_tcsrc.upload(c, j->tcsrc);
@@ -808,7 +819,8 @@ JobDev<W> job_view(pfc_batch *b, BatchJob *j, const DevClass<W> &cls, int which,
 // [block0, block0 + n) (n 0: all), flags into the search's slot.
 int tc_launch(pfc_batch *b, BatchJob *j, int cls, cudaStream_t st, uint32_t block0, uint32_t n) {
     BatchStats *bs = b->stats.p + j->slot;   // device address
-    return cls ? launch_setup64w_tc(j->c64.view(bs->counts + 1), j->tc_args, j->tc_ta, j->tc_tb, &bs->flags, st, block0, n)
+    return cls ? launch_setup64_tc(j->c64.view(bs->counts + 1), j->tc_args, j->tc_ta, j->tc_tb, j->pmax <= kLazyEnd,
+                                   &bs->flags, st, block0, n)
                : launch_setup32_tc(j->c32.view(bs->counts), j->tc_args, j->tc_ta, j->tc_tb, &bs->flags, st, block0, n);
 }
 
@@ -890,13 +902,13 @@ int admit_prepared(pfc_batch *b) {
     // chunks of candidate blocks ahead of each iteration (launch_iteration),
     // within a share of the iteration's budget, so that small searches are
     // not held up behind large setups.
-    if (c->setup_tc) {
+    {
         bool waited[pfc_batch::kTcStreams] = {};
         CK(cudaEventRecord(b->ev_tc0, c->st));
         for (BatchJob *j : fresh) {
             // (a timeline without walk steps keeps its setup windows: the
             // window that ends it also adds the check terms)
-            if (!j->d_tct.p || !j->nwalk) continue;
+            if (!j->d_tct.p || !j->nwalk || !(c->setup_tc || j->tc_top)) continue;
             SetupArgs<WideWord> &sw = j->tc_args;
             memset(&sw, 0, sizeof(sw));
             sw.mode = j->mode;
@@ -916,7 +928,8 @@ int admit_prepared(pfc_batch *b) {
             for (int cls = 0; cls < 2; ++cls) {
                 const uint32_t n = cls ? j->n64 : j->n32;
                 // small programs keep their setup windows (kernels.cuh kTcMinWords*)
-                if (!n || words < (cls ? kTcMinWords64 : kTcMinWords32)) continue;
+                if (!n || (words < (cls ? kTcMinWords64 : kTcMinWords32) && !(cls && j->tc_top))) continue;
+                if (!cls && !c->setup_tc) continue;
                 j->tc_blocks[cls] = cls ? tc_setup_blocks(n) : tc_setup_blocks32(n);
                 j->tc_block_cost[cls] = kTcTileCost * ((double)j->tc_ntiles[0] + j->tc_ntiles[1] + kTcFixedTiles);
                 (cls ? j->pos64 : j->pos32) = cls ? j->nsetup64 : j->nsetup32;

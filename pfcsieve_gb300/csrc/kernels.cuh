@@ -151,9 +151,10 @@ int launch_tc_pack(const WideWord *words, const uint32_t *src, uint32_t nw, uint
                    cudaStream_t st);
 // (candidate blocks of 64: [block0, block0 + nblocks), nblocks 0 to the end)
 uint32_t tc_setup_blocks(uint32_t cands);
-int launch_setup64w_tc(const ClassBuf<uint64_t> &c, const SetupArgs<WideWord> &a, const TcTiles &ta,
-                       const TcTiles &tb, uint32_t *err, cudaStream_t st, uint32_t block0 = 0,
-                       uint32_t nblocks = 0);
+// (lazy: every candidate is below 2^64/3)
+int launch_setup64_tc(const ClassBuf<uint64_t> &c, const SetupArgs<WideWord> &a, const TcTiles &ta,
+                      const TcTiles &tb, bool lazy, uint32_t *err, cudaStream_t st, uint32_t block0 = 0,
+                      uint32_t nblocks = 0);
 // class 32 on the same tiles (the class-32 and lazy class-64 programs are the same)
 uint32_t tc_setup_blocks32(uint32_t cands);
 // Smallest programs (896-bit words, both programs of the search) set up on the
@@ -166,6 +167,12 @@ uint32_t tc_setup_blocks32(uint32_t cands);
 // 0.54 / 0.44, at 2,265 3.77 / 0.79.
 constexpr uint64_t kTcMinWords32 = 240;
 constexpr uint64_t kTcMinWords64 = 216;
+// From 2^64/3 on, where the integer pipe takes 64-bit words: at 78 words 0.213 /
+// 0.255 ms, at 145 0.394 / 0.257, at 2,265 6.52 / 0.58; over a 3e7-wide range
+// at 78 words 1.14 / 1.83, at 145 2.16 / 1.84.  Programs for n below
+// kTcMinStartTop do not reach that size.
+constexpr uint64_t kTcMinWordsTop = 112;
+constexpr uint32_t kTcMinStartTop = 40000;
 int launch_setup32_tc(const ClassBuf<uint32_t> &c, const SetupArgs<WideWord> &a, const TcTiles &ta,
                       const TcTiles &tb, uint32_t *err, cudaStream_t st, uint32_t block0 = 0, uint32_t nblocks = 0);
 // start residues of a split walk: boundary k's into s0/s1 + (k-1) * c.cap

@@ -1,7 +1,7 @@
-// setup_tc.cu -- the setup of class-32 candidates and of class-64 candidates
-// below 2^64/3 (the lazy class) with the table-word fold on the tensor cores
-// (tcgen05), for programs of at least kTcMinWords32 / kTcMinWords64 words
-// (kernels.cuh).  The description below is of class 64; class 32 follows it.
+// setup_tc.cu -- the setup of the candidates' residues with the table-word fold
+// on the tensor cores (tcgen05), for programs of at least kTcMinWords32 / 64 /
+// Top words (kernels.cuh).  The description below is of class 64 below 2^64/3
+// (the lazy class); the other classes follow it.
 //
 // The setup evaluates a program of table words Z (products of primes,
 // kernels.cuh Prog) into each candidate's residue.  The costly part on the
@@ -44,10 +44,9 @@
 // through shared memory.  So a tile needs no barrier among the threads.
 // Class 32 (p < 2^31) runs the same kernel with 4 planes, 64 candidates per CTA
 // (N = 64 x 4 = 256 again), T' < 2^48 reduced by one 32-bit round and one
-// Montgomery product (R = 2^32) per word.  The result equals
-// setup_kernel<Cls64L>'s or setup_kernel<Cls32>'s: the same product of the
-// same words in the same Horner order, exact arithmetic, canonical residues
-// at the end.  Every wait is bounded; after one that gave up the kernel sets
+// Montgomery product (R = 2^32) per word; class 64 from 2^64/3 on keeps
+// canonical residues.  The result equals setup_kernel's: the same product,
+// exact arithmetic, canonical residues at the end.  Every wait is bounded; after one that gave up the kernel sets
 // bit 1 of `flags`, frees its TMEM and stores nothing.
 #include <cuda_runtime.h>
 
@@ -163,6 +162,43 @@ struct TcClass<Cls64L> {
         return cios_round(redc64l(s, (uint32_t)u, c.p, c.q), s, (uint32_t)(u >> 32), c.p, c.q);
     }
     __device__ static __forceinline__ W canon(W s, const Cand &c) { return s >= c.p ? s - c.p : s; }
+};
+
+// class 64 from 2^64/3: canonical residues, R = 2^64
+template <>
+struct TcClass<Cls64> {
+    using W = uint64_t;
+    using M = Mont64;
+    static constexpr int kPlanes = 8;
+    static constexpr uint64_t kIdle = TcClass<Cls64L>::kIdle;
+    struct __align__(16) Cand {
+        W p, q;   // p^-1 mod 2^64
+    };
+    __device__ static __forceinline__ Cand cand(const M &m) { return {m.p, m.pinv}; }
+    __device__ static __forceinline__ W power(const M &m, uint32_t bits) {
+        const uint32_t k = (bits + 63) / 64, down = 64 * k - bits;
+        const W x = m.mont_R_pow(k - 1);
+        return down ? m.mul(x, 1ull << (64 - down)) : x;
+    }
+    __device__ static __forceinline__ W div256(const M &m, W x) { return m.mul(x, 1ull << 56); }
+    __device__ static __forceinline__ W bias(const M &m) { return TcClass<Cls64L>::bias(m); }
+    // (eight digits hold -0x8080.. .. 0x7F7F.., 2^64 values)
+    __device__ static __forceinline__ W digits(W w, W p) {
+        return (w > 0x7F7F7F7F7F7F7F7Full ? w - p : w) + 0x8080808080808080ull;
+    }
+    // as the lazy class, where (T' mod 2^32 + m p) / 2^32 is at most p and the
+    // rest of T' below 2^48: less p where the sum passes it
+    __device__ static __forceinline__ W reduce(const uint32_t (&t)[4], const Cand &c) {
+        const uint64_t L = (uint64_t)t[0] + ((uint64_t)t[1] << 16), H = (uint64_t)t[2] + ((uint64_t)t[3] << 16);
+        const uint32_t tw0 = (uint32_t)L;
+        const uint64_t Mh = (L >> 32) + H;
+        const uint32_t mm = 0u - tw0 * (uint32_t)c.q;
+        const uint64_t lo = (uint64_t)mm * (uint32_t)c.p;
+        const uint64_t u = (uint64_t)mm * (uint32_t)(c.p >> 32) + (lo >> 32) + (tw0 != 0 ? 1u : 0u) + Mh;
+        return u < Mh || u >= c.p ? u - c.p : u;
+    }
+    __device__ static __forceinline__ W prod(W s, W u, const Cand &c) { return redc64(s, u, c.p, c.q); }
+    __device__ static __forceinline__ W canon(W s, const Cand &) { return s; }
 };
 
 // class 32: canonical residues, R = 2^32
@@ -586,9 +622,10 @@ static int launch_tc(const ClassBuf<typename TcClass<T>::W> &c, const SetupArgs<
     return 1;
 }
 
-int launch_setup64w_tc(const ClassBuf<uint64_t> &c, const SetupArgs<WideWord> &a, const TcTiles &ta,
-                       const TcTiles &tb, uint32_t *flags, cudaStream_t st, uint32_t block0, uint32_t nblocks) {
-    return launch_tc<Cls64L>(c, a, ta, tb, flags, st, block0, nblocks);
+int launch_setup64_tc(const ClassBuf<uint64_t> &c, const SetupArgs<WideWord> &a, const TcTiles &ta,
+                      const TcTiles &tb, bool lazy, uint32_t *flags, cudaStream_t st, uint32_t block0, uint32_t nblocks) {
+    return lazy ? launch_tc<Cls64L>(c, a, ta, tb, flags, st, block0, nblocks)
+                : launch_tc<Cls64>(c, a, ta, tb, flags, st, block0, nblocks);
 }
 
 int launch_setup32_tc(const ClassBuf<uint32_t> &c, const SetupArgs<WideWord> &a, const TcTiles &ta,
