@@ -151,8 +151,8 @@ int slow_products(pfc_ctx *c, uint64_t lo, uint64_t hi, SlowProducts &out) {
 // shared memory, the power of R fixed once.  Below 2^31 the arithmetic is
 // 32-bit.
 //
-// What bounds it is the multiply pipe, where a wide multiply takes four times
-// as long as a plain one, so the reductions per k are what counts.  Every k:
+// What bounds it is the multiply pipe, where a wide multiply takes more than twice
+// as long as a plain one: the reductions per k are what counts.  Every k:
 // the products of D consecutive k are a polynomial of degree D in the first,
 // tabulated by finite differences, D modular additions and one product for D
 // of them (D = 4 below 2^31, 8 above).  Composites: above 2^31 two of them in

@@ -58,13 +58,16 @@
 //
 // What bounds it: the CUDA cores' issue slots and their ALU pipe (byte permutes
 // and packed minima).  Cycles per 32 candidates and step on an SM's quarter,
-// 4.8e5 (class 32) and 1.2e5 candidates, per-step kernels to this one: class
-// 32 17.7 to 13.4 (words of 47 digits), 19.6 to 14.4 (63); class 64 35.9 to
-// 18.2 (63), 38.3 to 19.3 (47), from 2^64/3 (3.0e5 candidates) 69.5 to 20.3.  At
-// that rate 68% of the issue slots are used,
-// the ALU 58% of the time, the tensor cores 30 to 36%.  A CTA's fixed part,
-// about 1,500 steps long, is planes (7 to 14 thousand cycles), the first
-// products' way through the roles (5 thousand), and the last replays.
+// per-step kernels to this one: class 32 (4.8e5 candidates) 17.7 to 12.5 (words
+// of 47 digits), 19.6 to 13.4 (63); class 64 (1.2e5) 35.9 to 18.0 (63), 38.3 to
+// 19.0 (47), from 2^64/3 (3.0e5) 69.5 to 20.5.  At that rate about 70% of the
+// issue slots are used, the ALU 60% of the time, the tensor cores 30 to 36%.
+// (The testers' loop runs over whole units, unrolled, and a suspect's residue
+// is read only when there is one: a tile at a time took 13.4 cycles in class
+// 32, 11% more instructions; the reducers' and the chain's unrolled units 18.3
+// to 18.0 in class 64.)  A CTA's fixed part, about 1,500 steps long, is planes
+// (7 to 14 thousand cycles), the first products' way through the roles (5
+// thousand), and the last replays.
 //
 // Every wait is bounded; when one gives up the CTA raises bit 2 of *err,
 // waits (bounded) for its copies, frees its TMEM and stores nothing.
@@ -705,84 +708,87 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
         volatile uint32_t *qs = reinterpret_cast<uint32_t *>(sm + L::kOffQs);
         const W *rs = reinterpret_cast<const W *>(sm + L::kOffR) + b0 * kCands + cl;
         const uint32_t col = tbase + lanes + L::kColDF + buf * L::kDF + b0 * 16;
-        const uint32_t window = 2 * half;
+        const uint32_t window = 2 * half, window2 = window * 0x10001u;
         const uint32_t sh = C::shift(m.p);
         const float scale = C::kScale / ldexpf((float)m.p, -(int)sh);
         uint32_t tph = 0, unit = 0, rph = 0;
-        for (uint32_t t = buf; t < ntiles; t += kBufs) {
-            if (t % C::kUnit == buf) warp_wait(bar_r(unit), rph, fail);   // the unit's first tile of this group
-            const W *rt = rs + (unit * C::kUnit + t % C::kUnit) * L::kRTile;
-            W r[kB + 1];   // residues at the blocks' starts and at the last one's end
+        for (uint32_t t0 = 0; t0 < ntiles; t0 += C::kUnit) {   // (whole units; a stream's tiles are)
+            warp_wait(bar_r(unit), rph, fail);
+            const W *ru = rs + unit * (C::kUnit * L::kRTile);
 #pragma unroll
-            for (int b = 0; b <= kB; ++b) r[b] = rt[b * kCands];
-            uint32_t A[kB];   // in both halves (16 bits, from 22 or 21 + 1)
-#pragma unroll
-            for (int b = 0; b < kB; ++b) {
-                const uint32_t f = __float_as_uint(fmaf(C::value(r[b + 1], sh), scale, 12582912.0f)) >> C::kShift;
-                A[b] = __byte_perm(f, f, 0x1010);
-            }
-            warp_wait(bar_t(buf), tph, fail);
-            tph ^= 1;
-            fence_after();
-            uint32_t vh[16], vl[16];
-            ld16(col, vh);
-            ld16(col + kRowsTile, vl);
-            uint32_t mb[kB];
-#pragma unroll
-            for (int b = 0; b < kB; ++b) {
-                wait_ld();
-                uint32_t w[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j)   // bits 8..23 of two neighbours
-                    w[j] = __byte_perm(vh[2 * j] * 4096u + vl[2 * j], vh[2 * j + 1] * 4096u + vl[2 * j + 1], 0x6521);
-                if (b + 1 < kB) {   // the next block's sums arrive meanwhile
-                    ld16(col + 16 * (b + 1), vh);
-                    ld16(col + kRowsTile + 16 * (b + 1), vl);
-                } else {
-                    fence_before();
-                    __syncwarp();
-                    if (lane == 0) {
-                        mbar_arrive(bar_tf(buf));
-                        if (t % C::kUnit == C::kUnit - kBufs + buf) mbar_arrive(bar_rf(unit));   // the unit's last
-                    }
-                }
-                uint32_t m0 = ~0u, m1 = ~0u;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    m0 = __viaddmin_u16x2(w[j], ~A[b], m0);   // X - A + half
-                    m1 = __viaddmin_u16x2(w[j], A[b], m1);    // X + A + half + 1
-                }
-                mb[b] = __viaddmin_u16x2(m0, 0u, m1);
-            }
-            if (t % C::kUnit == C::kUnit - kBufs + buf && ++unit == (uint32_t)C::kRUnits) {
-                unit = 0;
-                rph ^= 1;
-            }
-            const uint32_t least = __viaddmin_u16x2(mb[0], 0u, mb[1]);
-            if (__any_sync(kFull, min(least & 0xFFFFu, least >> 16) <= window)) {   // queue the suspects
+            for (uint32_t i = 0; i < (uint32_t)C::kUnit / kBufs; ++i) {   // this group's tiles of the unit
+                const W *rt = ru + (buf + i * kBufs) * L::kRTile;   // residues: its blocks' starts, the last one's end
+                uint32_t A[kB];   // in both halves (16 bits, from 22 or 21 + 1)
 #pragma unroll
                 for (int b = 0; b < kB; ++b) {
-                    const unsigned ps = __ballot_sync(kFull, act && min(mb[b] & 0xFFFFu, mb[b] >> 16) <= window);
-                    if (!ps) continue;
-                    uint32_t i = 0;
-                    if (lane == 0) i = atomicAdd(suspects, (uint32_t)__popc(ps));
-                    i = __shfl_sync(kFull, i, 0) + __popc(ps & ((1u << lane) - 1u));
-                    if ((ps >> lane) & 1u) {
-                        const uint32_t round = i / (32 * kBatches), e = i % (32 * kBatches);
-                        // room once the batch's previous round has been replayed
-                        for (uint32_t it = 0; reinterpret_cast<volatile uint32_t *>(replayed)[e / 32] < round; ++it)
-                            if (*failed || it >= 8 * kWaitLimit) {
-                                *failed = 1;
-                                break;
-                            }
-                        const uint32_t s = t >= tiles ? 1u : 0u;
-                        qr[e] = r[b];
-                        qk[e] = (s << 31) | (((t - (s ? tiles : 0u)) * kBlocksTile + b0 + b) << 7) | cl;
-                        __threadfence_block();
-                        qs[e] = round + 1;
-                    }
-                    __syncwarp();
+                    const uint32_t f =
+                        __float_as_uint(fmaf(C::value(rt[(b + 1) * kCands], sh), scale, 12582912.0f)) >> C::kShift;
+                    A[b] = __byte_perm(f, f, 0x1010);
                 }
+                warp_wait(bar_t(buf), tph, fail);
+                tph ^= 1;
+                fence_after();
+                uint32_t vh[16], vl[16];
+                ld16(col, vh);
+                ld16(col + kRowsTile, vl);
+                uint32_t mb[kB];
+#pragma unroll
+                for (int b = 0; b < kB; ++b) {
+                    wait_ld();
+                    uint32_t w[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)   // bits 8..23 of two neighbours
+                        w[j] = __byte_perm(vh[2 * j] * 4096u + vl[2 * j], vh[2 * j + 1] * 4096u + vl[2 * j + 1], 0x6521);
+                    if (b + 1 < kB) {   // the next block's sums arrive meanwhile
+                        ld16(col + 16 * (b + 1), vh);
+                        ld16(col + kRowsTile + 16 * (b + 1), vl);
+                    } else {
+                        fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar_tf(buf));
+                    }
+                    uint32_t m0 = ~0u, m1 = ~0u;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        m0 = __viaddmin_u16x2(w[j], ~A[b], m0);   // X - A + half
+                        m1 = __viaddmin_u16x2(w[j], A[b], m1);    // X + A + half + 1
+                    }
+                    mb[b] = __viaddmin_u16x2(m0, 0u, m1);
+                }
+                // the least of both halves, in both
+                uint32_t least = __viaddmin_u16x2(mb[0], 0u, mb[1]);
+                least = __viaddmin_u16x2(least, 0u, __byte_perm(least, least, 0x1032));
+                if (__any_sync(kFull, least <= window2)) {   // queue the suspects
+                    const uint32_t t = t0 + buf + i * kBufs;
+#pragma unroll
+                    for (int b = 0; b < kB; ++b) {
+                        const unsigned ps = __ballot_sync(kFull, act && min(mb[b] & 0xFFFFu, mb[b] >> 16) <= window);
+                        if (!ps) continue;
+                        uint32_t at = 0;
+                        if (lane == 0) at = atomicAdd(suspects, (uint32_t)__popc(ps));
+                        at = __shfl_sync(kFull, at, 0) + __popc(ps & ((1u << lane) - 1u));
+                        if ((ps >> lane) & 1u) {
+                            const uint32_t round = at / (32 * kBatches), e = at % (32 * kBatches);
+                            // room once the batch's previous round has been replayed
+                            for (uint32_t it = 0; reinterpret_cast<volatile uint32_t *>(replayed)[e / 32] < round; ++it)
+                                if (*failed || it >= 8 * kWaitLimit) {
+                                    *failed = 1;
+                                    break;
+                                }
+                            const uint32_t s = t >= tiles ? 1u : 0u;
+                            qr[e] = rt[b * kCands];
+                            qk[e] = (s << 31) | (((t - (s ? tiles : 0u)) * kBlocksTile + b0 + b) << 7) | cl;
+                            __threadfence_block();
+                            qs[e] = round + 1;
+                        }
+                        __syncwarp();
+                    }
+                }
+            }
+            if (lane == 0) mbar_arrive(bar_rf(unit));
+            if (++unit == (uint32_t)C::kRUnits) {
+                unit = 0;
+                rph ^= 1;
             }
         }
         __syncwarp();
@@ -809,7 +815,7 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
                 warp_wait(bar_e(ge), eph, fail);
                 fence_after();
                 if (un >= (uint32_t)C::kUUnits) warp_wait(bar_uf(us0), uph, fail);
-#pragma unroll 1
+#pragma unroll
                 for (uint32_t i = 0; i < (uint32_t)C::kUnit; ++i) {
                     uint32_t v[C::kPlanes][4];
 #pragma unroll
@@ -866,7 +872,7 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
             for (uint32_t ul = 0; ul < units; ++ul, ++un) {
                 warp_wait(bar_u(us0), uph, fail);
                 if (un >= (uint32_t)C::kRUnits) warp_wait(bar_rf(slot), phase, fail);
-#pragma unroll 1
+#pragma unroll
                 for (uint32_t i = 0; i < (uint32_t)C::kUnit; ++i) {
                     typename C::U u[4];
 #pragma unroll
