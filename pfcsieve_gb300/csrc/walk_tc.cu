@@ -50,22 +50,21 @@
 // takes 32 cycles, with A in shared memory 48), the residue's in TMEM (class
 // 32) or shared memory (class 64, where TMEM is full).  Roles: 16 warps test
 // (four groups of a thread per candidate, two groups per buffer, two blocks of
-// each tile), one (class 64: two) groups of four warps reduce the block
-// products, four warps carry the residues, two warps copy words and issue the
-// tests' MMAs, one the residues', four (one) replay.  Chain, reduction and
-// tests run in units of tiles, handed over through shared memory, so that a
-// role waits once per unit and not once per tile.
+// each tile), in class 32 four warps reduce the block products and four carry
+// the residues, in class 64 three groups of four do both in turn, two warps copy
+// words and issue the tests' MMAs, one the residues', four (one) replay.  Chain,
+// reduction and tests run in units of tiles, handed over through shared memory,
+// so that a role waits once per unit and not once per tile.
 //
 // What bounds it: the CUDA cores' issue slots and their ALU pipe (byte permutes
 // and packed minima).  Cycles per 32 candidates and step on an SM's quarter,
 // per-step kernels to this one: class 32 (4.8e5 candidates) 17.7 to 12.5 (words
-// of 47 digits), 19.6 to 13.4 (63); class 64 (1.2e5) 35.9 to 18.0 (63), 38.3 to
-// 19.0 (47), from 2^64/3 (3.0e5) 69.5 to 20.5.  At that rate about 70% of the
+// of 47 digits), 19.6 to 13.4 (63); class 64 (1.2e5) 35.9 to 17.0 (63), 38.3 to
+// 17.9 (47), from 2^64/3 (3.0e5) 69.5 to 20.4.  At that rate about 70% of the
 // issue slots are used, the ALU 60% of the time, the tensor cores 30 to 36%.
 // (The testers' loop runs over whole units, unrolled, and a suspect's residue
 // is read only when there is one: a tile at a time took 13.4 cycles in class
-// 32, 11% more instructions; the reducers' and the chain's unrolled units 18.3
-// to 18.0 in class 64.)  A CTA's fixed part, about 1,500 steps long, is planes
+// 32, 11% more instructions.)  A CTA's fixed part, about 1,500 steps long, is planes
 // (7 to 14 thousand cycles), the first products' way through the roles (5
 // thousand), and the last replays.
 //
@@ -129,7 +128,7 @@ struct ChainClass<Cls32> {
     static constexpr bool kInTmem = true;      // 3 planes of K / 2 columns
     static constexpr int kBlocksE = 16;        // blocks per MMA of the residues, in
     static constexpr int kBufsE = 2;           // two buffers of sums
-    static constexpr int kReduceGroups = 1, kReplayWarps = 4;
+    static constexpr int kReduceGroups = 1, kChainGroups = 1, kReplayWarps = 4;
     static constexpr int kUnit = 4, kUUnits = 2, kRUnits = 3;   // tiles the chain takes at a time; units kept
     static constexpr uint32_t kIdle = 0x7FFFFFFFu;
     static constexpr float kScale = 4194304.0f;   // 2^22: |r| < p
@@ -176,8 +175,8 @@ struct ChainClass<Cls64L> {
     static constexpr bool kInTmem = false;
     static constexpr int kBlocksE = 32;
     static constexpr int kBufsE = 1;
-    static constexpr int kReduceGroups = 2, kReplayWarps = 1;
-    static constexpr int kUnit = 2, kUUnits = 4, kRUnits = 4;
+    static constexpr int kReduceGroups = 0, kChainGroups = 3, kReplayWarps = 1;
+    static constexpr int kUnit = 2, kUUnits = 0, kRUnits = 6;
     static constexpr uint64_t kIdle = 0x1FFFFFFFFFFFFFFFull;
     static constexpr float kScale = 2097152.0f;   // 2^21: r < 2p
     static constexpr int kShift = 5;
@@ -225,7 +224,7 @@ struct ChainClass<Cls64> {
     static constexpr int kPlanes = 6;
     static constexpr bool kInTmem = false;
     static constexpr int kBlocksE = L::kBlocksE, kBufsE = L::kBufsE;
-    static constexpr int kReduceGroups = L::kReduceGroups, kReplayWarps = L::kReplayWarps;
+    static constexpr int kReduceGroups = L::kReduceGroups, kChainGroups = L::kChainGroups, kReplayWarps = L::kReplayWarps;
     static constexpr int kUnit = L::kUnit, kUUnits = L::kUUnits, kRUnits = L::kRUnits;
     static constexpr uint64_t kIdle = L::kIdle;
     static constexpr float kScale = 4194304.0f;   // 2^22: r < p
@@ -253,14 +252,14 @@ struct ChainClass<Cls64> {
 };
 
 // Warp roles, in groups of four warps (a thread per candidate): testers
-// (tiles in turn), reducers (quads in turn), the chain; then single warps: the
+// (tiles in turn), reducers (class 32), the chain; then single warps: the
 // tests' MMAs (one per buffer), the residues' MMAs, replays.
 template <class T>
 struct Role {
     using C = ChainClass<T>;
     static constexpr int kReduce = 4 * kTesterGroups;
     static constexpr int kChain = kReduce + 4 * C::kReduceGroups;
-    static constexpr int kTestMma = kChain + 4;
+    static constexpr int kTestMma = kChain + 4 * C::kChainGroups;
     static constexpr int kChainMma = kTestMma + kBufs;
     static constexpr int kReplay = kChainMma + 1;
     static constexpr int kThreads = 32 * (kReplay + C::kReplayWarps);
@@ -496,6 +495,7 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
     uint32_t digits = *a.digits[0];
     if (a.nstreams > 1) digits = max(digits, *a.digits[1]);
     const uint32_t half = (uint32_t)(digits * (0.504f / 256.0f) + 0.045f) + 1u;
+    constexpr uint32_t kBlocksUnit = C::kUnit * kBlocksTile, kUnitsE = C::kBlocksE / kBlocksUnit;   // units per buffer of residue sums
     const uint32_t bar = smem_u32(sm + L::kOffBar);
     constexpr uint32_t kB0 = kFStages + L::kWStages, kB1 = kB0 + 2 * kBufs, kB2 = kB1 + 2 * C::kRUnits,
                        kB3 = kB2 + 2 * L::kBufsE, kB4 = kB3 + 2 * C::kUUnits;
@@ -535,9 +535,9 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
         }
         for (uint32_t i = 0; i < L::kBufsE; ++i) {
             mbar_init(bar_e(i), 1);
-            mbar_init(bar_ef(i), 4 * C::kReduceGroups);
+            mbar_init(bar_ef(i), 4 * (C::kReduceGroups ? C::kReduceGroups : C::kChainGroups));
         }
-        for (uint32_t i = 0; i < C::kUUnits; ++i) {
+        for (int i = 0; i < C::kUUnits; ++i) {
             mbar_init(bar_u(i), 4);
             mbar_init(bar_uf(i), 4);
         }
@@ -628,7 +628,7 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
         }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     } else if (warp < Role<T>::kTestMma) {
-        if (warp >= Role<T>::kChain) {
+        if (warp < Role<T>::kReduce + 4) {
             cand_p[cl] = m.p;
             cand_q[cl] = C::qv(m);
         }
@@ -794,116 +794,171 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
         __syncwarp();
         __threadfence_block();
         if (lane == 0) atomicAdd(testers_done, 1u);
-    } else if (warp < Role<T>::kChain) {
-        // --------------------------------------------------------- reducers
+    } else if (warp < Role<T>::kTestMma) {
+        // ------------------------------------------------ reducers and chain
         const W p = m.p;
         const typename C::Q q = C::qv(m);
-        const uint32_t grp = (warp - Role<T>::kReduce) / 4;
         const uint2 shifts = make_uint2(a.shift11, a.shift22);
-        typename C::U *us = reinterpret_cast<typename C::U *>(sm + L::kOffU) + cl;
-        constexpr int kBlocksUnit = C::kUnit * kBlocksTile;
-        constexpr uint32_t kUnitsE = C::kBlocksE / kBlocksUnit;
+        W *rs = reinterpret_cast<W *>(sm + L::kOffR) + cl;
         const uint32_t units = tiles / C::kUnit;
-        uint32_t ge = 0, eph = 0;           // buffer of sums, its phase
-        uint32_t us0 = 0, uph = 1;          // slot, phase of its release
-        uint32_t ul = 0;                    // unit of the stream
-        for (uint32_t un = 0; un < units * a.nstreams; ++un) {
-            const uint32_t te = ul % kUnitsE;
-            const bool ends = te == kUnitsE - 1 || ul + 1 == units;
-            const bool mine = C::kReduceGroups == 1 || un % C::kReduceGroups == grp;
-            if (mine) {
-                warp_wait(bar_e(ge), eph, fail);
-                fence_after();
-                if (un >= (uint32_t)C::kUUnits) warp_wait(bar_uf(us0), uph, fail);
+        // the block products of tile i of unit te of buffer ge
+        auto reduce_tile = [&](uint32_t ge, uint32_t te, uint32_t i, typename C::U *u) {
+            uint32_t v[C::kPlanes][4];
 #pragma unroll
-                for (uint32_t i = 0; i < (uint32_t)C::kUnit; ++i) {
-                    uint32_t v[C::kPlanes][4];
+            for (int pl = 0; pl < C::kPlanes; ++pl)
+                ld4(tbase + lanes + L::kColDE + ge * L::kDE + pl * C::kBlocksE + te * kBlocksUnit + i * 4, v[pl]);
+            wait_ld();
 #pragma unroll
-                    for (int pl = 0; pl < C::kPlanes; ++pl)
-                        ld4(tbase + lanes + L::kColDE + ge * L::kDE + pl * C::kBlocksE + te * kBlocksUnit + i * 4, v[pl]);
-                    wait_ld();
-                    typename C::U u[4];
+            for (int b = 0; b < 4; ++b) {
+                uint32_t e[C::kPlanes];
 #pragma unroll
-                    for (int b = 0; b < 4; ++b) {
-                        uint32_t e[C::kPlanes];
-#pragma unroll
-                        for (int pl = 0; pl < C::kPlanes; ++pl) e[pl] = v[pl][b];
-                        u[b] = C::reduce(e, p, q, shifts);
-                    }
-#pragma unroll
-                    for (int b = 0; b < 4; ++b) us[(us0 * kBlocksUnit + i * 4 + b) * kCands] = u[b];
-                }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_u(us0));
+                for (int pl = 0; pl < C::kPlanes; ++pl) e[pl] = v[pl][b];
+                u[b] = C::reduce(e, p, q, shifts);
             }
-            if (ends) {
-                if (!mine) {   // (its last unit of the buffer is behind it)
-                    warp_wait(bar_e(ge), eph, fail);
+        };
+        // a stream's first residue, and its last one into place
+        auto second = [&](uint32_t s) { return (s ? a.second[1] : a.second[0]) != 0; };
+        auto start = [&](uint32_t s) -> W {
+            const W *in = second(s) ? c.s1 : c.s0;
+            if (split && sub) in = (second(s) ? sp->s1 : sp->s0) + (size_t)(sub - 1) * sp->pitch;
+            return act ? in[ci] : (W)0;
+        };
+        auto finish = [&](uint32_t s, W r) {
+            if (!act || *failed) return;
+            if (last) (second(s) ? c.s1 : c.s0)[ci] = T::canon(m, r);
+            atomicAdd(c.nnext + ci, hi - lo);   // (the streams' ends may fall to two groups)
+        };
+        if constexpr (C::kReduceGroups != 0) {
+            // Class 32: one group reduces, one moves the residues.  A buffer of
+            // sums is a unit.
+            static_assert(C::kReduceGroups == 0 || kUnitsE == 1, "one unit a buffer");
+            typename C::U *us = reinterpret_cast<typename C::U *>(sm + L::kOffU) + cl;
+            uint32_t us0 = 0, uph = 0;   // slot of block products, its use
+            if (warp < Role<T>::kChain) {
+                for (uint32_t un = 0; un < units * a.nstreams; ++un) {
+                    const uint32_t ge = un % L::kBufsE;
+                    warp_wait(bar_e(ge), (un / L::kBufsE) & 1, fail);
+                    fence_after();
+                    if (un >= (uint32_t)C::kUUnits) warp_wait(bar_uf(us0), uph ^ 1, fail);
+#pragma unroll
+                    for (uint32_t i = 0; i < (uint32_t)C::kUnit; ++i) {
+                        typename C::U u[4];
+                        reduce_tile(ge, 0, i, u);
+#pragma unroll
+                        for (int b = 0; b < 4; ++b) us[(us0 * kBlocksUnit + i * 4 + b) * kCands] = u[b];
+                    }
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(bar_u(us0));
+                        mbar_arrive(bar_ef(ge));
+                    }
+                    if (++us0 == (uint32_t)C::kUUnits) {
+                        us0 = 0;
+                        uph ^= 1;
+                    }
                 }
+            } else {
+                uint32_t un = 0, slot = 0, phase = 1;   // phase of the slot's release before its use
+                for (uint32_t s = 0; s < a.nstreams; ++s) {
+                    W r = start(s);
+                    for (uint32_t ul = 0; ul < units; ++ul, ++un) {
+                        warp_wait(bar_u(us0), uph, fail);
+                        if (un >= (uint32_t)C::kRUnits) warp_wait(bar_rf(slot), phase, fail);
+#pragma unroll
+                        for (uint32_t i = 0; i < (uint32_t)C::kUnit; ++i) {
+                            typename C::U u[4];
+#pragma unroll
+                            for (int b = 0; b < 4; ++b) u[b] = us[(us0 * kBlocksUnit + i * 4 + b) * kCands];
+                            W *rt = rs + (slot * C::kUnit + i) * L::kRTile;
+#pragma unroll
+                            for (int b = 0; b < 4; ++b) {
+                                rt[b * kCands] = r;
+                                r = C::prod(r, u[b], p, q);
+                            }
+                            rt[4 * kCands] = r;
+                        }
+                        __syncwarp();
+                        if (lane == 0) {
+                            mbar_arrive(bar_r(slot));
+                            mbar_arrive(bar_uf(us0));
+                        }
+                        if (++slot == (uint32_t)C::kRUnits) {
+                            slot = 0;
+                            phase ^= 1;
+                        }
+                        if (++us0 == (uint32_t)C::kUUnits) {
+                            us0 = 0;
+                            uph ^= 1;
+                        }
+                    }
+                    finish(s, r);
+                }
+            }
+        } else {
+            // Class 64: the groups take units in turn, reduce a unit's block
+            // products, which waits for no other group, then move the residue
+            // on from where the group before left it.  (In class 32 this took
+            // 1 to 3% longer than the two roles, here 6% less.)
+            static_assert(C::kChainGroups <= C::kRUnits, "a group's next slot is one turn on at most");
+            uint32_t ul = (warp - Role<T>::kChain) / 4, s = 0;   // unit of the stream, stream
+            uint32_t slot = ul, turn = 0;                        // the unit's slot of residues, its uses before
+            if (ul >= units) {   // (a stream of two units: the third group starts in the second)
+                ul -= units;
+                ++s;
+            }
+            // a buffer of sums is released by every group, when it has read its
+            // last unit there or has none
+            uint32_t seen = 0;   // buffers released by this group
+            auto pass = [&](uint32_t end) {
+                for (; seen < end; ++seen) {
+                    warp_wait(bar_e(seen % L::kBufsE), (seen / L::kBufsE) & 1, fail);
+                    if (lane == 0) mbar_arrive(bar_ef(seen % L::kBufsE));
+                }
+            };
+            for (uint32_t un = slot; un < units * a.nstreams; un += C::kChainGroups) {
+                const uint32_t g = s * nsupers_e + ul / kUnitsE, te = ul % kUnitsE, ge = g % L::kBufsE;
+                pass(g);
+                warp_wait(bar_e(ge), (g / L::kBufsE) & 1, fail);
+                fence_after();
+                typename C::U u[kBlocksUnit];
+#pragma unroll
+                for (uint32_t i = 0; i < (uint32_t)C::kUnit; ++i) reduce_tile(ge, te, i, u + 4 * i);
                 fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(bar_ef(ge));
-                if (++ge == (uint32_t)L::kBufsE) {
-                    ge = 0;
-                    eph ^= 1;
+                if (te + C::kChainGroups >= kUnitsE || ul + C::kChainGroups >= units) {
+                    if (lane == 0) mbar_arrive(bar_ef(ge));
+                    seen = g + 1;
                 }
-            }
-            if (++us0 == (uint32_t)C::kUUnits) {
-                us0 = 0;
-                uph ^= 1;
-            }
-            if (++ul == units) ul = 0;
-        }
-    } else if (warp < Role<T>::kTestMma) {
-        // ------------------------------------------------------------ chain
-        const W p = m.p;
-        const typename C::Q q = C::qv(m);
-        const typename C::U *us = reinterpret_cast<const typename C::U *>(sm + L::kOffU) + cl;
-        W *rs = reinterpret_cast<W *>(sm + L::kOffR) + cl;
-        constexpr int kBlocksUnit = C::kUnit * kBlocksTile;
-        const uint32_t units = tiles / C::kUnit;
-        uint32_t un = 0, slot = 0, phase = 1;   // phase of the slot's release before its use
-        uint32_t us0 = 0, uph = 0;
-        for (uint32_t s = 0; s < a.nstreams; ++s) {
-            const bool second = (s ? a.second[1] : a.second[0]) != 0;
-            const W *in = second ? c.s1 : c.s0;
-            if (split && sub) in = (second ? sp->s1 : sp->s0) + (size_t)(sub - 1) * sp->pitch;
-            W r = act ? in[ci] : (W)0;
-            for (uint32_t ul = 0; ul < units; ++ul, ++un) {
-                warp_wait(bar_u(us0), uph, fail);
-                if (un >= (uint32_t)C::kRUnits) warp_wait(bar_rf(slot), phase, fail);
+                if (turn) warp_wait(bar_rf(slot), (turn - 1) & 1, fail);
+                W r = 0;
+                if (un) {   // (at a stream's start too: the units stay in order)
+                    const uint32_t before = slot ? slot - 1 : C::kRUnits - 1;
+                    warp_wait(bar_r(before), slot ? turn & 1 : (turn - 1) & 1, fail);
+                    r = rs[(before * C::kUnit + C::kUnit - 1) * L::kRTile + 4 * kCands];
+                }
+                if (ul == 0) r = start(s);
+                W *ru = rs + slot * (C::kUnit * L::kRTile);
 #pragma unroll
                 for (uint32_t i = 0; i < (uint32_t)C::kUnit; ++i) {
-                    typename C::U u[4];
-#pragma unroll
-                    for (int b = 0; b < 4; ++b) u[b] = us[(us0 * kBlocksUnit + i * 4 + b) * kCands];
-                    W *rt = rs + (slot * C::kUnit + i) * L::kRTile;
 #pragma unroll
                     for (int b = 0; b < 4; ++b) {
-                        rt[b * kCands] = r;
-                        r = C::prod(r, u[b], p, q);
+                        ru[i * L::kRTile + b * kCands] = r;
+                        r = C::prod(r, u[4 * i + b], p, q);
                     }
-                    rt[4 * kCands] = r;
+                    ru[i * L::kRTile + 4 * kCands] = r;
                 }
                 __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(bar_r(slot));
-                    mbar_arrive(bar_uf(us0));
-                }
-                if (++slot == (uint32_t)C::kRUnits) {
-                    slot = 0;
-                    phase ^= 1;
-                }
-                if (++us0 == (uint32_t)C::kUUnits) {
-                    us0 = 0;
-                    uph ^= 1;
+                if (lane == 0) mbar_arrive(bar_r(slot));
+                if (ul + 1 == units) finish(s, r);
+                for (ul += C::kChainGroups; ul >= units && s < a.nstreams; ++s) ul -= units;
+                slot += C::kChainGroups;
+                if (slot >= (uint32_t)C::kRUnits) {
+                    slot -= C::kRUnits;
+                    ++turn;
                 }
             }
-            if (act && !*failed) {
-                if (last) (second ? c.s1 : c.s0)[ci] = T::canon(m, r);
-                if (split) atomicAdd(c.nnext + ci, hi - lo);
-                else c.nnext[ci] += hi - lo;
-            }
+            pass(nsupers_e * a.nstreams);
         }
     } else if (warp < Role<T>::kChainMma) {
         // ------------------------------------- the tests' copies and MMAs
