@@ -477,6 +477,19 @@ def step_recipe(cls32, lazy):
     return {"imad_wide": 7, "imad": 2}
 
 
+# What a test of the tensor-core walk leaves to the CUDA cores (walk_tc.cu):
+# one multiply-add, half a byte permute, one packed add-and-minimum per residue
+# sign, against the issue rate; its matrix products are 2 planes x 48 or 64
+# digits per test.
+TC_TEST_OPS = 2.5
+
+
+def walk_is_tc(nmin, nmax):
+    """Whether a walk of this length takes the tensor-core kernel at any number of candidates (class 32 needs
+    the longest, about 3,000 steps; kernels.cuh WalkTimes)."""
+    return nmax - nmin >= 4000
+
+
 def hit_order(f):
     """Hits sorted by (p, |n|, type, nc), for comparing two runs."""
     if len(f) == 0:
@@ -550,15 +563,16 @@ def mixed_roofline(jobs, outcomes, seconds, peaks, tc_s=0.0, setup_tc=True):
     return {"bound": "int (multiply pipe)", "achieved": achieved / 1e12, "peak": peaks["imad"] / 1e12,
             "unit": "Tops/s IMAD-equivalent (IMAD.WIDE, IMAD.HI weighted by measured rates)",
             "frac": achieved / peaks["imad"], "traffic": None,
-            "kernel": "batch_kernel and setup_tc_kernel (every class and kind of the batch, over its wall time)",
+            "kernel": "batch_kernel, walk_tc_many_kernel and setup_tc_kernel (every class and kind of the batch, over its "
+                      "wall time; walks counted as the multiplies of the per-step kernels)",
             "alg_ops": total, "seconds": seconds, "searches_crossing_a_class_boundary": crossing,
             "peak_source": "measured in this run (pfc_bench_int_peak, 32-bit IMAD chains)",
             "tensor_setup": tensor_line(2 * tc_macs, seconds)}
 
 
 def tensor_line(flops, seconds):
-    """The tensor-core setups' fold over the batch's wall time (the setups
-    overlap the iterations), against the measured dense bf16 peak
+    """The tensor cores' work over a time (the batch's setups: over its wall
+    time, which iterations overlap), against the measured dense bf16 peak
     (MEASURED_PEAKS.json, burst)."""
     if not flops or not seconds:
         return None
@@ -746,6 +760,23 @@ def run_ours(args, wl, world, rank, local, dist):
     peak = peaks["imad"]
     achieved = walk_steps * imad_eq / it_s
     alg_ops = walk_steps * imad_eq
+    cls = "Cls32" if cls32 else ("Cls64L" if lazy else "Cls64")
+    per_step = {"achieved": achieved / 1e12, "frac": achieved / peak, "multiplies_per_walk_step": recipe,
+                "imad_equivalent_per_walk_step": imad_eq}
+    tensor = None
+    if walk_is_tc(wl["nmin"], wl["nmax"]):
+        depth = 48 if wl["nmax"] - 1 <= 202000 else 64
+        flops = walk_steps * 4 * depth
+        tensor = tensor_line(flops, it_s)
+        bound, kernel = "issue slots (CUDA cores)", "walk_tc_kernel<%s, %d>" % (cls, depth)
+        unit = "Tops/s (instructions a test needs on the CUDA cores)"
+        peak, alg_ops = peaks["iadd_xor"], walk_steps * TC_TEST_OPS
+        achieved = alg_ops / it_s
+        peak_source = "measured in this run (pfc_bench_int_peak, add and xor chains: the issue rate)"
+    else:
+        bound, kernel = "int (multiply pipe)", "walk_kernel<%s>" % cls
+        unit = "Tops/s IMAD-equivalent (IMAD.WIDE, IMAD.HI weighted by measured rates)"
+        peak_source = "measured in this run (pfc_bench_int_peak, 32-bit IMAD chains)"
     # DRAM bytes of the walk launches of one step, from the committed ncu
     # capture of this workload (profiles/walk_kernel_traffic.json)
     traffic = None
@@ -816,22 +847,21 @@ def run_ours(args, wl, world, rank, local, dist):
                        "l2": "256 MB buffer overwritten before each step (candidate state < L2)",
                        "parallelism": "p-range shards, one per GPU" if world > 1 else "1 GPU",
                        "device": name, "sms": sms, "walk_variants": tuned},
-            "roofline": {"bound": "int (multiply pipe)", "achieved": achieved / 1e12, "peak": peak / 1e12,
-                         "unit": "Tops/s IMAD-equivalent (IMAD.WIDE, IMAD.HI weighted by measured rates)",
-                         "frac": achieved / peak, "traffic": traffic,
-                         "kernel": "walk_kernel<%s>" % ("Cls32" if cls32 else ("Cls64L" if lazy else "Cls64")),
+            "roofline": {"bound": bound, "achieved": achieved / 1e12, "peak": peak / 1e12, "unit": unit,
+                         "frac": achieved / peak, "traffic": traffic, "kernel": kernel, "tensor": tensor,
                          "walk_steps_per_step": int(walk_steps),
-                         "multiplies_per_walk_step": recipe,
-                         "imad_equivalent_per_walk_step": imad_eq,
                          "alg_ops_per_step": alg_ops,
                          "kernel_ms_per_step": it_s * 1e3,
-                         "peak_source": "measured in this run (pfc_bench_int_peak, 32-bit IMAD chains)",
+                         "peak_source": peak_source,
+                         # the multiplies of a walk that steps each residue through
+                         # each n, over the IMAD peak (the per-step kernels' roofline)
+                         "per_step_algorithm": per_step,
                          "int_peaks_tops": {k: v / 1e12 for k, v in peaks.items()},
                          # not a roofline fraction: the same steps priced at the
                          # reference's 20 IMAD-class operations per 64-bit Montgomery
                          # multiplication, over the peak (above 1 where this path's
                          # 32-bit steps do that work in less multiply-pipe time)
-                         "reference_cost_model_ratio": walk_steps / it_s * 20 / peak},
+                         "reference_cost_model_ratio": walk_steps / it_s * 20 / peaks["imad"]},
             "mulmods": {"walk_per_s": walk_steps * args.steps / (ms_max * 1e-3) * world,
                         "walk_per_pair": steps_per_cand / (wl["nmax"] - wl["nmin"]),
                         "setup_per_candidate": setup_mm},
