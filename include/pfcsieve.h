@@ -107,10 +107,9 @@ int pfc_ctx_set_graphs(pfc_ctx *ctx, int on);
  * every candidate in one chain.  Results are identical. */
 int pfc_ctx_set_split(pfc_ctx *ctx, int on);
 
-/* Tensor-core setup.  The setup of class-32 candidates and of class-64
- * candidates below 2^64/3 folds each table word against the candidate's
+/* Tensor-core setup.  The setup folds each table word against the candidate's
  * position residues; this exact integer contraction runs on the tensor cores
- * (tcgen05, fp16 byte planes with fp32 sums kept below 2^24, so exact), on
+ * (tcgen05, fp16 digit planes with fp32 sums kept below 2^24, so exact), on
  * 1792-bit words that are products of pairs of the program's 896-bit words,
  * and the CUDA cores do the Montgomery products, with the same result as the
  * integer-pipe setup.  No counterpart in the reference, whose setup

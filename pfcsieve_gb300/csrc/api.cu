@@ -845,6 +845,17 @@ static int enqueue_iter_range(pfc_job *j, uint32_t lo, uint32_t hi, bool split =
     ensure_words(j, hi - lo);
     const bool words = words_fit(j, top_mult(j, hi), hi - lo);
     const bool tc32 = words && walk_tc32_applies(j, hi - lo), tc64 = words && walk_tc64_applies(j, hi - lo);
+    const bool per_step = (j->use32 && !tc32) || (j->use64 && !tc64);
+    // Where only tensor-core walks run, and not split, the compositorial's
+    // table lists the composite n alone; else it holds 1 at prime n, which
+    // keeps both chains, and the sub-ranges of a split, at the same steps.
+    // (4.5% of the combined search's steps near n = 2e5, 7% of a compositorial
+    // one's near 1e6.)
+    uint32_t composites = 0;
+    if ((j->mode & PFC_COMPOSITORIAL) && !split && !per_step && (tc32 || tc64)) {
+        const std::vector<uint32_t> &q = *c->primes;   // (at least up to nmax)
+        composites = hi - lo - (uint32_t)(std::lower_bound(q.begin(), q.end(), hi) - std::lower_bound(q.begin(), q.end(), lo));
+    }
     auto walk = [&](const WalkArgs &w) {
         const int fused = w.mult2 != nullptr;
         const bool lazy = j->seg_hi <= kLazyWalkEnd;
@@ -852,9 +863,14 @@ static int enqueue_iter_range(pfc_job *j, uint32_t lo, uint32_t hi, bool split =
             const uint32_t top = top_mult(j, hi);
             WalkTcArgs t{};
             t.nstreams = fused ? 2 : 1;
-            t.lo = lo;
-            t.hi = hi;
-            t.base = w.base;
+            walk_tc_args(t, top, lo, hi, w.base);
+            if (composites && fused) {
+                t.lo1 = t.base1 = 0;
+                t.hi1 = composites;
+            } else if (composites) {
+                t.lo = t.base = 0;
+                t.hi = composites;
+            }
             // the factorial's multipliers are n itself (the fused walk's
             // table of them is for the per-step kernels)
             t.mult[0] = fused ? nullptr : w.mult;
@@ -862,9 +878,8 @@ static int enqueue_iter_range(pfc_job *j, uint32_t lo, uint32_t hi, bool split =
             t.type[0] = w.type;
             t.type[1] = w.type2;
             t.second[1] = 1;
-            for (uint32_t s = 0; s < t.nstreams; ++s) {
-                c->launches += launch_walk_words(t.mult[s], t.base, lo, hi, top, j->words[s].p, t, (int)s, c->st);
-            }
+            c->launches += launch_walk_words(t.mult[0], t.base, t.lo, t.hi, top, j->words[0].p, t, 0, c->st);
+            if (fused) c->launches += launch_walk_words(t.mult[1], t.base1, t.lo1, t.hi1, top, j->words[1].p, t, 1, c->st);
             if (tc32)
                 c->launches += launch_walk_tc32(j->c32.view(counts_ptr(j)), t, top, h, split ? &sp32 : nullptr,
                                                 &j->stats.p->tc_err, c->st);
@@ -899,11 +914,11 @@ static int enqueue_iter_range(pfc_job *j, uint32_t lo, uint32_t hi, bool split =
         // per-step fused walk, factorial (n; the plain factorial walk forms n
         // itself, shared by its two candidates, and gains nothing from a table)
         const size_t need = ((size_t)(hi - lo) + 15) & ~(size_t)15;
-        const bool comp = true, fact = (j->mode & PFC_FACTORIAL) && ((j->use32 && !tc32) || (j->use64 && !tc64));
-        if (comp && j->cmult.n < need) CK(j->cmult.alloc(c, std::max<size_t>(need, 4096)));
+        const bool fact = (j->mode & PFC_FACTORIAL) && per_step;
+        if (j->cmult.n < need) CK(j->cmult.alloc(c, std::max<size_t>(need, 4096)));
         if (fact && j->ramp.n < need) CK(j->ramp.alloc(c, std::max<size_t>(need, 4096)));
-        c->launches += launch_cmult(comp ? j->cmult.p : nullptr, fact ? j->ramp.p : nullptr, j->primebits.p,
-                                    j->nmin, lo, hi, c->st);
+        c->launches += composites ? launch_composites(j->cmult.p, j->primebits.p, j->nmin, lo, hi, c->st)
+                                  : launch_cmult(j->cmult.p, fact ? j->ramp.p : nullptr, j->primebits.p, j->nmin, lo, hi, c->st);
         w.base = lo;
     }
     if (j->mode == (PFC_FACTORIAL | PFC_COMPOSITORIAL)) {

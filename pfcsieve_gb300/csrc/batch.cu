@@ -1070,11 +1070,9 @@ static bool plan_tc_walk(pfc_batch *b, int l, int shape, const std::vector<Batch
             at += chains(j) * bytes;
             if (from >= w.hi) continue;
             WalkTcArgs a{};
-            walk_tc_args(a, top);
+            walk_tc_args(a, top, base + (uint32_t)(from - ns),
+                         base + (uint32_t)(std::min<uint64_t>(from + piece[i], w.hi) - ns), base);
             a.nstreams = chains(j);
-            a.lo = base + (uint32_t)(from - ns);
-            a.hi = base + (uint32_t)(std::min<uint64_t>(from + piece[i], w.hi) - ns);
-            a.base = base;
             const bool prim = j->mode == PFC_PRIMORIAL, comp = j->mode == PFC_COMPOSITORIAL;
             a.mult[0] = prim ? j->d_qlist.p : comp ? j->d_cmult.p : nullptr;
             a.mult[1] = j->d_cmult.p;

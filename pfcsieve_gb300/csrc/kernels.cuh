@@ -202,10 +202,15 @@ struct WalkTcArgs {
     int32_t type[2];           // factor type of a stream's hits
     uint32_t second[2];        // 1: the stream walks the residue s1
     uint32_t nstreams;
-    uint32_t lo, hi, base;
+    uint32_t lo, hi, base;           // steps of the first stream,
+    uint32_t lo1, hi1, base1;        // and of the second
+    uint32_t credit[2];              // steps that a stream adds to the candidates' count (a split walk: its own)
     uint32_t nb, shift11, shift22;   // set by walk_tc_args: steps per block, 2^11, 2^22
 };
-void walk_tc_args(WalkTcArgs &a, uint32_t top);
+// (both streams over [lo, hi), each step credited)
+void walk_tc_args(WalkTcArgs &a, uint32_t top, uint32_t lo, uint32_t hi, uint32_t base);
+// the composite n of [lo, hi) in order (prime flags as launch_cmult)
+int launch_composites(uint32_t *out, const uint32_t *primebits, uint32_t nmin, uint32_t lo, uint32_t hi, cudaStream_t st);
 uint32_t walk_tc_align(uint32_t top);   // sub-ranges of a split walk start at multiples of this from lo
 size_t walk_tc_words_bytes(uint32_t top, uint32_t steps);
 // (the table of steps [lo, hi) into `out`, for the walk's stream `stream`)

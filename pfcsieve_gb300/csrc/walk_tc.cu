@@ -56,6 +56,10 @@
 // reduction and tests run in units of tiles, handed over through shared memory,
 // so that a role waits once per unit and not once per tile.
 //
+// A launch walks one stream (a chain of each candidate) or the combined
+// search's two one after the other, each over its own list of multipliers; one
+// stream has kernels of its own, without the second's bookkeeping (2 to 3%).
+//
 // What bounds it: the CUDA cores' issue slots and their ALU pipe (byte permutes
 // and packed minima).  Cycles per 32 candidates and step on an SM's quarter,
 // per-step kernels to this one: class 32 (4.8e5 candidates) 17.7 to 12.5 (words
@@ -299,7 +303,7 @@ struct Lay {
     static constexpr uint32_t kOffBar = kOffPq + kCands * sizeof(typename C::Q);
     static constexpr uint32_t kBars = kFStages + kWStages + 2 * kBufs + 2 * C::kRUnits + 2 * kBufsE + 2 * C::kUUnits + kBufs + 1;
     static constexpr uint32_t kOffMisc = kOffBar + kBars * 8;   // failed, TMEM address, suspects, testers done, [batch] rounds replayed
-    static constexpr uint32_t kSmem = kOffMisc + 16 + kBatches * 4;
+    static constexpr uint32_t kSmem = kOffMisc + 16 + kBatches * 4 + 8;   // and the steps [lo, hi)
     static_assert(kOffF % 128 == 0 && kOffW % 128 == 0 && kOffR % 16 == 0 && kOffBar % 8 == 0, "walk_tc alignment");
     static_assert(kSmem <= 227 * 1024, "walk_tc shared memory");
 };
@@ -463,8 +467,9 @@ __global__ void __launch_bounds__(128) walk_words_many_kernel(const WalkWordsWin
     walk_words<K>(win, (blockIdx.x - win.first_cta) * blockDim.x + threadIdx.x);
 }
 
-// one CTA: candidates 128 cta .. of c, sub-range `sub` of a split walk (sp, or null)
-template <class T, int K>
+// one CTA: candidates 128 cta .. of c, sub-range `sub` of a split walk (sp, or
+// null); NS 1 for walks of one stream, 2 for one or two
+template <class T, int K, int NS>
 __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const WalkTcArgs &a, const HitBuf &h,
                                         const SplitArgs<typename T::W> *sp, uint32_t *err, uint32_t cta, uint32_t sub) {
     using C = ChainClass<T>;
@@ -473,11 +478,12 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
     using W = typename T::W;
     extern __shared__ __align__(1024) unsigned char sm[];
     const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+    const uint32_t nstreams = NS == 1 ? 1u : a.nstreams;
     const uint32_t cnt = min(*c.count, c.cap);
     const uint32_t c0 = cta * kCands;
     if (c0 >= cnt) return;   // whole CTA idle
 
-    uint32_t lo = a.lo, hi = a.hi;
+    uint32_t lo = a.lo, hi = a.hi;   // steps of the first stream (of both in a split walk)
     const bool split = sp && sp->n > 1, last = !split || sub + 1 >= sp->n;
 #pragma unroll
     for (int k = 0; k < kMaxSplit; ++k)
@@ -486,14 +492,16 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
             hi = sp->start[k + 1];
         }
     const uint32_t super0 = (lo - a.lo) / (kBlocksSuper * a.nb);   // sub-ranges start at supertiles
-    const uint32_t supers = ((hi - lo + a.nb - 1) / a.nb + kBlocksSuper - 1) / kBlocksSuper;   // of a stream
-    const uint32_t tiles = supers * kTilesSuper, ntiles = tiles * a.nstreams;
-
-    const uint32_t nsupers_e = (supers + C::kBlocksE / kBlocksSuper - 1) / (C::kBlocksE / kBlocksSuper);
+    constexpr uint32_t kPer = C::kBlocksE / kBlocksSuper;   // supertiles per buffer of residue sums
+    const uint32_t per = kBlocksSuper * a.nb;
+    const uint32_t supers = (hi - lo + per - 1) / per;   // supertiles of the first stream, of the second
+    const uint32_t supers1 = nstreams < 2 ? 0u : split ? supers : (a.hi1 - a.lo1 + per - 1) / per;
+    const uint32_t tiles = supers * kTilesSuper, ntiles = tiles + supers1 * kTilesSuper;   // of the first stream, of both
+    const uint32_t nsupers_e = (supers + kPer - 1) / kPer, nge = nsupers_e + (supers1 + kPer - 1) / kPer;
     // the test's window around +-A in units of 2^-16: the f_b are off by up to
     // 0.504 units of 2^-24 each, A by 0.045 of 2^-16
     uint32_t digits = *a.digits[0];
-    if (a.nstreams > 1) digits = max(digits, *a.digits[1]);
+    if (nstreams > 1) digits = max(digits, *a.digits[1]);
     const uint32_t half = (uint32_t)(digits * (0.504f / 256.0f) + 0.045f) + 1u;
     constexpr uint32_t kBlocksUnit = C::kUnit * kBlocksTile, kUnitsE = C::kBlocksE / kBlocksUnit;   // units per buffer of residue sums
     const uint32_t bar = smem_u32(sm + L::kOffBar);
@@ -514,6 +522,7 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
     volatile uint32_t *failed = misc;
     const uint32_t fail = smem_u32(misc);
     uint32_t *taddr_slot = misc + 1, *suspects = misc + 2, *testers_done = misc + 3, *replayed = misc + 4;
+    const volatile uint32_t *range = misc + 4 + kBatches;   // lo, hi: read where they are rarely needed
     W *cand_p = reinterpret_cast<W *>(sm + L::kOffP);
     auto *cand_q = reinterpret_cast<typename C::Q *>(sm + L::kOffPq);
 
@@ -545,6 +554,8 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
         *failed = 0;
         *suspects = *testers_done = 0;
         for (uint32_t i = 0; i < kBatches; ++i) replayed[i] = 0;
+        misc[4 + kBatches] = lo;
+        misc[5 + kBatches] = hi;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     for (uint32_t i = tid; i < kBatches * 32; i += Role<T>::kThreads) reinterpret_cast<uint32_t *>(sm + L::kOffQs)[i] = 0;
@@ -560,22 +571,22 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
     // buffer, supertile(s) g of block words; the first ones start here (none
     // after a wait that gave up: a copy may then still be pending on its barrier)
     const unsigned char *tab0 = a.words[0] + (size_t)super0 * S::kSuper;
-    const unsigned char *tab1 = a.nstreams > 1 ? a.words[1] + (size_t)super0 * S::kSuper : nullptr;
-    constexpr uint32_t kPer = C::kBlocksE / kBlocksSuper;   // supertiles per buffer of residue sums
-    const uint32_t nge = nsupers_e * a.nstreams;
+    const unsigned char *tab1 = nstreams > 1 ? a.words[1] + (size_t)super0 * S::kSuper : nullptr;
     auto load_f = [&](uint32_t t, uint32_t b, uint32_t stage) {
-        const uint32_t tl = t >= tiles ? t - tiles : t;
+        const bool other = NS > 1 && t >= tiles;   // the second stream's
+        const uint32_t tl = other ? t - tiles : t;
         if (elect() && !*failed)
             copy_in(smem_u32(sm + L::kOffF) + (2 * b + stage) * S::kFTile,
-                    (t >= tiles ? tab1 : tab0) + (size_t)(tl / kTilesSuper) * S::kSuper + S::kWTile +
+                    (other ? tab1 : tab0) + (size_t)(tl / kTilesSuper) * S::kSuper + S::kWTile +
                         (tl % kTilesSuper) * S::kFTile,
                     S::kFTile, bar_f(2 * b + stage));
         __syncwarp();
     };
     auto load_w = [&](uint32_t g) {
-        const uint32_t gl = (g >= nsupers_e ? g - nsupers_e : g) * kPer, n = min(kPer, supers - gl);
+        const bool other = NS > 1 && g >= nsupers_e;
+        const uint32_t gl = (other ? g - nsupers_e : g) * kPer, n = min(kPer, (other ? supers1 : supers) - gl);
         const uint32_t dst = smem_u32(sm + L::kOffW) + (g % L::kWStages) * L::kWStage, bw = bar_w(g % L::kWStages);
-        const unsigned char *src = (g >= nsupers_e ? tab1 : tab0) + (size_t)gl * S::kSuper;
+        const unsigned char *src = (other ? tab1 : tab0) + (size_t)gl * S::kSuper;
         if (elect() && !*failed) {
             expect(bw, n * S::kWTile);
             for (uint32_t i = 0; i < n; ++i)
@@ -775,7 +786,7 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
                                     *failed = 1;
                                     break;
                                 }
-                            const uint32_t s = t >= tiles ? 1u : 0u;
+                            const uint32_t s = NS > 1 && t >= tiles ? 1u : 0u;
                             qr[e] = rt[b * kCands];
                             qk[e] = (s << 31) | (((t - (s ? tiles : 0u)) * kBlocksTile + b0 + b) << 7) | cl;
                             __threadfence_block();
@@ -800,7 +811,7 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
         const typename C::Q q = C::qv(m);
         const uint2 shifts = make_uint2(a.shift11, a.shift22);
         W *rs = reinterpret_cast<W *>(sm + L::kOffR) + cl;
-        const uint32_t units = tiles / C::kUnit;
+        const uint32_t units = tiles / C::kUnit, all_units = ntiles / C::kUnit;   // of the first stream, of both
         // the block products of tile i of unit te of buffer ge
         auto reduce_tile = [&](uint32_t ge, uint32_t te, uint32_t i, typename C::U *u) {
             uint32_t v[C::kPlanes][4];
@@ -826,7 +837,7 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
         auto finish = [&](uint32_t s, W r) {
             if (!act || *failed) return;
             if (last) (second(s) ? c.s1 : c.s0)[ci] = T::canon(m, r);
-            atomicAdd(c.nnext + ci, hi - lo);   // (the streams' ends may fall to two groups)
+            atomicAdd(c.nnext + ci, split ? range[1] - range[0] : s ? a.credit[1] : a.credit[0]);   // (the streams' ends may fall to two groups)
         };
         if constexpr (C::kReduceGroups != 0) {
             // Class 32: one group reduces, one moves the residues.  A buffer of
@@ -835,7 +846,7 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
             typename C::U *us = reinterpret_cast<typename C::U *>(sm + L::kOffU) + cl;
             uint32_t us0 = 0, uph = 0;   // slot of block products, its use
             if (warp < Role<T>::kChain) {
-                for (uint32_t un = 0; un < units * a.nstreams; ++un) {
+                for (uint32_t un = 0; un < all_units; ++un) {
                     const uint32_t ge = un % L::kBufsE;
                     warp_wait(bar_e(ge), (un / L::kBufsE) & 1, fail);
                     fence_after();
@@ -860,9 +871,10 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
                 }
             } else {
                 uint32_t un = 0, slot = 0, phase = 1;   // phase of the slot's release before its use
-                for (uint32_t s = 0; s < a.nstreams; ++s) {
+                for (uint32_t s = 0; s < nstreams; ++s) {
                     W r = start(s);
-                    for (uint32_t ul = 0; ul < units; ++ul, ++un) {
+                    const uint32_t end = s ? all_units : units;
+                    for (; un < end; ++un) {
                         warp_wait(bar_u(us0), uph, fail);
                         if (un >= (uint32_t)C::kRUnits) warp_wait(bar_rf(slot), phase, fail);
 #pragma unroll
@@ -903,8 +915,10 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
             static_assert(C::kChainGroups <= C::kRUnits, "a group's next slot is one turn on at most");
             uint32_t ul = (warp - Role<T>::kChain) / 4, s = 0;   // unit of the stream, stream
             uint32_t slot = ul, turn = 0;                        // the unit's slot of residues, its uses before
-            if (ul >= units) {   // (a stream of two units: the third group starts in the second)
+            uint32_t left = units;                               // units of the stream
+            if (NS > 1 && ul >= units) {   // (a stream of two units: the third group starts in the second)
                 ul -= units;
+                left = all_units - units;
                 ++s;
             }
             // a buffer of sums is released by every group, when it has read its
@@ -916,7 +930,7 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
                     if (lane == 0) mbar_arrive(bar_ef(seen % L::kBufsE));
                 }
             };
-            for (uint32_t un = slot; un < units * a.nstreams; un += C::kChainGroups) {
+            for (uint32_t un = slot; un < all_units; un += C::kChainGroups) {
                 const uint32_t g = s * nsupers_e + ul / kUnitsE, te = ul % kUnitsE, ge = g % L::kBufsE;
                 pass(g);
                 warp_wait(bar_e(ge), (g / L::kBufsE) & 1, fail);
@@ -926,7 +940,7 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
                 for (uint32_t i = 0; i < (uint32_t)C::kUnit; ++i) reduce_tile(ge, te, i, u + 4 * i);
                 fence_before();
                 __syncwarp();
-                if (te + C::kChainGroups >= kUnitsE || ul + C::kChainGroups >= units) {
+                if (te + C::kChainGroups >= kUnitsE || ul + C::kChainGroups >= left) {
                     if (lane == 0) mbar_arrive(bar_ef(ge));
                     seen = g + 1;
                 }
@@ -950,15 +964,20 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_r(slot));
-                if (ul + 1 == units) finish(s, r);
-                for (ul += C::kChainGroups; ul >= units && s < a.nstreams; ++s) ul -= units;
+                if (ul + 1 == left) finish(s, r);
+                ul += C::kChainGroups;
+                while (NS > 1 && ul >= left && s < 2) {
+                    ul -= left;
+                    left = all_units - units;
+                    ++s;
+                }
                 slot += C::kChainGroups;
                 if (slot >= (uint32_t)C::kRUnits) {
                     slot -= C::kRUnits;
                     ++turn;
                 }
             }
-            pass(nsupers_e * a.nstreams);
+            pass(nge);
         }
     } else if (warp < Role<T>::kChainMma) {
         // ------------------------------------- the tests' copies and MMAs
@@ -1057,13 +1076,15 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
             const uint32_t key = mine ? qk[e] : 0u;
             const W r = mine ? qr[e] : (W)0;
             const uint32_t cand = key & (kCands - 1);
-            const uint32_t k = lo + ((key & 0x7FFFFFFFu) >> 7) * a.nb;
-            const uint32_t *mult = (key >> 31) ? a.mult[1] : a.mult[0];
+            const bool other = NS > 1 && key >> 31;   // the second stream
+            const uint32_t k = (other && !split ? a.lo1 : range[0]) + ((key & 0x7FFFFFFFu) >> 7) * a.nb;
+            const uint32_t end = other && !split ? a.hi1 : range[1];
+            const uint32_t *mult = other ? a.mult[1] : a.mult[0];
             const bool replay = mine && !*failed;
             __syncwarp();
             if (lane == 0) reinterpret_cast<volatile uint32_t *>(replayed)[b % kBatches] = round + 1;   // entries taken
-            replay_suspect<T>(replay, cand_p[cand], cand_q[cand], r, k, k < hi ? min(a.nb, hi - k) : 0u,
-                              mult ? mult + (k - a.base) : nullptr, (key >> 31) ? a.type[1] : a.type[0], h);
+            replay_suspect<T>(replay, cand_p[cand], cand_q[cand], r, k, k < end ? min(a.nb, end - k) : 0u,
+                              mult ? mult + (k - (other ? a.base1 : a.base)) : nullptr, other ? a.type[1] : a.type[0], h);
             if (n < 32) break;
         }
     }
@@ -1079,10 +1100,10 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tbase) : "memory");
 }
 
-template <class T, int K>
+template <class T, int K, int NS>
 __global__ void __launch_bounds__(Role<T>::kThreads, 1)
     walk_tc_kernel(ClassBuf<typename T::W> c, WalkTcArgs a, HitBuf h, SplitArgs<typename T::W> sp, uint32_t *err) {
-    walk_tc<T, K>(c, a, h, &sp, err, blockIdx.x, blockIdx.y);
+    walk_tc<T, K, NS>(c, a, h, &sp, err, blockIdx.x, blockIdx.y);
 }
 
 // The walks of many searches in one launch (a batch's iteration): each CTA
@@ -1094,7 +1115,7 @@ __global__ void __launch_bounds__(Role<T>::kThreads, 1)
     if (threadIdx.x == 0) w = wins[window_of(wins, n, blockIdx.x)];
     __syncthreads();
     h.tagval = w.tag;
-    walk_tc<T, K>(w.c, w.a, h, nullptr, w.err, blockIdx.x - w.first_cta, 0);
+    walk_tc<T, K, 2>(w.c, w.a, h, nullptr, w.err, blockIdx.x - w.first_cta, 0);
 }
 
 // ------------------------------------------------------------------ launches
@@ -1110,6 +1131,40 @@ size_t walk_tc_words_bytes(uint32_t top, uint32_t steps) {
     const uint32_t per = walk_tc_align(top);
     const size_t nsuper = ((size_t)steps + per - 1) / per;
     return kTableHead + nsuper * (word_depth(top) == 48 ? WordShape<48>::kSuper : WordShape<64>::kSuper);
+}
+
+// One CTA: each thread counts the composites in its share of the flags' words,
+// and after a scan over the threads writes them.
+static __global__ void __launch_bounds__(1024) composites_kernel(uint32_t *out, const uint32_t *primebits, uint32_t nmin,
+                                                                 uint32_t lo, uint32_t hi) {
+    __shared__ uint32_t part[32];
+    const uint32_t o0 = lo - nmin, o1 = hi - nmin, w0 = o0 / 32, w1 = (o1 + 31) / 32, lane = threadIdx.x % 32;
+    const uint32_t per = (w1 - w0 + 1023) / 1024;
+    const uint32_t a = min(w0 + threadIdx.x * per, w1), b = min(a + per, w1);
+    auto word = [&](uint32_t w) {   // bit k: offset 32 w + k is in the range and composite
+        uint32_t v = ~__ldg(primebits + w);
+        if (32 * w < o0) v &= ~0u << (o0 - 32 * w);
+        if (o1 - 32 * w < 32) v &= ~(~0u << (o1 - 32 * w));
+        return v;
+    };
+    uint32_t count = 0;
+    for (uint32_t w = a; w < b; ++w) count += __popc(word(w));
+    uint32_t sum = count;   // inclusive over the warp
+    for (uint32_t d = 1; d < 32; d <<= 1) {
+        const uint32_t v = __shfl_up_sync(kFull, sum, d);
+        if (lane >= d) sum += v;
+    }
+    if (lane == 31) part[threadIdx.x / 32] = sum;
+    __syncthreads();
+    uint32_t at = sum - count;
+    for (uint32_t k = 0; k < threadIdx.x / 32; ++k) at += part[k];
+    for (uint32_t w = a; w < b; ++w)
+        for (uint32_t v = word(w); v; v &= v - 1) out[at++] = nmin + 32 * w + __ffs(v) - 1;
+}
+int launch_composites(uint32_t *out, const uint32_t *primebits, uint32_t nmin, uint32_t lo, uint32_t hi, cudaStream_t st) {
+    if (hi <= lo) return 0;
+    composites_kernel<<<1, 1024, 0, st>>>(out, primebits, nmin, lo, hi);
+    return 1;
 }
 
 static uint32_t supers_of(uint32_t top, uint32_t steps) {
@@ -1163,20 +1218,24 @@ static bool configure(Kernel kernel, uint32_t smem, bool (&configured)[64]) {
     return configured[dev] = true;
 }
 
-void walk_tc_args(WalkTcArgs &a, uint32_t top) {
+void walk_tc_args(WalkTcArgs &a, uint32_t top, uint32_t lo, uint32_t hi, uint32_t base) {
+    a.lo = a.lo1 = lo;
+    a.hi = a.hi1 = hi;
+    a.base = a.base1 = base;
+    a.credit[0] = a.credit[1] = hi - lo;
     a.nb = walk_tc_block(top);
     a.shift11 = 1u << 11;
     a.shift22 = 1u << 22;
 }
 
-template <class T, int K>
+template <class T, int K, int NS>
 static int launch_tc(const ClassBuf<typename T::W> &c, const WalkTcArgs &a, const HitBuf &h,
                      const SplitArgs<typename T::W> &sp, uint32_t *err, cudaStream_t st) {
     using L = Lay<T, K>;
     static bool configured[64] = {false};
-    if (!configure(walk_tc_kernel<T, K>, L::kSmem, configured)) return 0;
+    if (!configure(walk_tc_kernel<T, K, NS>, L::kSmem, configured)) return 0;
     const dim3 grid((c.cap + kCands - 1) / kCands, sp.n);
-    walk_tc_kernel<T, K><<<grid, Role<T>::kThreads, L::kSmem, st>>>(c, a, h, sp, err);
+    walk_tc_kernel<T, K, NS><<<grid, Role<T>::kThreads, L::kSmem, st>>>(c, a, h, sp, err);
     return 1;
 }
 
@@ -1202,14 +1261,15 @@ int launch_walk_tc64_many(const WalkTcWin<uint64_t> *wins, uint32_t n, uint32_t 
 }
 
 template <class T>
-static int launch_tc(const ClassBuf<typename T::W> &c, WalkTcArgs a, uint32_t top, const HitBuf &h,
+static int launch_tc(const ClassBuf<typename T::W> &c, const WalkTcArgs &a, uint32_t top, const HitBuf &h,
                      const SplitArgs<typename T::W> *sp, uint32_t *err, cudaStream_t st) {
     if (!c.cap || a.hi <= a.lo) return 0;
     SplitArgs<typename T::W> one{};
     one.n = 1;
-    walk_tc_args(a, top);
-    if (word_depth(top) == 48) return launch_tc<T, 48>(c, a, h, sp ? *sp : one, err, st);
-    return launch_tc<T, 64>(c, a, h, sp ? *sp : one, err, st);
+    const SplitArgs<typename T::W> &parts = sp ? *sp : one;
+    if (word_depth(top) == 48)
+        return a.nstreams > 1 ? launch_tc<T, 48, 2>(c, a, h, parts, err, st) : launch_tc<T, 48, 1>(c, a, h, parts, err, st);
+    return a.nstreams > 1 ? launch_tc<T, 64, 2>(c, a, h, parts, err, st) : launch_tc<T, 64, 1>(c, a, h, parts, err, st);
 }
 
 int launch_walk_tc32(const ClassBuf<uint32_t> &c, const WalkTcArgs &a, uint32_t top, const HitBuf &h,

@@ -60,6 +60,7 @@ def test_lengths_and_word_shapes(nmin, length):
     (5, 10**9, 40, (), False), (2, 2**40, 2700, (), False), (5, 10**9, 2800, (), True), (1, 2**40, 60000, (), True),
     (5, 10**8, 150000, (517, 1541, 9000, 20001), False), (2, 2**50, 150000, (517, 1541, 9000, 20001), False),
     (5, 2**64 - 60000, 59999, (517, 1541, 9000, 20001), False), (2, 2**64 // 3 - 30000, 60000, (), True),
+    (4, 2**50, 20000, (503, 504, 1009, 1010, 1041), False), (5, 10**9, 20000, (503, 504, 1009, 1010, 1041), False),
     (4, 2**31 - 70000, 150000, (), True), (5, 2**31 - 70000, 150000, (), True),
 ])
 def test_candidate_counts_and_ranges(mode, p, span, cuts, split):
