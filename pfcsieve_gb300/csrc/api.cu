@@ -45,6 +45,7 @@ struct pfc_job {
     TcProg tcp[2];
     uint64_t tc_words = 0;        // 896-bit words of the search's programs (both)
     bool top_tc = false;          // segments from 2^64/3 on set up on the tensor cores
+    bool no_tiles = false;        // there was no room for the tensor-core setup's tiles
     bool narrow = false;          // a64 and b64 are there (ensure_narrow)
     DArr<uint8_t> tct;
     DArr<uint32_t> tc_src, tc_groups;
@@ -57,6 +58,7 @@ struct pfc_job {
     DArr<uint32_t> cmult;       // compositorial multipliers of the current chunk
     DArr<uint32_t> ramp;        // the combined search's factorial multipliers (n) of the chunk
     DArr<uint8_t> words[2];     // the tensor-core walk's tables of the current chunk, per stream
+    bool no_words = false;      // there was no room for them: the job's walks take the per-step kernels
     std::vector<uint32_t> h_qlist;
 
     DevClass<uint32_t> c32;
@@ -651,11 +653,11 @@ static int tc_prepare(pfc_job *j) {
 }
 
 static bool tc_setup_applies(const pfc_job *j) {
-    if (!j->use64 || !j->ctx->setup_tc) return false;
+    if (!j->use64 || !j->ctx->setup_tc || j->no_tiles) return false;
     return j->seg_hi <= kLazyEnd ? j->tc_words >= kTcMinWords64 : j->top_tc;
 }
 static bool tc_setup32_applies(const pfc_job *j) {
-    return j->use32 && j->ctx->setup_tc && j->tc_words >= kTcMinWords32;
+    return j->use32 && j->ctx->setup_tc && !j->no_tiles && j->tc_words >= kTcMinWords32;
 }
 
 // The programs in 64-bit words of a search that reaches 2^64/3, where its
@@ -676,10 +678,32 @@ static bool narrow_setup_applies(const pfc_job *j) {
     return j->use64 && j->seg_hi > kLazyEnd && !tc_setup_applies(j);
 }
 
+// What the segment's setup needs on the device (not during a capture, which
+// finds it there): the tensor cores' tiles, or, where the budget has no room
+// for them, the integer pipe's words.
+static int setup_prepare(pfc_job *j) {
+    if (tc_setup_applies(j) || tc_setup32_applies(j)) {
+        const int rc = tc_prepare(j);
+        if (rc && rc != PFC_ERR_NOMEM) return rc;
+        if (rc) {
+            cudaGetLastError();
+            j->tct.release(j->ctx);
+            j->tc_src.release(j->ctx);
+            j->tc_groups.release(j->ctx);
+            if (j->pmin >= kLazyEnd) {   // (the 896-bit words were for the tiles alone)
+                j->aw.release(j->ctx);
+                j->bw.release(j->ctx);
+            }
+            j->no_tiles = true;
+        }
+    }
+    return narrow_setup_applies(j) ? ensure_narrow(j) : PFC_OK;
+}
+
 static int enqueue_setup(pfc_job *j) {
     pfc_ctx *c = j->ctx;
-    if (narrow_setup_applies(j)) {
-        const int rc = ensure_narrow(j);
+    {
+        const int rc = setup_prepare(j);
         if (rc) return rc;
     }
     CK(cudaMemsetAsync(&j->stats.p->tc_err, 0, sizeof(uint32_t), c->st));   // of this segment's tensor-core kernels
@@ -700,8 +724,6 @@ static int enqueue_setup(pfc_job *j) {
     sw.nnext0 = 0;
     if (j->use32) {
         if (tc_setup32_applies(j)) {
-            const int rc = tc_prepare(j);
-            if (rc) return rc;
             const TcTiles ta{j->tct.p, j->tc_ntiles[0]},
                 tb{j->tct.p + (size_t)j->tc_ntiles[0] * tc_tile_bytes(), j->tc_ntiles[1]};
             SetupArgs<WideWord> stc = s32;
@@ -714,8 +736,6 @@ static int enqueue_setup(pfc_job *j) {
     }
     if (j->use64) {
         if (tc_setup_applies(j)) {
-            const int rc = tc_prepare(j);
-            if (rc) return rc;
             const TcTiles ta{j->tct.p, j->tc_ntiles[0]},
                 tb{j->tct.p + (size_t)j->tc_ntiles[0] * tc_tile_bytes(), j->tc_ntiles[1]};
             SetupArgs<WideWord> stc = sw;
@@ -795,12 +815,13 @@ static uint32_t top_mult(const pfc_job *j, uint32_t hi) {
 // capture).  Where the budget has no room left the walk takes the per-step
 // kernels, which need none.
 static void ensure_words(pfc_job *j, uint32_t steps) {
-    if (iter_end(j) == iter_begin(j) || !(walk_tc32_applies(j, steps) || walk_tc64_applies(j, steps))) return;
+    if (j->no_words || iter_end(j) == iter_begin(j) || !(walk_tc32_applies(j, steps) || walk_tc64_applies(j, steps))) return;
     const size_t need = walk_tc_words_bytes(top_mult(j, iter_end(j)), steps);
     for (int k = 0; k < (j->mode == (PFC_FACTORIAL | PFC_COMPOSITORIAL) ? 2 : 1); ++k)
         if (j->words[k].n < need && j->words[k].alloc(j->ctx, need) != cudaSuccess) {
             cudaGetLastError();
             for (auto &w : j->words) w.release(j->ctx);
+            j->no_words = true;   // (not tried again: the next call may be a capture)
             return;
         }
 }
@@ -1263,12 +1284,8 @@ static int segment_body_graph(pfc_job *j) {
         if ((j->mode & PFC_COMPOSITORIAL) && j->cmult.n < need) CK(j->cmult.alloc(c, std::max<size_t>(need, 4096)));
         if ((j->mode & PFC_FACTORIAL) && j->ramp.n < need) CK(j->ramp.alloc(c, std::max<size_t>(need, 4096)));
     }
-    if (tc_setup_applies(j) || tc_setup32_applies(j)) {
-        const int rc = tc_prepare(j);
-        if (rc) return rc;
-    }
-    if (narrow_setup_applies(j)) {
-        const int rc = ensure_narrow(j);
+    {
+        const int rc = setup_prepare(j);
         if (rc) return rc;
     }
     {
