@@ -411,6 +411,7 @@ struct BatchJob {
     // first program, tc_pw the paired words of each)
     std::vector<uint32_t> tcsrc, tcgroups;
     bool tc_top = false;      // class 64 reaches 2^64/3 and sets up on the tensor cores
+    bool no_tc = false;       // the memory budget has no room for the tiles
     uint32_t tc_second = 0;   // first word of the second program
     uint32_t tc_ng[2] = {0, 0}, tc_fsq[2] = {0, 0}, tc_nw[2] = {0, 0}, tc_pw[2] = {0, 0}, tc_ntiles[2] = {0, 0};
     uint64_t tc_corr[2] = {0, 0};
@@ -766,7 +767,7 @@ int upload_job(pfc_batch *b, BatchJob *j) {
     if (e == cudaSuccess) e = j->d_words64.upload(c, j->words64);
     if (e == cudaSuccess) e = j->d_wordsw.upload(c, j->wordsw);
     const uint64_t words = (uint64_t)j->tc_nw[0] + j->tc_nw[1];
-    const bool tc = (j->tc && c->setup_tc &&
+    const bool tc = (j->tc && c->setup_tc && !j->no_tc &&
                      ((j->use64 && words >= kTcMinWords64) || (j->use32 && words >= kTcMinWords32))) ||
                     j->tc_top;
     const size_t tb = tc_tile_bytes(), nt = (size_t)j->tc_ntiles[0] + j->tc_ntiles[1];
@@ -824,6 +825,19 @@ int tc_launch(pfc_batch *b, BatchJob *j, int cls, cudaStream_t st, uint32_t bloc
                : launch_setup32_tc(j->c32.view(bs->counts), j->tc_args, j->tc_ta, j->tc_tb, &bs->flags, st, block0, n);
 }
 
+// a search's host tables
+void free_tables(BatchJob *j) {
+    free_vec(j->tcgroups);
+    free_vec(j->tcsrc);
+    free_vec(j->words32);
+    free_vec(j->words64);
+    free_vec(j->wordsw);
+    free_vec(j->segs32);
+    free_vec(j->segs64);
+    free_vec(j->cmult);
+    free_vec(j->qlist);
+}
+
 // Move prepared searches onto the device while slots and the memory budget
 // allow; on return their candidates exist and their blocks are laid out.
 int admit_prepared(pfc_batch *b) {
@@ -838,9 +852,15 @@ int admit_prepared(pfc_batch *b) {
             continue;
         }
         j->slot = b->free_slots.back();
-        const int rc = upload_job(b, j);
-        if (rc == PFC_ERR_NOMEM && !(b->running.empty() && b->ready.empty() && fresh.empty()))
-            break;  // waits for running searches to free memory
+        int rc = upload_job(b, j);
+        const bool alone = b->running.empty() && b->ready.empty() && fresh.empty();
+        if (rc == PFC_ERR_NOMEM && !alone) break;  // waits for running searches to free memory
+        if (rc == PFC_ERR_NOMEM && j->tc && !j->no_tc) {   // once more without the tensor-core setup's tiles
+            free_tables(j);
+            j->no_tc = true;
+            prepare_job(j, b->prime_cache, false);
+            rc = j->prep_rc != PFC_OK ? j->prep_rc : upload_job(b, j);
+        }
         b->queued.pop_front();
         if (rc != PFC_OK) {
             release_device(b, j);
@@ -952,15 +972,7 @@ int admit_prepared(pfc_batch *b) {
         CK(cudaGetLastError());
     }
     for (BatchJob *j : fresh) {
-        free_vec(j->tcgroups);
-        free_vec(j->tcsrc);
-        free_vec(j->words32);  // on the device now
-        free_vec(j->words64);
-        free_vec(j->wordsw);
-        free_vec(j->segs32);
-        free_vec(j->segs64);
-        free_vec(j->cmult);
-        free_vec(j->qlist);
+        free_tables(j);   // on the device now
         j->state = kReady;
         b->ready.push_back(j);
     }
