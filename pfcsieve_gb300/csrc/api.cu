@@ -78,8 +78,8 @@ struct pfc_job {
     // split walk of the current segment (kernels.cuh SplitArgs): sub-ranges,
     // their boundaries, the setup programs of the starts (boundaries 1..n-1;
     // 896-bit words for class 32 and the lazy class 64, 64-bit words above
-    // 2^64/3) and the start residues per class ((n-1) blocks of s0, then
-    // (n-1) of s1, one class capacity each)
+    // 2^64/3) and the start residues per class (n blocks of s0, then n of s1,
+    // one class capacity each)
     uint32_t split_n = 1;
     uint32_t split_start[kMaxSplit + 1] = {0};
     bool split_wide = false, split_narrow = false;
@@ -858,10 +858,10 @@ static int enqueue_iter_range(pfc_job *j, uint32_t lo, uint32_t hi, bool split =
         for (uint32_t k = 0; k <= j->split_n; ++k) sp32.start[k] = sp64.start[k] = j->split_start[k];
         sp32.pitch = j->c32.cap;
         sp32.s0 = j->split32.p;
-        sp32.s1 = j->split32.p ? j->split32.p + (size_t)(j->split_n - 1) * j->c32.cap : nullptr;
+        sp32.s1 = j->split32.p ? j->split32.p + (size_t)j->split_n * j->c32.cap : nullptr;
         sp64.pitch = j->c64.cap;
         sp64.s0 = j->split64.p;
-        sp64.s1 = j->split64.p ? j->split64.p + (size_t)(j->split_n - 1) * j->c64.cap : nullptr;
+        sp64.s1 = j->split64.p ? j->split64.p + (size_t)j->split_n * j->c64.cap : nullptr;
     }
     ensure_words(j, hi - lo);
     const bool words = words_fit(j, top_mult(j, hi), hi - lo);
@@ -1104,18 +1104,26 @@ static int split_prepare(pfc_job *j) {
             j->split_narrow = narrow;
             memcpy(j->split_start, start, sizeof(uint32_t) * (S + 1));
         }
-        // start residues of boundaries 1..S-1 for s0 and s1, per class
-        const size_t need32 = (size_t)2 * (S - 1) * n32, need64 = (size_t)2 * (S - 1) * n64;
-        if (n32 && j->split32.n < need32) CK(j->split32.alloc(c, need32));
-        if (n64 && j->split64.n < need64) CK(j->split64.alloc(c, need64));
+        // start residues of the sub-ranges for s0 and s1, per class; where the
+        // budget has no room for them the walk stays plain
+        const size_t need32 = (size_t)2 * S * n32, need64 = (size_t)2 * S * n64;
+        cudaError_t e = cudaSuccess;
+        if (n32 && j->split32.n < need32) e = j->split32.alloc(c, need32);
+        if (e == cudaSuccess && n64 && j->split64.n < need64) e = j->split64.alloc(c, need64);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            j->split32.release(c);
+            j->split64.release(c);
+            return PFC_OK;
+        }
+        CK(e);
         j->split_n = S;
         return PFC_OK;
     }
     return PFC_OK;
 }
 
-// one setup launch per size class for the start residues of boundaries
-// 1..split_n-1
+// one setup launch per size class for the start residues of the sub-ranges
 static int enqueue_split_setup(pfc_job *j) {
     pfc_ctx *c = j->ctx;
     const uint32_t S = j->split_n;
@@ -1136,9 +1144,9 @@ static int enqueue_split_setup(pfc_job *j) {
     }
     if (j->use32 && j->c32.p.p)
         c->launches += launch_split_setup32(j->c32.view(counts_ptr(j)), sw, j->split32.p,
-                                            j->split32.p + (size_t)(S - 1) * j->c32.cap, c->st);
+                                            j->split32.p + (size_t)S * j->c32.cap, c->st);
     if (j->use64 && j->c64.p.p) {
-        uint64_t *s0 = j->split64.p, *s1 = j->split64.p + (size_t)(S - 1) * j->c64.cap;
+        uint64_t *s0 = j->split64.p, *s1 = j->split64.p + (size_t)S * j->c64.cap;
         if (lazy) c->launches += launch_split_setup64w(j->c64.view(counts_ptr(j) + 1), sw, s0, s1, c->st);
         else c->launches += launch_split_setup64(j->c64.view(counts_ptr(j) + 1), sn, s0, s1, c->st);
     }

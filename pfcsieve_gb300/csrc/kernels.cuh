@@ -75,11 +75,11 @@ struct WalkArgs {
 };
 
 // A walk over n split into sub-ranges: candidate i's sub-range k covers steps
-// [start[k], start[k+1]) and begins from the residue at start[k], which the
-// setup kernel computed into s0/s1 + (k-1) * pitch for k >= 1 (sub-range 0
-// begins from the candidate's own state).  One launch walks every (candidate,
-// sub-range) pair (grid y = k); the last sub-range leaves the candidate's
-// final residue in its state and every sub-range adds its steps to nnext.
+// [start[k], start[k+1]) and begins from the residue at start[k], in s0/s1 +
+// k * pitch.  One launch walks every (candidate, sub-range) pair (grid y = k);
+// the last sub-range leaves the candidate's final residue in its state, which
+// no sub-range reads (nothing orders the CTAs of a launch: sub-range 0 begins
+// from a copy), and every sub-range adds its steps to nnext.
 // Candidate sets too small to fill the GPU get more chains this way.
 constexpr int kMaxSplit = 8;
 template <class W>
@@ -87,11 +87,11 @@ struct SplitArgs {
     uint32_t start[kMaxSplit + 1];
     uint32_t n;        // sub-ranges (1 = no split)
     uint32_t pitch;    // stride of the start-residue arrays (the class capacity)
-    W *s0, *s1;        // start residues of sub-ranges 1 .. n-1
+    W *s0, *s1;        // start residues of the sub-ranges
 };
 
 // the setup programs of a split walk's boundaries 1..n-1 (n <= kMaxSplit),
-// evaluated in one launch (grid y = boundary - 1)
+// evaluated in one launch (grid y = sub-range; 0 copies the state)
 template <class SW>
 struct SplitSetup {
     unsigned mode;
@@ -175,7 +175,7 @@ constexpr uint64_t kTcMinWordsTop = 112;
 constexpr uint32_t kTcMinStartTop = 40000;
 int launch_setup32_tc(const ClassBuf<uint32_t> &c, const SetupArgs<WideWord> &a, const TcTiles &ta,
                       const TcTiles &tb, uint32_t *err, cudaStream_t st, uint32_t block0 = 0, uint32_t nblocks = 0);
-// start residues of a split walk: boundary k's into s0/s1 + (k-1) * c.cap
+// start residues of a split walk: sub-range k's into s0/s1 + k * c.cap
 int launch_split_setup32(const ClassBuf<uint32_t> &c, const SplitSetup<WideWord> &ss, uint32_t *s0, uint32_t *s1,
                          cudaStream_t st);
 int launch_split_setup64(const ClassBuf<uint64_t> &c, const SplitSetup<uint64_t> &ss, uint64_t *s0, uint64_t *s1,

@@ -37,9 +37,10 @@ __global__ void __launch_bounds__(256) setup_kernel(ClassBuf<typename T::W> c, S
     }
 }
 
-// The start residues of a split walk's boundaries, all in one launch: CTA
-// row blockIdx.y evaluates boundary y + 1's programs for every candidate
-// (the rows run side by side instead of one launch after another).
+// The start residues of a split walk's sub-ranges, all in one launch: CTA row
+// blockIdx.y evaluates boundary y's programs for every candidate (the rows run
+// side by side instead of one launch after another).  Row 0 copies the
+// candidate's state, which the walk's last sub-range overwrites.
 template <class T>
 __global__ void __launch_bounds__(256) split_setup_kernel(ClassBuf<typename T::W> c, SplitSetup<typename T::SW> ss,
                                                           typename T::W *out0, typename T::W *out1) {
@@ -47,17 +48,24 @@ __global__ void __launch_bounds__(256) split_setup_kernel(ClassBuf<typename T::W
     const uint32_t k = blockIdx.y;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t cnt = min(*c.count, c.cap);
-    if (blockIdx.x * blockDim.x >= cnt || k + 1 >= ss.n) return;   // whole CTAs only (staged words)
+    if (blockIdx.x * blockDim.x >= cnt || k >= ss.n) return;   // whole CTAs only (staged words)
     const bool act = i < cnt;
+    if (k == 0) {
+        if (act) {
+            out0[i] = c.s0[i];
+            out1[i] = c.s1[i];
+        }
+        return;
+    }
     typename T::M m;
     m.init(act ? c.p[i] : (W)3);
     const typename T::SC sc = T::sctx(m);
     W s0, s1 = 0;
     if (ss.mode == (PFC_FACTORIAL | PFC_COMPOSITORIAL)) {
-        s1 = run_prog<T>(m, sc, ss.a[k], m.one);
-        s0 = run_prog<T>(m, sc, ss.b[k], s1);
+        s1 = run_prog<T>(m, sc, ss.a[k - 1], m.one);
+        s0 = run_prog<T>(m, sc, ss.b[k - 1], s1);
     } else {
-        s0 = run_prog<T>(m, sc, ss.a[k], m.one);
+        s0 = run_prog<T>(m, sc, ss.a[k - 1], m.one);
     }
     if (act) {
         out0[(size_t)k * c.cap + i] = s0;
@@ -101,9 +109,9 @@ __device__ __forceinline__ void walk_body(ClassBuf<typename T::W> c, WalkArgs a,
     }
     // start residues: the candidate's state, or the sub-range's start
     W *in0 = c.s0, *in1 = c.s1;
-    if (SPLIT && sub > 0) {
-        in0 = sp.s0 + (size_t)(sub - 1) * sp.pitch;
-        in1 = sp.s1 + (size_t)(sub - 1) * sp.pitch;
+    if (SPLIT) {
+        in0 = sp.s0 + (size_t)sub * sp.pitch;
+        in1 = sp.s1 + (size_t)sub * sp.pitch;
     }
     if (FUSED) {
         x[0] = act[0] ? in0[idx[0]] : 0;
@@ -227,7 +235,7 @@ template <class T>
 static int launch_split_setup(const ClassBuf<typename T::W> &c, const SplitSetup<typename T::SW> &ss,
                               typename T::W *s0, typename T::W *s1, cudaStream_t st) {
     if (!c.cap || ss.n < 2 || ss.n > (uint32_t)kMaxSplit) return 0;
-    split_setup_kernel<T><<<dim3(grid_for(c.cap), ss.n - 1), 256, 0, st>>>(c, ss, s0, s1);
+    split_setup_kernel<T><<<dim3(grid_for(c.cap), ss.n), 256, 0, st>>>(c, ss, s0, s1);
     return 1;
 }
 int launch_split_setup32(const ClassBuf<uint32_t> &c, const SplitSetup<WideWord> &ss, uint32_t *s0, uint32_t *s1,

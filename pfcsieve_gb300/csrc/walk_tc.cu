@@ -831,7 +831,7 @@ __device__ __forceinline__ void walk_tc(const ClassBuf<typename T::W> &c, const 
         auto second = [&](uint32_t s) { return (s ? a.second[1] : a.second[0]) != 0; };
         auto start = [&](uint32_t s) -> W {
             const W *in = second(s) ? c.s1 : c.s0;
-            if (split && sub) in = (second(s) ? sp->s1 : sp->s0) + (size_t)(sub - 1) * sp->pitch;
+            if (split) in = (second(s) ? sp->s1 : sp->s0) + (size_t)sub * sp->pitch;
             return act ? in[ci] : (W)0;
         };
         auto finish = [&](uint32_t s, W r) {
