@@ -700,6 +700,22 @@ static int setup_prepare(pfc_job *j) {
     return narrow_setup_applies(j) ? ensure_narrow(j) : PFC_OK;
 }
 
+// the tensor-core setup's arguments: the paired programs and their tiles
+struct TcSetup {
+    SetupArgs<WideWord> a;
+    TcTiles ta, tb;
+};
+static TcSetup tc_setup_args(const pfc_job *j) {
+    TcSetup t;
+    t.a.mode = j->mode;
+    t.a.a = j->tc_view[0];
+    t.a.b = j->tc_view[1];
+    t.a.nnext0 = 0;
+    t.ta = TcTiles{j->tct.p, j->tc_ntiles[0]};
+    t.tb = TcTiles{j->tct.p + (size_t)j->tc_ntiles[0] * tc_tile_bytes(), j->tc_ntiles[1]};
+    return t;
+}
+
 static int enqueue_setup(pfc_job *j) {
     pfc_ctx *c = j->ctx;
     {
@@ -724,24 +740,16 @@ static int enqueue_setup(pfc_job *j) {
     sw.nnext0 = 0;
     if (j->use32) {
         if (tc_setup32_applies(j)) {
-            const TcTiles ta{j->tct.p, j->tc_ntiles[0]},
-                tb{j->tct.p + (size_t)j->tc_ntiles[0] * tc_tile_bytes(), j->tc_ntiles[1]};
-            SetupArgs<WideWord> stc = s32;
-            stc.a = j->tc_view[0];
-            stc.b = j->tc_view[1];
-            c->launches += launch_setup32_tc(j->c32.view(counts_ptr(j)), stc, ta, tb, &j->stats.p->tc_err, c->st);
+            const TcSetup t = tc_setup_args(j);
+            c->launches += launch_setup32_tc(j->c32.view(counts_ptr(j)), t.a, t.ta, t.tb, &j->stats.p->tc_err, c->st);
         } else {
             c->launches += launch_setup32(j->c32.view(counts_ptr(j)), s32, c->st);
         }
     }
     if (j->use64) {
         if (tc_setup_applies(j)) {
-            const TcTiles ta{j->tct.p, j->tc_ntiles[0]},
-                tb{j->tct.p + (size_t)j->tc_ntiles[0] * tc_tile_bytes(), j->tc_ntiles[1]};
-            SetupArgs<WideWord> stc = sw;
-            stc.a = j->tc_view[0];
-            stc.b = j->tc_view[1];
-            c->launches += launch_setup64_tc(j->c64.view(counts_ptr(j) + 1), stc, ta, tb, j->seg_hi <= kLazyEnd,
+            const TcSetup t = tc_setup_args(j);
+            c->launches += launch_setup64_tc(j->c64.view(counts_ptr(j) + 1), t.a, t.ta, t.tb, j->seg_hi <= kLazyEnd,
                                              &j->stats.p->tc_err, c->st);
         } else if (j->seg_hi <= kLazyEnd) {
             c->launches += launch_setup64w(j->c64.view(counts_ptr(j) + 1), sw, c->st);
@@ -1530,39 +1538,33 @@ static uint64_t powmod_h(uint64_t a, uint64_t e, uint64_t p) {
     return r;
 }
 
-// Run the job's setup programs of one word form on the single candidate p and
-// return its residues in plain form (s1: the combined search's compositorial).
-template <class W, class SW>
-static int setup_on_prime(pfc_job *j, const DevProg<SW> &a, const DevProg<SW> &b, uint64_t p, uint64_t &s0,
-                          uint64_t &s1) {
+// Run a setup (`launch`, which returns the kernels it launched) on the single
+// candidate p and return its residues in plain form (s1: the combined search's
+// compositorial).
+template <class W, class Launch>
+static int setup_on_prime(pfc_job *j, uint64_t p, uint64_t &s0, uint64_t &s1, Launch launch) {
     pfc_ctx *c = j->ctx;
     DevClass<W> cls;
-    DArr<uint32_t> cnt;
-    CK(cls.ensure(c, 1));
-    cudaError_t e = cnt.alloc(c, 1);
+    DArr<uint32_t> cnt;   // candidates, and the error flag of a tensor-core setup
     const W pw = (W)p;
-    const uint32_t one = 1;
+    uint32_t one[2] = {1, 0};
+    cudaError_t e = cls.ensure(c, 1);
+    if (e == cudaSuccess) e = cnt.alloc(c, 2);
     if (e == cudaSuccess) e = cudaMemcpyAsync(cls.p.p, &pw, sizeof(W), cudaMemcpyHostToDevice, c->st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(cnt.p, &one, sizeof(one), cudaMemcpyHostToDevice, c->st);
-    SetupArgs<SW> sa;
-    sa.mode = j->mode;
-    sa.a = a.view;
-    sa.b = b.view;
-    sa.nnext0 = 0;
+    if (e == cudaSuccess) e = cudaMemcpyAsync(cnt.p, one, sizeof(one), cudaMemcpyHostToDevice, c->st);
     if (e == cudaSuccess) {
-        const ClassBuf<W> view = cls.view(cnt.p);
-        if constexpr (sizeof(W) == 4) c->launches += launch_setup32(view, sa, c->st);
-        else if constexpr (std::is_same<SW, WideWord>::value) c->launches += launch_setup64w(view, sa, c->st);
-        else c->launches += launch_setup64(view, sa, c->st);
+        c->launches += launch(cls.view(cnt.p), cnt.p + 1);
         e = cudaGetLastError();
     }
     W h0 = 0, h1 = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h0, cls.s0.p, sizeof(W), cudaMemcpyDeviceToHost, c->st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h1, cls.s1.p, sizeof(W), cudaMemcpyDeviceToHost, c->st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(one, cnt.p, sizeof(one), cudaMemcpyDeviceToHost, c->st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
     cls.release(c);
     cnt.release(c);
     CK(e);
+    if (one[1]) return PFC_ERR_CUDA;   // a wait gave up
     // Montgomery form with R = 2^32 (class 32) or 2^64 -> plain
     const uint64_t rinv = powmod_h(2, (p - 1) - (sizeof(W) == 4 ? 32 : 64), p);
     s0 = mulmod_h((uint64_t)h0, rinv, p);
@@ -1570,52 +1572,111 @@ static int setup_on_prime(pfc_job *j, const DevProg<SW> &a, const DevProg<SW> &b
     return PFC_OK;
 }
 
+// The size classes of the job's p range (class 32, class 64 below and from
+// 2^64/3), each checked on one test prime of its own (kVerifyPrime).
+static bool has_class(const pfc_job *j, int t) {
+    return t == 0 ? j->pmin < kClassSplit : t == 1 ? j->pmax > kClassSplit && j->pmin < kLazyEnd : j->pmax > kLazyEnd;
+}
+
+static bool residues_match(unsigned mode, const SlowProducts &sp, int t, uint64_t s0, uint64_t s1) {
+    const uint64_t P = sp.P[t], C = sp.C[t], F = mulmod_h(P, C, kVerifyPrime[t]);
+    switch (mode) {
+        case PFC_FACTORIAL: return s0 == F;
+        case PFC_PRIMORIAL: return s0 == P;
+        case PFC_COMPOSITORIAL: return s0 == C;
+        default: return s0 == F && s1 == C;
+    }
+}
+
+// The tensor cores' form of the programs (merged and paired words, as the
+// tiles hold them) by the setup kernel of each class that takes it.  Tiles that
+// the budget has no room for are none that a segment would use.
+static int verify_tiles(pfc_job *j, const SlowProducts &sp) {
+    pfc_ctx *c = j->ctx;
+    const bool takes[3] = {has_class(j, 0) && j->tc_words >= kTcMinWords32,
+                           has_class(j, 1) && j->tc_words >= kTcMinWords64, j->top_tc};
+    if (!c->setup_tc || j->no_tiles || !(takes[0] || takes[1] || takes[2])) return PFC_OK;
+    const bool packed = j->tc_packed;
+    int rc = tc_prepare(j);
+    for (int t = 0; t < 3 && !rc; ++t) {
+        if (!takes[t]) continue;
+        const TcSetup s = tc_setup_args(j);
+        uint64_t s0 = 0, s1 = 0;
+        if (t == 0)
+            rc = setup_on_prime<uint32_t>(j, kVerifyPrime[t], s0, s1, [&](const ClassBuf<uint32_t> &v, uint32_t *err) {
+                return launch_setup32_tc(v, s.a, s.ta, s.tb, err, c->st);
+            });
+        else
+            rc = setup_on_prime<uint64_t>(j, kVerifyPrime[t], s0, s1, [&](const ClassBuf<uint64_t> &v, uint32_t *err) {
+                return launch_setup64_tc(v, s.a, s.ta, s.tb, t == 1, err, c->st);
+            });
+        if (!rc && !residues_match(j->mode, sp, t, s0, s1)) rc = PFC_ERR_VALIDATION;
+    }
+    if (!packed) {   // the segments' buffers come first
+        j->tct.release(c);
+        j->tc_src.release(c);
+        j->tc_groups.release(c);
+        j->tc_packed = false;
+    }
+    if (rc == PFC_ERR_NOMEM) {
+        cudaGetLastError();
+        rc = PFC_OK;
+    }
+    return rc;
+}
+
+// The programs by the integer pipe's setup kernel of each class; `bytes` adds
+// up their tables.
+static int verify_programs(pfc_job *j, const SlowProducts &sp, uint64_t &bytes) {
+    pfc_ctx *c = j->ctx;
+    const bool narrow = j->narrow;
+    int rc = ensure_narrow(j);
+    for (int t = 0; t < 3 && !rc; ++t) {
+        if (!has_class(j, t) || (t == 1 && !j->aw.words.p)) continue;
+        uint64_t s0 = 0, s1 = 0;
+        if (t == 2) {
+            const SetupArgs<uint64_t> s{j->mode, j->a64.view, j->b64.view, 0};
+            rc = setup_on_prime<uint64_t>(j, kVerifyPrime[t], s0, s1, [&](const ClassBuf<uint64_t> &v, uint32_t *) {
+                return launch_setup64(v, s, c->st);
+            });
+            bytes += (j->a64.words.n + j->b64.words.n) * 8;
+        } else {
+            const DevProg<WideWord> &a = t ? j->aw : j->a32, &b = t ? j->bw : j->b32;
+            const SetupArgs<WideWord> s{j->mode, a.view, b.view, 0};
+            if (t)
+                rc = setup_on_prime<uint64_t>(j, kVerifyPrime[t], s0, s1, [&](const ClassBuf<uint64_t> &v, uint32_t *) {
+                    return launch_setup64w(v, s, c->st);
+                });
+            else
+                rc = setup_on_prime<uint32_t>(j, kVerifyPrime[t], s0, s1, [&](const ClassBuf<uint32_t> &v, uint32_t *) {
+                    return launch_setup32(v, s, c->st);
+                });
+            bytes += (a.words.n + b.words.n) * sizeof(WideWord);
+        }
+        if (!rc && !residues_match(j->mode, sp, t, s0, s1)) rc = PFC_ERR_VALIDATION;
+    }
+    if (!narrow && j->narrow) {   // (built for the check)
+        j->a64.release(c);
+        j->b64.release(c);
+        j->narrow = false;
+    }
+    return rc;
+}
+
 extern "C" int pfc_job_verify_tables(pfc_job *j, uint64_t *table_bytes) {
     if (!j) return PFC_ERR_ARG;
     pfc_ctx *c = j->ctx;
     CK(cudaSetDevice(c->device));
     CK(cudaStreamSynchronize(c->st));
-    {
-        const int nrc = ensure_narrow(j);
-        if (nrc) return nrc;
-    }
     const uint32_t startN = j->nmin - 1;
     // slow side for the setup programs: k in [2, n0 - 1]
     SlowProducts sp;
     int rc = slow_products(c, 2, (uint64_t)startN + 1, sp);
     if (rc) return rc;
     uint64_t bytes = 0;
-    struct Form {
-        int form, t;   // setup form, test prime index
-        bool built;
-    } forms[3] = {{0, 0, j->a32.words.p != nullptr && j->pmin < kClassSplit},
-                  {1, 1, j->aw.words.p != nullptr && j->pmax > kClassSplit && j->pmin < kLazyEnd},
-                  {2, 2, j->a64.words.p != nullptr && j->pmax > kLazyEnd}};
-    for (const Form &f : forms) {
-        if (!f.built) continue;
-        const uint64_t p = kVerifyPrime[f.t];
-        uint64_t s0 = 0, s1 = 0;
-        if (f.form == 0) {
-            rc = setup_on_prime<uint32_t, WideWord>(j, j->a32, j->b32, p, s0, s1);
-            bytes += (j->a32.words.n + j->b32.words.n) * sizeof(WideWord);
-        } else if (f.form == 1) {
-            rc = setup_on_prime<uint64_t, WideWord>(j, j->aw, j->bw, p, s0, s1);
-            bytes += (j->aw.words.n + j->bw.words.n) * sizeof(WideWord);
-        } else {
-            rc = setup_on_prime<uint64_t, uint64_t>(j, j->a64, j->b64, p, s0, s1);
-            bytes += (j->a64.words.n + j->b64.words.n) * 8;
-        }
-        if (rc) return rc;
-        const uint64_t P = sp.P[f.t], C = sp.C[f.t], F = mulmod_h(P, C, p);
-        bool ok;
-        switch (j->mode) {
-            case PFC_FACTORIAL: ok = s0 == F; break;
-            case PFC_PRIMORIAL: ok = s0 == P; break;
-            case PFC_COMPOSITORIAL: ok = s0 == C; break;
-            default: ok = s0 == F && s1 == C; break;
-        }
-        if (!ok) return PFC_ERR_VALIDATION;
-    }
+    rc = verify_tiles(j, sp);
+    if (!rc) rc = verify_programs(j, sp, bytes);
+    if (rc) return rc;
     // walk tables of [nmin, nmax): the primorial's prime list, the
     // compositorial's prime flags, read back from the device
     if (j->mode != PFC_FACTORIAL && j->nmax > j->nmin) {
