@@ -670,7 +670,6 @@ static int ensure_narrow(pfc_job *j) {
     if (!ps) return PFC_ERR_ARG;
     CK(j->a64.upload(c, ps->na));
     CK(j->b64.upload(c, ps->nb));
-    j->setup_mulmods64 = ps->na.mulmods() + ps->nb.mulmods();
     j->narrow = true;
     return PFC_OK;
 }
@@ -1521,7 +1520,13 @@ extern "C" int pfc_segment_state(pfc_job *j, uint64_t *p, uint64_t *s0, uint64_t
 extern "C" uint64_t pfc_job_pairs(pfc_job *j) { return j ? j->pairs : 0; }
 
 extern "C" uint64_t pfc_job_setup_mulmods(pfc_job *j, int cls64) {
-    if (!j || (cls64 && ensure_narrow(j) != PFC_OK)) return 0;
+    if (!j) return 0;
+    if (cls64 && !j->setup_mulmods64 && j->pmax > kLazyEnd) {
+        // the 64-bit words, which the tensor-core setup leaves out: counted on
+        // the host, nothing of them is uploaded
+        const std::shared_ptr<const ProgSet> ps = ctx_progs(j->ctx, j->mode, j->nmin - 1, false, true);
+        if (ps) j->setup_mulmods64 = ps->na.mulmods() + ps->nb.mulmods();
+    }
     return cls64 ? j->setup_mulmods64 : j->setup_mulmods32;
 }
 

@@ -41,3 +41,18 @@ def test_the_check_runs_the_tiles(mode, nmin, lo, hi, classes):
     packs = 0 if not classes else 2 if mode == 5 else 1
     assert launches[1] - launches[0] == packs + classes
     assert len(set(nbytes)) == 1 and len(set(totals)) <= 1
+
+
+def test_setup_mulmods_is_a_read():
+    """The count of the 64-bit words that a search from 2^64/3 on leaves out: the same as with them, without work on
+    the device."""
+    case = (1, 400000, 400050, 2**63, 2**63 + 20000)
+    with pfc.Context(0) as c:
+        c.set_setup_tc(False)
+        with pfc.Job(c, *case) as job:
+            want = job.setup_mulmods(True)
+    words, squarings = pfc.setup_program_size(1, 400000, False)
+    assert want == words + squarings
+    with pfc.Context(0) as c, pfc.Job(c, *case) as job:
+        before = c.transfer_bytes(), c.launches
+        assert job.setup_mulmods(True) == want and (c.transfer_bytes(), c.launches) == before
