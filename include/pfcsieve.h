@@ -136,6 +136,11 @@ int pfc_ctx_set_walk_tc(pfc_ctx *ctx, int on);
 /* Number of kernels this context has launched so far. */
 uint64_t pfc_ctx_launch_count(pfc_ctx *ctx);
 
+/* Walk launches of this context so far, in searches and batches: *tc those on
+ * the tensor cores, *split those of searches cut into sub-ranges of n (either
+ * may be NULL).  What ran depends on sizes and on the memory budget. */
+int pfc_ctx_walk_counts(pfc_ctx *ctx, uint64_t *tc, uint64_t *split);
+
 /* Bytes this context has copied host->device and device->host so far. */
 int pfc_ctx_transfer_bytes(pfc_ctx *ctx, uint64_t *h2d, uint64_t *d2h);
 

@@ -80,6 +80,7 @@ def lib():
             "pfc_ctx_destroy": (ctypes.c_int, [vp]),
             "pfc_ctx_stream": (vp, [vp]),
             "pfc_ctx_launch_count": (u64, [vp]),
+            "pfc_ctx_walk_counts": (ctypes.c_int, [vp, P(u64), P(u64)]),
             "pfc_ctx_transfer_bytes": (ctypes.c_int, [vp, P(u64), P(u64)]),
             "pfc_ctx_device_info": (ctypes.c_int, [vp, ctypes.c_char_p, sz, P(ctypes.c_int)]),
             "pfc_job_create": (ctypes.c_int, [vp, ctypes.c_uint, u32, u32, u64, u64, P(vp)]),
@@ -180,6 +181,12 @@ class Context:
     @property
     def launches(self):
         return lib().pfc_ctx_launch_count(self.h)
+
+    def walk_counts(self):
+        """(walk launches on the tensor cores, walk launches in sub-ranges of n) so far."""
+        a, b = ctypes.c_uint64(0), ctypes.c_uint64(0)
+        _ck(lib().pfc_ctx_walk_counts(self.h, ctypes.byref(a), ctypes.byref(b)), "walk_counts")
+        return a.value, b.value
 
     def transfer_bytes(self):
         """(host->device, device->host) bytes copied so far."""

@@ -98,7 +98,7 @@ struct pfc_job {
     };
     cudaGraphExec_t graph = nullptr;
     GraphKey gkey{};
-    uint64_t graph_kernels = 0;
+    uint64_t graph_kernels = 0, graph_tc_walks = 0, graph_split_walks = 0;
     uint64_t segments = 0;   // segments committed (the first one runs without a graph)
 };
 
@@ -202,6 +202,13 @@ extern "C" int pfc_ctx_destroy(pfc_ctx *c) {
 extern "C" void *pfc_ctx_stream(pfc_ctx *c) { return c ? (void *)c->st : nullptr; }
 
 extern "C" uint64_t pfc_ctx_launch_count(pfc_ctx *c) { return c ? c->launches : 0; }
+
+extern "C" int pfc_ctx_walk_counts(pfc_ctx *c, uint64_t *tc, uint64_t *split) {
+    if (!c) return PFC_ERR_ARG;
+    if (tc) *tc = c->tc_walks;
+    if (split) *split = c->split_walks;
+    return PFC_OK;
+}
 
 extern "C" int pfc_ctx_transfer_bytes(pfc_ctx *c, uint64_t *h2d, uint64_t *d2h) {
     if (!c) return PFC_ERR_ARG;
@@ -886,6 +893,8 @@ static int enqueue_iter_range(pfc_job *j, uint32_t lo, uint32_t hi, bool split =
     }
     auto walk = [&](const WalkArgs &w) {
         const int fused = w.mult2 != nullptr;
+        c->tc_walks += tc32 + tc64;
+        if (split) c->split_walks += j->use32 + j->use64;
         const bool lazy = j->seg_hi <= kLazyWalkEnd;
         if (tc32 || tc64) {
             const uint32_t top = top_mult(j, hi);
@@ -1331,13 +1340,17 @@ static int segment_body_graph(pfc_job *j) {
     if (!j->graph || memcmp(&k, &j->gkey, sizeof(k)) != 0) {
         if (j->graph) cudaGraphExecDestroy(j->graph);
         j->graph = nullptr;
-        const uint64_t l0 = c->launches, d0 = c->d2h;
+        const uint64_t l0 = c->launches, d0 = c->d2h, t0 = c->tc_walks, s0 = c->split_walks;
         CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
         const int rc = enqueue_segment_body(j);
         cudaGraph_t g = nullptr;
         const cudaError_t e = cudaStreamEndCapture(c->st, &g);
         j->graph_kernels = c->launches - l0;
+        j->graph_tc_walks = c->tc_walks - t0;
+        j->graph_split_walks = c->split_walks - s0;
         c->launches = l0;   // counted when the graph is launched
+        c->tc_walks = t0;
+        c->split_walks = s0;
         c->d2h = d0;
         if (rc) {
             if (g) cudaGraphDestroy(g);
@@ -1351,6 +1364,8 @@ static int segment_body_graph(pfc_job *j) {
     }
     CK(cudaGraphLaunch(j->graph, c->st));
     c->launches += j->graph_kernels;
+    c->tc_walks += j->graph_tc_walks;
+    c->split_walks += j->graph_split_walks;
     c->d2h += sizeof(SegStats);
     CK(cudaStreamSynchronize(c->st));
     j->stats_fresh = true;

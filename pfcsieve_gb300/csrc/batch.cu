@@ -1297,6 +1297,7 @@ static void launch_tc_walks(pfc_batch *b, int l, int shape, const JobDev<typenam
     const int si = (l == 0 ? 0 : 3) + ((l == 2) != (shape == 1) ? 2 : 0);
     cudaStream_t st = b->st[si];
     for (const auto &ps : g.passes) {
+        ++b->ctx->tc_walks;
         cudaMemsetAsync(g.digits.p, 0, 2 * g.plan.size() * sizeof(uint32_t), st);
         b->ctx->launches += launch_walk_words_many(g.d_words.p + ps.words0, ps.words, ps.words_ctas, shape, st);
         if (l == 0) b->ctx->launches += launch_walk_tc32_many(g.d_w32.p + ps.win0, ps.wins, ps.ctas, shape, h, st);

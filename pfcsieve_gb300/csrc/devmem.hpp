@@ -29,6 +29,7 @@ struct pfc_ctx {
     char name[256] = {0};
     uint64_t budget = 0, used = 0;
     uint64_t launches = 0;
+    uint64_t tc_walks = 0, split_walks = 0;   // walk launches on the tensor cores, in sub-ranges
     uint64_t h2d = 0, d2h = 0;   // bytes copied by this context
     uint64_t *d_pat = nullptr;
     int walk_var[3][2] = {{0, 0}, {0, 0}, {0, 0}};   // walk variant per size class and kind (fused)
