@@ -1,10 +1,12 @@
 """Which walk runs (pfc_ctx_walk_counts), in the cases whose tests compare two walks: the tensor-core walk and the
 split where they are meant, none where they are switched off, on the stream, captured and replayed, and in
 batches with small memory budgets.  Integers: equal, no tolerance."""
+import numpy as np
 import pytest
 
 pfc = pytest.importorskip("pfcsieve_gb300")
 
+from oracle import oracle as o  # noqa: E402
 from tests import test_gpu_split_last as last  # noqa: E402
 from tests import test_gpu_walk_tc as tc  # noqa: E402
 
@@ -59,3 +61,28 @@ def test_batches(contexts, budget):
     on, off = contexts
     # its searches are of class 32, class 64 in both word shapes, and from 2^64/3; small tables take several passes
     assert on[0] >= (8 if budget else 4) and off[0] == 0
+
+
+@pytest.mark.parametrize("cls,lo", [(0, 10**9), (1, 2**40)])
+def test_every_per_step_variant_vs_oracle(contexts, cls, lo):
+    """Each compiled variant of the per-step walk, which the tensor-core walk stands in for at these sizes, gives
+    the oracle's residues, hits and checksum."""
+    hi = lo + 300000
+    cands = o.candidates(lo, hi)
+    for fused, modes in ((0, (1, 2, 4)), (1, (5,))):
+        for mode in modes:
+            ohits, osum, terms = o.sieve(mode, 3000, 7001, cands, want_terms=True)
+            for v in range({(0, 0): 3, (0, 1): 2, (1, 0): 4, (1, 1): 2}[cls, fused]):
+                with pfc.Context(0) as c:
+                    c.set_walk_tc(0)
+                    c.set_split(False)
+                    c.set_walk_variant(cls, fused, v)
+                    with pfc.Job(c, mode, 3000, 7001, lo, hi) as job:
+                        job.segment(lo, hi)
+                        p, s0, s1 = job.segment_state()
+                        k = np.argsort(p)
+                        assert np.array_equal(p[k], cands) and np.array_equal(s0[k], terms[:, 0]), (mode, v)
+                        assert mode != 5 or np.array_equal(s1[k], terms[:, 2]), v
+                        assert np.array_equal(o.sort_factors(job.drain_hits()), ohits), (mode, v)
+                        assert job.totals()[0] == osum, (mode, v)
+    assert all(n == (0, 0) for n in contexts)
