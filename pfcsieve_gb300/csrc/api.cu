@@ -58,7 +58,7 @@ struct pfc_job {
     DArr<uint32_t> cmult;       // compositorial multipliers of the current chunk
     DArr<uint32_t> ramp;        // the combined search's factorial multipliers (n) of the chunk
     DArr<uint8_t> words[2];     // the tensor-core walk's tables of the current chunk, per stream
-    bool no_words = false;      // there was no room for them: the job's walks take the per-step kernels
+    bool no_words = false;      // there was no room for them: the segment's walks take the per-step kernels
     std::vector<uint32_t> h_qlist;
 
     DevClass<uint32_t> c32;
@@ -91,7 +91,7 @@ struct pfc_job {
     // the post-generation part of a segment captured as a CUDA graph, replayed
     // while the key (buffers, launch shapes, kernel choices) is unchanged
     struct GraphKey {
-        const void *p32, *p64, *hits, *cmult, *ramp, *split32, *split64, *words[2];
+        const void *p32, *p64, *hits, *cmult, *ramp, *split32, *split64, *words[2], *tct, *tc_groups;
         uint64_t cap32, cap64, hitcap;
         int lazy, use32, use64, var[3][2], setup_tc, walk_tc;
         uint32_t split_n, split_start[kMaxSplit + 1];
@@ -226,8 +226,41 @@ extern "C" int pfc_ctx_device_info(pfc_ctx *c, char *name, size_t cap, int *sms)
 
 // --------------------------------------------------------------------- job
 
+// The tiles, and their word sources and groups (packed again on next use).
+static void release_tiles(pfc_job *j) {
+    j->tct.release(j->ctx);
+    j->tc_src.release(j->ctx);
+    j->tc_groups.release(j->ctx);
+    j->tc_packed = false;
+}
+static void release_words(pfc_job *j) {
+    for (auto &w : j->words) w.release(j->ctx);
+    j->no_words = true;   // (not tried again in this segment: the next call may be a capture)
+}
+
+static void release_split_progs(pfc_job *j) {
+    if (j->graph) cudaGraphExecDestroy(j->graph);   // (its key holds no pointer to them)
+    j->graph = nullptr;
+    for (auto *v : {&j->split_wa, &j->split_wb}) {
+        for (auto &pg : *v) pg.release(j->ctx);
+        v->clear();
+    }
+    for (auto *v : {&j->split_na, &j->split_nb}) {
+        for (auto &pg : *v) pg.release(j->ctx);
+        v->clear();
+    }
+}
+
+void pfc::reclaim_spare(pfc_ctx *c) {
+    for (pfc_job *j : c->jobs) {
+        if (j->words[0].p || j->words[1].p) release_words(j);
+        if (j->tct.p) release_tiles(j);
+    }
+}
+
 static int job_release(pfc_job *j) {
     pfc_ctx *c = j->ctx;
+    c->jobs.erase(std::remove(c->jobs.begin(), c->jobs.end(), j), c->jobs.end());
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->st);
     if (j->graph) cudaGraphExecDestroy(j->graph);
@@ -250,10 +283,7 @@ static int job_release(pfc_job *j) {
     j->c64.release(c);
     j->hits.release(c);
     j->stats.release(c);
-    for (auto &pg : j->split_wa) pg.release(c);
-    for (auto &pg : j->split_wb) pg.release(c);
-    for (auto &pg : j->split_na) pg.release(c);
-    for (auto &pg : j->split_nb) pg.release(c);
+    release_split_progs(j);
     j->split32.release(c);
     j->split64.release(c);
     if (j->h_stats) c->pinned_stats.push_back(j->h_stats);   // kept for the next job
@@ -548,6 +578,7 @@ extern "C" int pfc_job_create(pfc_ctx *c, unsigned mode, uint32_t nmin, uint32_t
         delete j;
         return cuda_fail(e);
     }
+    c->jobs.push_back(j);
     *out = j;
     return PFC_OK;
 }
@@ -613,6 +644,7 @@ static int enqueue_gen(pfc_job *j, uint64_t lo, uint64_t hi) {
     CK(cudaGetLastError());
     j->seg_lo = lo;
     j->seg_hi = hi;
+    j->no_words = false;
     j->stage = 1;
     return PFC_OK;
 }
@@ -626,8 +658,9 @@ extern "C" int pfc_gen_candidates(pfc_job *j, uint64_t p_lo, uint64_t p_hi) {
     return enqueue_gen(j, p_lo, p_hi);
 }
 
-// The wide programs as fp16 tiles for the tensor-core setup, packed once per
-// job on the context stream (before any capture of a segment graph).
+// The wide programs as fp16 tiles for the tensor-core setup, packed on the
+// context stream (before any capture of a segment graph) and kept while the
+// budget has room for them.
 static int tc_prepare(pfc_job *j) {
     if (j->tc_packed) return PFC_OK;
     pfc_ctx *c = j->ctx;
@@ -636,9 +669,9 @@ static int tc_prepare(pfc_job *j) {
     std::vector<uint32_t> src(pa.src), groups(pa.groups);
     src.insert(src.end(), pb.src.begin(), pb.src.end());
     groups.insert(groups.end(), pb.groups.begin(), pb.groups.end());
-    CK(j->tct.alloc(c, std::max<size_t>((na + nb) * tb, 16)));
-    CK(j->tc_src.upload(c, src));
-    CK(j->tc_groups.upload(c, groups));
+    CK(j->tct.alloc(c, std::max<size_t>((na + nb) * tb, 16), true));
+    CK(j->tc_src.upload(c, src, true));
+    CK(j->tc_groups.upload(c, groups, true));
     // the words: the lazy class-64 copy of the programs, or the class-32 one (the same programs)
     const bool w64 = j->aw.view.ngroups || j->bw.view.ngroups;
     const WideWord *wa = w64 ? j->aw.words.p : j->a32.words.p, *wb = w64 ? j->bw.words.p : j->b32.words.p;
@@ -693,9 +726,7 @@ static int setup_prepare(pfc_job *j) {
         if (rc && rc != PFC_ERR_NOMEM) return rc;
         if (rc) {
             cudaGetLastError();
-            j->tct.release(j->ctx);
-            j->tc_src.release(j->ctx);
-            j->tc_groups.release(j->ctx);
+            release_tiles(j);
             if (j->pmin >= kLazyEnd) {   // (the 896-bit words were for the tiles alone)
                 j->aw.release(j->ctx);
                 j->bw.release(j->ctx);
@@ -832,10 +863,9 @@ static void ensure_words(pfc_job *j, uint32_t steps) {
     if (j->no_words || iter_end(j) == iter_begin(j) || !(walk_tc32_applies(j, steps) || walk_tc64_applies(j, steps))) return;
     const size_t need = walk_tc_words_bytes(top_mult(j, iter_end(j)), steps);
     for (int k = 0; k < (j->mode == (PFC_FACTORIAL | PFC_COMPOSITORIAL) ? 2 : 1); ++k)
-        if (j->words[k].n < need && j->words[k].alloc(j->ctx, need) != cudaSuccess) {
+        if (j->words[k].n < need && j->words[k].alloc(j->ctx, need, true) != cudaSuccess) {
             cudaGetLastError();
-            for (auto &w : j->words) w.release(j->ctx);
-            j->no_words = true;   // (not tried again: the next call may be a capture)
+            release_words(j);
             return;
         }
 }
@@ -878,9 +908,25 @@ static int enqueue_iter_range(pfc_job *j, uint32_t lo, uint32_t hi, bool split =
         sp64.s1 = j->split64.p ? j->split64.p + (size_t)j->split_n * j->c64.cap : nullptr;
     }
     ensure_words(j, hi - lo);
-    const bool words = words_fit(j, top_mult(j, hi), hi - lo);
-    const bool tc32 = words && walk_tc32_applies(j, hi - lo), tc64 = words && walk_tc64_applies(j, hi - lo);
-    const bool per_step = (j->use32 && !tc32) || (j->use64 && !tc64);
+    bool tc32, tc64, per_step;
+    auto choose = [&]() {
+        const bool words = words_fit(j, top_mult(j, hi), hi - lo);
+        tc32 = words && walk_tc32_applies(j, hi - lo);
+        tc64 = words && walk_tc64_applies(j, hi - lo);
+        per_step = (j->use32 && !tc32) || (j->use64 && !tc64);
+    };
+    choose();
+    if (j->mode & PFC_COMPOSITORIAL) {
+        // multiplier tables of the chunk: compositorial (n or 1) and, for the
+        // per-step fused walk, factorial (n; the plain factorial walk forms n
+        // itself, shared by its two candidates, and gains nothing from a table).
+        // Room for them may be made from the words'.
+        const size_t need = ((size_t)(hi - lo) + 15) & ~(size_t)15;
+        if (j->cmult.n < need) CK(j->cmult.alloc(c, std::max<size_t>(need, 4096)));
+        choose();
+        if ((j->mode & PFC_FACTORIAL) && per_step && j->ramp.n < need) CK(j->ramp.alloc(c, std::max<size_t>(need, 4096)));
+        choose();
+    }
     // Where only tensor-core walks run, and not split, the compositorial's
     // table lists the composite n alone; else it holds 1 at prime n, which
     // keeps both chains, and the sub-ranges of a split, at the same steps.
@@ -947,13 +993,7 @@ static int enqueue_iter_range(pfc_job *j, uint32_t lo, uint32_t hi, bool split =
         return PFC_OK;
     }
     if (j->mode & PFC_COMPOSITORIAL) {
-        // multiplier tables of the chunk: compositorial (n or 1) and, for the
-        // per-step fused walk, factorial (n; the plain factorial walk forms n
-        // itself, shared by its two candidates, and gains nothing from a table)
-        const size_t need = ((size_t)(hi - lo) + 15) & ~(size_t)15;
         const bool fact = (j->mode & PFC_FACTORIAL) && per_step;
-        if (j->cmult.n < need) CK(j->cmult.alloc(c, std::max<size_t>(need, 4096)));
-        if (fact && j->ramp.n < need) CK(j->ramp.alloc(c, std::max<size_t>(need, 4096)));
         c->launches += composites ? launch_composites(j->cmult.p, j->primebits.p, j->nmin, lo, hi, c->st)
                                   : launch_cmult(j->cmult.p, fact ? j->ramp.p : nullptr, j->primebits.p, j->nmin, lo, hi, c->st);
         w.base = lo;
@@ -1068,6 +1108,15 @@ static int split_prepare(pfc_job *j) {
         const double x = b / 2.0;
         return x < 41 ? 0.0 : x * (1.0 - 1.0 / std::log(x)) / std::log(2.0) / 896.0 * 15.0;
     };
+    // where the budget has no room for a split the walk stays plain
+    auto no_split = [&](cudaError_t e) {
+        if (e != cudaErrorMemoryAllocation) return cuda_fail(e);
+        cudaGetLastError();
+        release_split_progs(j);
+        j->split32.release(c);
+        j->split64.release(c);
+        return PFC_OK;
+    };
     for (; S >= 2; --S) {
         uint32_t start[kMaxSplit + 1];
         const uint32_t align = tc ? walk_tc_align(top_mult(j, hi)) : 16u;
@@ -1098,41 +1147,36 @@ static int split_prepare(pfc_job *j) {
             }
             // boundaries too dear: fewer sub-ranges or none
             if (tc && !keep ? tc_us(S, (double)cost, (double)most) >= tc_us(1, 0, 0) : cost * 6 > walk) continue;
-            for (auto &pg : j->split_wa) pg.release(c);
-            for (auto &pg : j->split_wb) pg.release(c);
-            for (auto &pg : j->split_na) pg.release(c);
-            for (auto &pg : j->split_nb) pg.release(c);
+            release_split_progs(j);
             j->split_wa.assign(wide ? S - 1 : 0, DevProg<WideWord>());
             j->split_wb.assign(wide ? S - 1 : 0, DevProg<WideWord>());
             j->split_na.assign(narrow ? S - 1 : 0, DevProg<uint64_t>());
             j->split_nb.assign(narrow ? S - 1 : 0, DevProg<uint64_t>());
+            cudaError_t e = cudaSuccess;
+            auto up = [&](auto &dst, const auto &prog) {
+                if (e == cudaSuccess) e = dst.upload(c, prog, {}, true);
+            };
             for (uint32_t k = 1; k < S; ++k) {
                 if (wide) {
-                    CK(j->split_wa[k - 1].upload(c, ps[k]->wa));
-                    CK(j->split_wb[k - 1].upload(c, ps[k]->wb));
+                    up(j->split_wa[k - 1], ps[k]->wa);
+                    up(j->split_wb[k - 1], ps[k]->wb);
                 }
                 if (narrow) {
-                    CK(j->split_na[k - 1].upload(c, ps[k]->na));
-                    CK(j->split_nb[k - 1].upload(c, ps[k]->nb));
+                    up(j->split_na[k - 1], ps[k]->na);
+                    up(j->split_nb[k - 1], ps[k]->nb);
                 }
             }
+            if (e != cudaSuccess) return no_split(e);
             j->split_wide = wide;
             j->split_narrow = narrow;
             memcpy(j->split_start, start, sizeof(uint32_t) * (S + 1));
         }
-        // start residues of the sub-ranges for s0 and s1, per class; where the
-        // budget has no room for them the walk stays plain
+        // start residues of the sub-ranges for s0 and s1, per class
         const size_t need32 = (size_t)2 * S * n32, need64 = (size_t)2 * S * n64;
         cudaError_t e = cudaSuccess;
-        if (n32 && j->split32.n < need32) e = j->split32.alloc(c, need32);
-        if (e == cudaSuccess && n64 && j->split64.n < need64) e = j->split64.alloc(c, need64);
-        if (e == cudaErrorMemoryAllocation) {
-            cudaGetLastError();
-            j->split32.release(c);
-            j->split64.release(c);
-            return PFC_OK;
-        }
-        CK(e);
+        if (n32 && j->split32.n < need32) e = j->split32.alloc(c, need32, true);
+        if (e == cudaSuccess && n64 && j->split64.n < need64) e = j->split64.alloc(c, need64, true);
+        if (e != cudaSuccess) return no_split(e);
         j->split_n = S;
         return PFC_OK;
     }
@@ -1336,6 +1380,8 @@ static int segment_body_graph(pfc_job *j) {
     k.setup_tc = c->setup_tc;
     k.walk_tc = 2 * c->walk_tc + (j->seg_lo >= kTcMinP) + 8 * (int)(j->seg_lo >> 62);
     for (int i = 0; i < 2; ++i) k.words[i] = j->words[i].p;
+    k.tct = j->tct.p;
+    k.tc_groups = j->tc_groups.p;
     if (j->split_n > 1) memcpy(k.split_start, j->split_start, sizeof(k.split_start));
     if (!j->graph || memcmp(&k, &j->gkey, sizeof(k)) != 0) {
         if (j->graph) cudaGraphExecDestroy(j->graph);
@@ -1560,16 +1606,17 @@ static uint64_t powmod_h(uint64_t a, uint64_t e, uint64_t p) {
 
 // Run a setup (`launch`, which returns the kernels it launched) on the single
 // candidate p and return its residues in plain form (s1: the combined search's
-// compositorial).
+// compositorial).  With `spare` its buffers are: the launch takes tiles, which
+// may not make room for them.
 template <class W, class Launch>
-static int setup_on_prime(pfc_job *j, uint64_t p, uint64_t &s0, uint64_t &s1, Launch launch) {
+static int setup_on_prime(pfc_job *j, uint64_t p, uint64_t &s0, uint64_t &s1, bool spare, Launch launch) {
     pfc_ctx *c = j->ctx;
     DevClass<W> cls;
     DArr<uint32_t> cnt;   // candidates, and the error flag of a tensor-core setup
     const W pw = (W)p;
     uint32_t one[2] = {1, 0};
-    cudaError_t e = cls.ensure(c, 1);
-    if (e == cudaSuccess) e = cnt.alloc(c, 2);
+    cudaError_t e = cls.ensure(c, 1, spare);
+    if (e == cudaSuccess) e = cnt.alloc(c, 2, spare);
     if (e == cudaSuccess) e = cudaMemcpyAsync(cls.p.p, &pw, sizeof(W), cudaMemcpyHostToDevice, c->st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(cnt.p, one, sizeof(one), cudaMemcpyHostToDevice, c->st);
     if (e == cudaSuccess) {
@@ -1623,21 +1670,16 @@ static int verify_tiles(pfc_job *j, const SlowProducts &sp) {
         const TcSetup s = tc_setup_args(j);
         uint64_t s0 = 0, s1 = 0;
         if (t == 0)
-            rc = setup_on_prime<uint32_t>(j, kVerifyPrime[t], s0, s1, [&](const ClassBuf<uint32_t> &v, uint32_t *err) {
+            rc = setup_on_prime<uint32_t>(j, kVerifyPrime[t], s0, s1, true, [&](const ClassBuf<uint32_t> &v, uint32_t *err) {
                 return launch_setup32_tc(v, s.a, s.ta, s.tb, err, c->st);
             });
         else
-            rc = setup_on_prime<uint64_t>(j, kVerifyPrime[t], s0, s1, [&](const ClassBuf<uint64_t> &v, uint32_t *err) {
+            rc = setup_on_prime<uint64_t>(j, kVerifyPrime[t], s0, s1, true, [&](const ClassBuf<uint64_t> &v, uint32_t *err) {
                 return launch_setup64_tc(v, s.a, s.ta, s.tb, t == 1, err, c->st);
             });
         if (!rc && !residues_match(j->mode, sp, t, s0, s1)) rc = PFC_ERR_VALIDATION;
     }
-    if (!packed) {   // the segments' buffers come first
-        j->tct.release(c);
-        j->tc_src.release(c);
-        j->tc_groups.release(c);
-        j->tc_packed = false;
-    }
+    if (!packed) release_tiles(j);   // the segments' buffers come first
     if (rc == PFC_ERR_NOMEM) {
         cudaGetLastError();
         rc = PFC_OK;
@@ -1656,7 +1698,7 @@ static int verify_programs(pfc_job *j, const SlowProducts &sp, uint64_t &bytes) 
         uint64_t s0 = 0, s1 = 0;
         if (t == 2) {
             const SetupArgs<uint64_t> s{j->mode, j->a64.view, j->b64.view, 0};
-            rc = setup_on_prime<uint64_t>(j, kVerifyPrime[t], s0, s1, [&](const ClassBuf<uint64_t> &v, uint32_t *) {
+            rc = setup_on_prime<uint64_t>(j, kVerifyPrime[t], s0, s1, false, [&](const ClassBuf<uint64_t> &v, uint32_t *) {
                 return launch_setup64(v, s, c->st);
             });
             bytes += (j->a64.words.n + j->b64.words.n) * 8;
@@ -1664,11 +1706,11 @@ static int verify_programs(pfc_job *j, const SlowProducts &sp, uint64_t &bytes) 
             const DevProg<WideWord> &a = t ? j->aw : j->a32, &b = t ? j->bw : j->b32;
             const SetupArgs<WideWord> s{j->mode, a.view, b.view, 0};
             if (t)
-                rc = setup_on_prime<uint64_t>(j, kVerifyPrime[t], s0, s1, [&](const ClassBuf<uint64_t> &v, uint32_t *) {
+                rc = setup_on_prime<uint64_t>(j, kVerifyPrime[t], s0, s1, false, [&](const ClassBuf<uint64_t> &v, uint32_t *) {
                     return launch_setup64w(v, s, c->st);
                 });
             else
-                rc = setup_on_prime<uint32_t>(j, kVerifyPrime[t], s0, s1, [&](const ClassBuf<uint32_t> &v, uint32_t *) {
+                rc = setup_on_prime<uint32_t>(j, kVerifyPrime[t], s0, s1, false, [&](const ClassBuf<uint32_t> &v, uint32_t *) {
                     return launch_setup32(v, s, c->st);
                 });
             bytes += (a.words.n + b.words.n) * sizeof(WideWord);

@@ -54,21 +54,30 @@ struct pfc_ctx {
     std::deque<std::pair<unsigned, uint32_t>> prog_order;
     size_t prog_bytes = 0;
     static constexpr size_t kProgCacheBytes = 64u << 20;
+    std::vector<pfc_job *> jobs;   // whose spare buffers reclaim_spare gives back
 };
 
 namespace pfc {
 
+// Gives back what the context's jobs hold but can do without: the word tables
+// of the tensor-core walk and the tiles of the tensor-core setup.
+void reclaim_spare(pfc_ctx *c);
+
 // A buffer of the context's pool, ordered on the context stream (work on
 // other streams must wait for that stream before using it; every caller
-// synchronises it first).  Counted against the memory budget while held.
-inline cudaError_t dalloc_bytes(pfc_ctx *c, void **p, size_t bytes) {
+// synchronises it first).  Counted against the memory budget while held.  A
+// `spare` one is one that its caller can do without: it takes what room there
+// is, where any other has the jobs' spare buffers given back to make room.
+inline cudaError_t dalloc_bytes(pfc_ctx *c, void **p, size_t bytes, bool spare = false) {
     *p = nullptr;
     if (bytes == 0) return cudaSuccess;
+    if (c->used + bytes > c->budget && !spare) reclaim_spare(c);
     if (c->used + bytes > c->budget) return cudaErrorMemoryAllocation;
     cudaError_t e = cudaMallocFromPoolAsync(p, bytes, c->pool, c->st);
     if (e == cudaErrorMemoryAllocation) {
         // give the pool's idle blocks back to the device and try once more
         cudaGetLastError();
+        if (!spare) reclaim_spare(c);
         e = cudaStreamSynchronize(c->st);
         if (e == cudaSuccess) e = cudaMemPoolTrimTo(c->pool, 0);
         if (e == cudaSuccess) e = cudaMallocFromPoolAsync(p, bytes, c->pool, c->st);
@@ -90,14 +99,14 @@ template <class T>
 struct DArr {
     T *p = nullptr;
     size_t n = 0;
-    cudaError_t alloc(pfc_ctx *c, size_t count) {
+    cudaError_t alloc(pfc_ctx *c, size_t count, bool spare = false) {
         release(c);
-        cudaError_t e = dalloc_bytes(c, (void **)&p, count * sizeof(T));
+        cudaError_t e = dalloc_bytes(c, (void **)&p, count * sizeof(T), spare);
         if (e == cudaSuccess) n = count;
         return e;
     }
-    cudaError_t upload(pfc_ctx *c, const std::vector<T> &v) {
-        cudaError_t e = alloc(c, std::max<size_t>(v.size(), 1));
+    cudaError_t upload(pfc_ctx *c, const std::vector<T> &v, bool spare = false) {
+        cudaError_t e = alloc(c, std::max<size_t>(v.size(), 1), spare);
         if (e != cudaSuccess) return e;
         if (v.empty()) return cudaMemsetAsync(p, 0, sizeof(T), c->st);
         c->h2d += v.size() * sizeof(T);
@@ -116,16 +125,16 @@ struct DevProg {
     DArr<uint32_t> groups;
     Prog<W> view{};
     // (extra: words behind the program's own, of its tensor-core form)
-    cudaError_t upload(pfc_ctx *c, const HostProg<W> &h, const std::vector<W> &extra = {}) {
+    cudaError_t upload(pfc_ctx *c, const HostProg<W> &h, const std::vector<W> &extra = {}, bool spare = false) {
         cudaError_t e;
         if (extra.empty()) {
-            e = words.upload(c, h.words);
+            e = words.upload(c, h.words, spare);
         } else {
             std::vector<W> all(h.words);
             all.insert(all.end(), extra.begin(), extra.end());
-            e = words.upload(c, all);
+            e = words.upload(c, all, spare);
         }
-        if (e == cudaSuccess) e = groups.upload(c, h.groups);
+        if (e == cudaSuccess) e = groups.upload(c, h.groups, spare);
         view.words = words.p;
         view.groups = groups.p;
         view.ngroups = (uint32_t)(h.groups.size() / 3);
@@ -144,14 +153,14 @@ struct DevClass {
     DArr<W> p, s0, s1;
     DArr<uint32_t> nnext;
     uint32_t cap = 0;
-    cudaError_t ensure(pfc_ctx *c, uint32_t want) {
+    cudaError_t ensure(pfc_ctx *c, uint32_t want, bool spare = false) {
         if (want <= cap && p.p) return cudaSuccess;
         release(c);
         const size_t n = std::max<uint32_t>(want, 256);
-        cudaError_t e = p.alloc(c, n);
-        if (e == cudaSuccess) e = s0.alloc(c, n);
-        if (e == cudaSuccess) e = s1.alloc(c, n);
-        if (e == cudaSuccess) e = nnext.alloc(c, n);
+        cudaError_t e = p.alloc(c, n, spare);
+        if (e == cudaSuccess) e = s0.alloc(c, n, spare);
+        if (e == cudaSuccess) e = s1.alloc(c, n, spare);
+        if (e == cudaSuccess) e = nnext.alloc(c, n, spare);
         if (e == cudaSuccess) cap = (uint32_t)n;
         return e;
     }
