@@ -855,6 +855,13 @@ int admit_prepared(pfc_batch *b) {
         int rc = upload_job(b, j);
         const bool alone = b->running.empty() && b->ready.empty() && fresh.empty();
         if (rc == PFC_ERR_NOMEM && !alone) break;  // waits for running searches to free memory
+        if (rc == PFC_ERR_NOMEM) {   // once more in the room of earlier iterations' window records
+            for (auto &row : b->tcw)
+                for (auto &g : row) g.release(c);
+            for (auto &row : b->wins)
+                for (auto &d : row) d.release(c);
+            rc = upload_job(b, j);
+        }
         if (rc == PFC_ERR_NOMEM && j->tc && !j->no_tc) {   // once more without the tensor-core setup's tiles
             free_tables(j);
             j->no_tc = true;
@@ -1054,10 +1061,10 @@ static bool plan_tc_walk(pfc_batch *b, int l, int shape, const std::vector<Batch
     const size_t nw = g.plan.size();
     cudaError_t e = cudaSuccess;
     auto room = [&](auto &arr, size_t n) {
-        if (e == cudaSuccess && arr.n < n) e = arr.alloc(c, n + n / 4);
+        if (e == cudaSuccess && arr.n < n) e = arr.alloc(c, n + n / 4, true);
     };
     if (tables > c->budget / 16) return false;
-    if (g.tables.n < tables) e = g.tables.alloc(c, tables);
+    if (g.tables.n < tables) e = g.tables.alloc(c, tables, true);
     room(g.digits, 2 * nw);
     room(g.d_words, 2 * nw * npass);
     if (l == 0) room(g.d_w32, nw * npass);
@@ -1125,6 +1132,17 @@ static bool plan_tc_walk(pfc_batch *b, int l, int shape, const std::vector<Batch
         g.fin.push_back(w);
     }
     return true;
+}
+
+// device room for the records of the iteration's windows
+static cudaError_t window_room(pfc_batch *b) {
+    cudaError_t e = cudaSuccess;
+    for (int l = 0; l < pfc_batch::kLists; ++l)
+        for (int k = 0; k < pfc_batch::kKinds; ++k) {
+            const size_t n = b->w[l][k].size();
+            if (e == cudaSuccess && b->wins[l][k].n < n) e = b->wins[l][k].alloc(b->ctx, n + n / 2 + 64);
+        }
+    return e;
 }
 
 // One window per search and class.  Throughput policy: every search advances
@@ -1254,26 +1272,40 @@ uint32_t build_tasks(pfc_batch *b) {
                 lists[l][kind].push_back({cost, w});
         }
     }
+    auto per_step = [&](int l, int shape) {   // no room for the tables: per-step windows
+        auto &g = b->tcw[l][shape];
+        lists[l][kWalkTask].insert(lists[l][kWalkTask].end(), g.plan.begin(), g.plan.end());
+        g.plan.clear();
+    };
     for (int l = 0; l < pfc_batch::kLists; ++l)
         for (int shape = 0; shape < 2; ++shape)
-            if (!plan_tc_walk(b, l, shape, by_slot)) {   // no room for tables: per-step
-                auto &g = b->tcw[l][shape];
-                lists[l][kWalkTask].insert(lists[l][kWalkTask].end(), g.plan.begin(), g.plan.end());
-                g.plan.clear();
+            if (!plan_tc_walk(b, l, shape, by_slot)) per_step(l, shape);
+    auto lay_out = [&]() {
+        for (int l = 0; l < pfc_batch::kLists; ++l)
+            for (int k = 0; k < pfc_batch::kKinds; ++k) {
+                auto &lst = lists[l][k];
+                std::sort(lst.begin(), lst.end(), [](const auto &x, const auto &y) { return x.first > y.first; });
+                b->w[l][k].clear();
+                uint64_t first = 0;
+                for (auto &e : lst) {
+                    e.second.first_cta = (uint32_t)first;
+                    first += e.second.nblocks;
+                    b->w[l][k].push_back(e.second);
+                }
+                b->ctas[l][k] = first;
             }
-    for (int l = 0; l < pfc_batch::kLists; ++l)
-        for (int k = 0; k < pfc_batch::kKinds; ++k) {
-            auto &lst = lists[l][k];
-            std::sort(lst.begin(), lst.end(), [](const auto &x, const auto &y) { return x.first > y.first; });
-            b->w[l][k].clear();
-            uint64_t first = 0;
-            for (auto &e : lst) {
-                e.second.first_cta = (uint32_t)first;
-                first += e.second.nblocks;
-                b->w[l][k].push_back(e.second);
+    };
+    lay_out();
+    if (window_room(b) == cudaErrorMemoryAllocation) {   // the windows' records come before the tables
+        cudaGetLastError();
+        for (int l = 0; l < pfc_batch::kLists; ++l)
+            for (int shape = 0; shape < 2; ++shape) {
+                per_step(l, shape);
+                plan_tc_walk(b, l, shape, by_slot);   // (of no windows)
+                b->tcw[l][shape].release(b->ctx);
             }
-            b->ctas[l][k] = first;
-        }
+        lay_out();
+    }
     return L;
 }
 
@@ -1320,11 +1352,11 @@ bool tc_chunks_pending(const pfc_batch *b) {
 
 int launch_iteration(pfc_batch *b) {
     pfc_ctx *c = b->ctx;
+    CK(window_room(b));
     for (int l = 0; l < pfc_batch::kLists; ++l)
         for (int k = 0; k < pfc_batch::kKinds; ++k) {
             const size_t n = b->w[l][k].size();
             if (!n) continue;
-            if (b->wins[l][k].n < n) CK(b->wins[l][k].alloc(c, n + n / 2 + 64));
             CK(cudaMemcpyAsync(b->wins[l][k].p, b->w[l][k].data(), n * sizeof(Window), cudaMemcpyHostToDevice, c->st));
             c->h2d += n * sizeof(Window);
         }

@@ -80,3 +80,41 @@ def test_words_and_tiles_make_room():
     at = least(both)
     for k in STEPS:
         assert both(at + k) == want, k
+
+
+def batch(searches, budget):
+    """One search after another through one batch: each is alone in it."""
+    with pfc.Context(0, budget=budget) as c:
+        c.set_walk_tc(2)
+        with pfc.Batch(c) as b:
+            out = []
+            for s in searches:
+                i = b.submit(*s)
+                b.run()
+                st = b.status(i)
+                if st.status:
+                    raise pfc.PFCError(st.status, "batch")
+                out.append((st.term_checksum, st.primecount, o.sort_factors(b.hits(i)).tobytes()))
+            return out, c.walk_counts()[0], c.launches
+
+
+@pytest.mark.parametrize("search", SEARCHES[:3])
+def test_every_budget_of_a_batch(search):
+    want, most, _ = batch([search], 0)
+    at = least(lambda b: batch([search], b))
+    routes = set()
+    for k in [256 * i for i in range(600)] + STEPS:
+        got, tc, launches = batch([search], at + k)
+        assert got == want, k
+        routes.add((tc, launches))
+    tcs = {tc for tc, _ in routes}
+    assert {0, most} <= tcs, "both walks"
+    assert len({n for tc, n in routes if tc == most}) > 1, "no budget left the tiles out"
+
+
+@pytest.mark.parametrize("search", SEARCHES[:3])
+def test_a_batch_gives_its_window_records_back(search):
+    """The least budget of a search alone is enough for it after another one as well."""
+    small = (1, 101, 9000, 10**9, 10**9 + 20000)
+    want = batch([small, search], 0)[0]
+    assert batch([small, search], least(lambda b: batch([search], b)))[0] == want
