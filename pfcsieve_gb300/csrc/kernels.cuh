@@ -169,10 +169,11 @@ constexpr uint64_t kTcMinWords32 = 240;
 constexpr uint64_t kTcMinWords64 = 216;
 // From 2^64/3 on, where the integer pipe takes 64-bit words: at 78 words 0.213 /
 // 0.255 ms, at 145 0.394 / 0.257, at 2,265 6.52 / 0.58; over a 3e7-wide range
-// at 78 words 1.14 / 1.83, at 145 2.16 / 1.84.  Programs for n below
-// kTcMinStartTop do not reach that size.
+// at 78 words 1.14 / 1.83, at 145 2.16 / 1.84.  Programs for n up to
+// kTcMinStartTop do not reach that size (the combined search's do first, from
+// nmin 33,504 on).
 constexpr uint64_t kTcMinWordsTop = 112;
-constexpr uint32_t kTcMinStartTop = 40000;
+constexpr uint32_t kTcMinStartTop = 33000;
 int launch_setup32_tc(const ClassBuf<uint32_t> &c, const SetupArgs<WideWord> &a, const TcTiles &ta,
                       const TcTiles &tb, uint32_t *err, cudaStream_t st, uint32_t block0 = 0, uint32_t nblocks = 0);
 // start residues of a split walk: sub-range k's into s0/s1 + k * c.cap
