@@ -609,15 +609,8 @@ static int launch_tc(const ClassBuf<typename TcClass<T>::W> &c, const SetupArgs<
     const uint32_t all = (c.cap + kCands - 1) / kCands;
     if (block0 >= all) return 0;
     if (nblocks == 0 || nblocks > all - block0) nblocks = all - block0;
-    static bool configured[64] = {false};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-    if (!configured[dev]) {
-        if (cudaFuncSetAttribute(setup_tc_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)TcLayout<T>::kSmemBytes) != cudaSuccess)
-            return 0;
-        configured[dev] = true;
-    }
+    static std::atomic<bool> configured[64];
+    if (!configure(setup_tc_kernel<T>, TcLayout<T>::kSmemBytes, configured)) return 0;
     setup_tc_kernel<T><<<nblocks, kTcThreads, TcLayout<T>::kSmemBytes, st>>>(c, a, ta, tb, flags, block0, 256u);
     return 1;
 }

@@ -5,6 +5,7 @@
 // One thread owns one candidate prime p (two in class-32 single-chain walks)
 // for a launch; its residues live in registers between the loads at launch
 // start and the stores at launch end.
+#include <atomic>
 #include <type_traits>
 
 #include "walk.cuh"
@@ -297,7 +298,7 @@ int walk_variant_shape(int cls, bool fused, int variant, int *nc, int *b) {
 
 // SM count of the current device (cached per device)
 static int device_sms() {
-    static int cached[64] = {0};
+    static std::atomic<int> cached[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 152;
     if (!cached[dev]) {

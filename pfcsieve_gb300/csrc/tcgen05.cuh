@@ -2,10 +2,23 @@
 // shared-memory descriptors, bounded mbarrier waits, bulk copies, MMAs and TMEM
 // access of tcgen05, all for one CTA.
 #pragma once
+#include <atomic>
 #include <cstdint>
 
 namespace pfc {
 namespace {
+
+// raises a kernel's dynamic shared memory once per device (host threads with
+// contexts of their own may do so at once)
+template <class Kernel>
+bool configure(Kernel kernel, uint32_t smem, std::atomic<bool> (&configured)[64]) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    if (!configured[dev] &&
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        return false;
+    return configured[dev] = true;
+}
 
 constexpr uint32_t kWaitLimit = 1u << 20;      // mbarrier polls before giving up
 

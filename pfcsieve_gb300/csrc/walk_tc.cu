@@ -1207,17 +1207,6 @@ int launch_walk_words_many(const WalkWordsWin *wins, uint32_t n, uint32_t ctas, 
     return 1;
 }
 
-// raises a kernel's dynamic shared memory once per device
-template <class Kernel>
-static bool configure(Kernel kernel, uint32_t smem, bool (&configured)[64]) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-    if (!configured[dev] &&
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return false;
-    return configured[dev] = true;
-}
-
 void walk_tc_args(WalkTcArgs &a, uint32_t top, uint32_t lo, uint32_t hi, uint32_t base) {
     a.lo = a.lo1 = lo;
     a.hi = a.hi1 = hi;
@@ -1232,7 +1221,7 @@ template <class T, int K, int NS>
 static int launch_tc(const ClassBuf<typename T::W> &c, const WalkTcArgs &a, const HitBuf &h,
                      const SplitArgs<typename T::W> &sp, uint32_t *err, cudaStream_t st) {
     using L = Lay<T, K>;
-    static bool configured[64] = {false};
+    static std::atomic<bool> configured[64];
     if (!configure(walk_tc_kernel<T, K, NS>, L::kSmem, configured)) return 0;
     const dim3 grid((c.cap + kCands - 1) / kCands, sp.n);
     walk_tc_kernel<T, K, NS><<<grid, Role<T>::kThreads, L::kSmem, st>>>(c, a, h, sp, err);
@@ -1242,7 +1231,7 @@ static int launch_tc(const ClassBuf<typename T::W> &c, const WalkTcArgs &a, cons
 template <class T, int K>
 static int launch_many(const WalkTcWin<typename T::W> *wins, uint32_t n, uint32_t ctas, const HitBuf &h, cudaStream_t st) {
     using L = Lay<T, K>;
-    static bool configured[64] = {false};
+    static std::atomic<bool> configured[64];
     if (!n || !configure(walk_tc_many_kernel<T, K>, L::kSmem, configured)) return 0;
     walk_tc_many_kernel<T, K><<<ctas, Role<T>::kThreads, L::kSmem, st>>>(wins, n, h);
     return 1;
