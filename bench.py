@@ -31,7 +31,7 @@ pipe would be busy with the algorithm's own multiplies.
 
 Unless --no-mixed, the line also carries `batched`: a sample of the mixed
 workload (searches drawn by pfcsieve_gb300.serving.mixed_jobs, seed 0) run as
-one batch (pfc_batch_*) and one search at a time (pfc_job_run), with every
+one batch (pfc_batch_*) and one search at a time (Job.run), with every
 search's totals and hits compared between the two, and the same searches
 served by the request loop with Poisson arrivals (200 per second, seed 1):
 p50 and p99 latency from arrival to result, against the same arrivals served

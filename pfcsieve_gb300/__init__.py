@@ -308,7 +308,7 @@ class Job:
 
     def run(self, cap=1 << 20):
         """Whole p range; returns the raw hits (unsorted)."""
-        # pfc_job_run's loop with the hits drained per segment: a buffer of
+        # the loop of pfc_job_run, with the hits drained per segment: a buffer of
         # `cap` records, 16 MB, cost 160 us a call in page clearing, more than
         # half of a search of 8e6 pairs
         parts, total, lo = [], 0, self.pmin
@@ -321,7 +321,7 @@ class Job:
                 parts.append(h)
             lo = hi
         if total > cap:
-            raise PFCError(PFC_ERR_HIT_OVERFLOW, "pfc_job_run: %d hits do not fit %d; rerun with cap=%d"
+            raise PFCError(PFC_ERR_HIT_OVERFLOW, "Job.run: %d hits do not fit %d; rerun with cap=%d"
                            % (total, cap, total))
         return parts[0] if len(parts) == 1 else np.concatenate(parts) if parts else np.zeros(0, dtype=FACTOR_DTYPE)
 

@@ -9,7 +9,7 @@ pfc_batch on one GPU:
   uniform in [101, 1e7), p-range length log-uniform in [1e5, 1e8] from p0
   log-uniform in [1e8, 2^63].
 * run_batched() runs a list of searches as one batch; run_plain() runs them
-  one after the other, one search per launch sequence (pfc_job_run), as the
+  one after the other, one search per launch sequence (Job.run), as the
   reference would.
 * serve() is the request loop: searches arrive by a Poisson process, join the
   running batch at the next iteration (continuous batching: the engine admits
@@ -85,7 +85,7 @@ def run_batched(ctx, searches, iteration_work=None, keep_hits=True):
 
 
 def run_plain(ctx, searches, keep_hits=True):
-    """One search after the other through pfc_job_run.
+    """One search after the other through Job.run.
 
     Returns ({index: Outcome}, seconds, per-search service times, seconds
     spent building host tables in pfc_job_create)."""
