@@ -7,8 +7,10 @@
 Workload (default): the combined factorial + compositorial search (-! -c) over
 n in [101, 200000) and p in [10^9, 10^9 + 10^8): about 4.8e6 candidate primes
 x 199,899 n = 9.7e11 pairs per step.  Inputs are the scalar search bounds; the
-tables live in HBM from job creation on.  The walk kernels are chosen by the
-autotuner (pfc_autotune) first; the choice is in config.walk_variants.
+tables live in HBM from job creation on.  Which walk ran is asked of the
+library (pfc_ctx_walk_counts, config.walk); the per-step kernels' shapes are
+chosen by the autotuner (pfc_autotune) first, and config.walk_variants names
+them where those kernels ran.
 
 One step = candidate generation + setup + iterate over the whole n range +
 check + hit read-back, through the C ABI stage calls on the context stream.
@@ -20,14 +22,15 @@ user makes: table build and upload, all segments, hit drain, CPU
 re-verification of every hit, 2-PRP filter and checksum, timed on the host.
 
 The roofline object covers the iterate (walk) kernel, the dominant one.  The
-walk is bound by the integer multiply pipe: each step of a residue chain needs
-a fixed set of multiplies (class 32: two 32x32->64 multiplies and one
-multiply-low; class 64 below 2^64/3: four 32x32->64 multiplies and one
-multiply-low).  Each kind's throughput is measured in
-this run (pfc_bench_int_peak); `achieved` is the walk's steps per second x the
+tensor-core walk is bound by the CUDA cores' issue slots: `achieved` is its
+tests per second x the instructions that a test leaves to them (TC_TEST_OPS),
+`peak` the measured issue rate.  A per-step walk is bound by the integer
+multiply pipe: each step of a residue chain needs a fixed set of multiplies
+(class 32: two 32x32->64 multiplies and one multiply-low; class 64 below
+2^64/3: four and one), and `achieved` is the walk's steps per second x the
 IMAD-equivalent cost of a step (each multiply weighted by IMAD rate / its own
-rate), `peak` is the IMAD rate, so `frac` is the fraction of time the multiply
-pipe would be busy with the algorithm's own multiplies.
+rate), `peak` the IMAD rate.  All rates are measured in this run
+(pfc_bench_int_peak).
 
 Unless --no-mixed, the line also carries `batched`: a sample of the mixed
 workload (searches drawn by pfcsieve_gb300.serving.mixed_jobs, seed 0) run as
@@ -484,12 +487,6 @@ def step_recipe(cls32, lazy):
 TC_TEST_OPS = 2.5
 
 
-def walk_is_tc(nmin, nmax):
-    """Whether a walk of this length takes the tensor-core kernel at any number of candidates (class 32 needs
-    the longest, about 3,000 steps; kernels.cuh WalkTimes)."""
-    return nmax - nmin >= 4000
-
-
 def hit_order(f):
     """Hits sorted by (p, |n|, type, nc), for comparing two runs."""
     if len(f) == 0:
@@ -501,26 +498,35 @@ def hit_order(f):
 # integer-pipe setup when the tensor-core setup is on: kTcMinWords32 and
 # kTcMinWords64 of pfcsieve_gb300/csrc/kernels.cuh
 TC_MIN_WORDS = {32: 240, 64: 216}
+# and kTcMinWordsTop, class 64 from 2^64/3 on
+TC_MIN_WORDS_TOP = 112
 
 
-def mixed_roofline(jobs, outcomes, seconds, peaks, tc_s=0.0, setup_tc=True):
-    """Multiply-pipe roofline of a batched run: the algorithmic multiplies of
-    every search (per candidate: its setup program's table words and squarings
-    -- pfc_setup_program_size -- and its walk steps: n for !, composite n for
-    the compositorial, prime n for #, both for -! -c), weighted by the measured
-    issue rates (IMAD 1, IMAD.WIDE and IMAD.HI by their rates relative to
-    IMAD), over the batch's wall time inside pfc_batch_step (iterations and
-    the tensor-core setups of admitted searches overlap).  Per unit (see
+def mixed_roofline(jobs, outcomes, seconds, peaks, tc_s=0.0, setup_tc=True, tc_steps=None):
+    """Roofline of a batched run over its wall time inside pfc_batch_step
+    (iterations and the tensor-core setups of admitted searches overlap): the
+    work every search needs (per candidate: its setup program's table words and
+    squarings -- pfc_setup_program_size -- and its walk steps: n for !,
+    composite n for the compositorial, prime n for #, both for -! -c).  Without
+    `tc_steps` all of it counts as multiplies, weighted by the measured issue
+    rates (IMAD 1, IMAD.WIDE and IMAD.HI by their rates relative to IMAD),
+    against the IMAD peak.  `tc_steps`, the candidate-steps per class that the
+    batch says it walked on the tensor cores, count as their tests'
+    instructions against the measured issue rate instead, and the fraction is
+    the time both take at those rates over the wall time (the count as
+    multiplies alone then stands in `per_step_algorithm`, which is no fraction
+    of what ran).  Per unit (see
     arith.cuh, walk.cuh, setup_tc.cu): 896-bit word on the integer pipe
     36 IMAD.WIDE + 2 IMAD (class 32), 76 + 3 (class 64 below 2^64/3); with the
     tensor-core setup, which multiplies pairs of them into 1792-bit words, per
     896-bit word 1.5 + 1 (class 32: half a 32-bit reduction and half a
     Montgomery product) and 5 + 1.5 (class 64: half the one-round reduction and
-    half the two-round product), with the fold's 112 x 4 (class 32) or 112 x 8
-    (class 64) byte-plane multiply-adds per 896-bit word on the tensor pipe,
+    half the two-word product), with the fold's 112 x 4 (class 32) or 112 x 8
+    (class 64) digit multiply-adds per 896-bit word on the tensor pipe (what the
+    fold needs: a tile issues 240 per pair of words, and its idle lanes),
     reported apart against the measured dense bf16 peak (fp16 runs at the same
-    rate), for programs of at least TC_MIN_WORDS words (smaller ones keep the
-    integer-pipe setup); 64-bit
+    rate), for programs of at least TC_MIN_WORDS words (from 2^64/3 on
+    TC_MIN_WORDS_TOP; smaller ones keep the integer-pipe setup); 64-bit
     word and class-64 squaring 8 IMAD.WIDE + 2 IMAD; class-32 squaring
     IMAD.WIDE + IMAD + IMAD.HI; walk steps as step_recipe.  Restores,
     corrections and replays are overhead, as in the single-search roofline.
@@ -531,7 +537,9 @@ def mixed_roofline(jobs, outcomes, seconds, peaks, tc_s=0.0, setup_tc=True):
     h = peaks["imad"] / peaks["mul_hi"]
     lazy_end = 0x5555555555555556
     unit = {32: (36 * w + 2, w + 1 + h), 64: (76 * w + 3, 8 * w + 2), 65: (8 * w + 2, 8 * w + 2)}
-    tc_word = {32: 1.5 * w + 1, 64: 5 * w + 1.5}
+    tc_word = {32: 1.5 * w + 1, 64: 5 * w + 1.5, 65: 5 * w + 1.5}
+    tc_least = {**TC_MIN_WORDS, 65: TC_MIN_WORDS_TOP}
+    walks = {32: [0.0, 0.0], 64: [0.0, 0.0], 65: [0.0, 0.0]}   # steps of a class, cost of one
     tc_macs = 0.0
     top = max(s.nmax for s in jobs) + 1
     isp = np.ones(top, dtype=bool)
@@ -544,30 +552,50 @@ def mixed_roofline(jobs, outcomes, seconds, peaks, tc_s=0.0, setup_tc=True):
     for i, s in enumerate(jobs):
         cls = 32 if s.pmax <= 2**31 else (64 if s.pmax <= lazy_end else 65)
         crossing += int(s.pmin < 2**31 < s.pmax or s.pmin < lazy_end < s.pmax)
-        key = (s.mode, s.nmin, cls != 65)
-        if key not in sizes:
-            sizes[key] = pfc.setup_program_size(*key)
-        words, sq = sizes[key]
         n = s.nmax - s.nmin
+
+        def size(wide):
+            key = (s.mode, s.nmin, wide)
+            if key not in sizes:
+                sizes[key] = pfc.setup_program_size(*key)
+            return sizes[key]
+        words, sq = size(True)
+        tc = setup_tc and words >= tc_least[cls]
+        if cls == 65 and not tc:
+            words, sq = size(False)
         primes = int(pc[s.nmax] - pc[s.nmin])
         steps = {1: n, 2: primes, 4: n - primes, 5: 2 * n - primes}[s.mode]
         recipe = step_recipe(cls == 32, cls == 64)
         step = sum(k * peaks["imad"] / peaks[name] for name, k in recipe.items())
         cw, cs = unit[cls]
-        tc = setup_tc and cls in (32, 64) and words >= TC_MIN_WORDS[cls]
         if tc:
             cw = tc_word[cls]
-            tc_macs += outcomes[i].primecount * words * 112 * (8 if cls == 64 else 4)
+            tc_macs += outcomes[i].primecount * words * 112 * (4 if cls == 32 else 8)
+        walks[cls][0] += outcomes[i].primecount * steps
+        walks[cls][1] = step
         total += outcomes[i].primecount * (words * cw + sq * cs + steps * step)
     achieved = total / seconds
-    return {"bound": "int (multiply pipe)", "achieved": achieved / 1e12, "peak": peaks["imad"] / 1e12,
+    line = {"bound": "int (multiply pipe)", "achieved": achieved / 1e12, "peak": peaks["imad"] / 1e12,
             "unit": "Tops/s IMAD-equivalent (IMAD.WIDE, IMAD.HI weighted by measured rates)",
             "frac": achieved / peaks["imad"], "traffic": None,
-            "kernel": "batch_kernel, walk_tc_many_kernel and setup_tc_kernel (every class and kind of the batch, over its "
-                      "wall time; walks counted as the multiplies of the per-step kernels)",
+            "kernel": "batch_kernel and setup_tc_kernel (every class and kind of the batch, over its wall time)",
             "alg_ops": total, "seconds": seconds, "searches_crossing_a_class_boundary": crossing,
             "peak_source": "measured in this run (pfc_bench_int_peak, 32-bit IMAD chains)",
             "tensor_setup": tensor_line(2 * tc_macs, seconds)}
+    if tc_steps and sum(tc_steps):
+        line["per_step_algorithm"] = {k: line[k] for k in ("achieved", "peak", "unit", "frac")}
+        # (a search that crosses 2^31 walks in two classes and is counted in one)
+        on_tc = {c: min(t, walks[c][0]) for c, t in zip((32, 64, 65), tc_steps)}
+        tests = TC_TEST_OPS * sum(on_tc.values()) / peaks["iadd_xor"]
+        rest = (total - sum(on_tc[c] * walks[c][1] for c in on_tc)) / peaks["imad"]
+        line.update(bound="CUDA cores (issue slots of the tensor-core walk's tests, multiply pipe of the rest)",
+                    achieved=(tests + rest) / seconds, peak=1.0, frac=(tests + rest) / seconds,
+                    unit="seconds of needed instructions at the measured rates per second",
+                    kernel="walk_tc_many_kernel, batch_kernel and setup_tc_kernel (every class and kind of the batch, "
+                           "over its wall time)",
+                    walk_steps_on_tensor_cores=sum(on_tc.values()) / max(sum(v[0] for v in walks.values()), 1.0),
+                    peak_source="measured in this run (pfc_bench_int_peak, IMAD and add/xor chains)")
+    return line
 
 
 def tensor_line(flops, seconds):
@@ -617,7 +645,7 @@ def run_mixed(ctx, njobs, warmup, steps=1, iteration_work=None, peaks=None):
                  for i in range(len(jobs)))
     lat_p = sv.fcfs_latencies(arrivals, service)
     roof = mixed_roofline(jobs, out_b, timing["step_s"], peaks, tc_s=timing["setup_tc_s"],
-                          setup_tc=ctx.setup_tc) if peaks else None
+                          setup_tc=ctx.setup_tc, tc_steps=timing["tc_walk_steps"]) if peaks else None
     return {
         "workload": "first %d of the 512 mixed searches (seed 0)" % len(jobs),
         "pairs": int(pairs),
@@ -713,7 +741,7 @@ def run_ours(args, wl, world, rank, local, dist):
         step()
     torch.cuda.synchronize()
     barrier(dist)
-    launches0 = ctx.launches
+    launches0, walks0 = ctx.launches, ctx.walk_counts()[0]
     pairs0 = job.pairs
     clk = ClockSampler(local)
     clk.start()
@@ -729,6 +757,7 @@ def run_ours(args, wl, world, rank, local, dist):
     ms = t0.elapsed_time(t1)
     it_ms = [a.elapsed_time(b) for a, b in evs]
     launches = ctx.launches - launches0
+    tc_walks = ctx.walk_counts()[0] - walks0
     pairs = job.pairs - pairs0
     ms_max = barrier_max(dist, ms)
     pairs_total = pairs * world
@@ -764,7 +793,7 @@ def run_ours(args, wl, world, rank, local, dist):
     per_step = {"achieved": achieved / 1e12, "frac": achieved / peak, "multiplies_per_walk_step": recipe,
                 "imad_equivalent_per_walk_step": imad_eq}
     tensor = None
-    if walk_is_tc(wl["nmin"], wl["nmax"]):
+    if tc_walks:
         depth = 48 if wl["nmax"] - 1 <= 202000 else 64
         flops = walk_steps * 4 * depth
         tensor = tensor_line(flops, it_s)
@@ -846,7 +875,9 @@ def run_ours(args, wl, world, rank, local, dist):
                        "pairs_per_step": int(pairs_total // args.steps),
                        "l2": "256 MB buffer overwritten before each step (candidate state < L2)",
                        "parallelism": "p-range shards, one per GPU" if world > 1 else "1 GPU",
-                       "device": name, "sms": sms, "walk_variants": tuned},
+                       "device": name, "sms": sms,
+                       "walk": "tensor cores, %d launches a step" % (tc_walks // args.steps) if tc_walks else "per step",
+                       "walk_variants": None if tc_walks else tuned},
             "roofline": {"bound": bound, "achieved": achieved / 1e12, "peak": peak / 1e12, "unit": unit,
                          "frac": achieved / peak, "traffic": traffic, "kernel": kernel, "tensor": tensor,
                          "walk_steps_per_step": int(walk_steps),

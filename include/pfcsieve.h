@@ -389,6 +389,11 @@ int pfc_batch_take_hits(pfc_batch *b, uint64_t id, pfc_factor *buf, size_t cap, 
 int pfc_batch_release(pfc_batch *b, uint64_t id);
 /* Iterations run so far. */
 uint64_t pfc_batch_iterations(pfc_batch *b);
+
+/* Candidate-steps that the batch has walked on the tensor cores so far, of
+ * class 32, class 64 below 2^64/3 and the rest (a step of the combined search
+ * counts for both chains). */
+int pfc_batch_tc_walk_steps(pfc_batch *b, double steps[3]);
 /* Work of one iteration in candidate-steps (a class-64 candidate step counts
  * 3).  Default by policy: 1.6e12 for THROUGHPUT (about 0.6 s of GPU time:
  * every iteration ends with a tail, so long ones waste least), 5e10 for

@@ -117,6 +117,7 @@ def lib():
             "pfc_batch_take_hits": (ctypes.c_int, [vp, u64, vp, sz, P(sz)]),
             "pfc_batch_release": (ctypes.c_int, [vp, u64]),
             "pfc_batch_iterations": (u64, [vp]),
+            "pfc_batch_tc_walk_steps": (ctypes.c_int, [vp, P(ctypes.c_double)]),
             "pfc_batch_set_iteration_work": (ctypes.c_int, [vp, ctypes.c_double]),
             "pfc_batch_set_policy": (ctypes.c_int, [vp, ctypes.c_int]),
             "pfc_batch_set_hit_capacity": (ctypes.c_int, [vp, u32]),
@@ -424,6 +425,12 @@ class Batch:
     @property
     def iterations(self):
         return lib().pfc_batch_iterations(self.h)
+
+    def tc_walk_steps(self):
+        """Candidate-steps walked on the tensor cores so far, per size class (pfc_batch_tc_walk_steps)."""
+        steps = (ctypes.c_double * 3)()
+        _ck(lib().pfc_batch_tc_walk_steps(self.h, steps), "pfc_batch_tc_walk_steps")
+        return list(steps)
 
     def timing(self):
         t = BatchTimes()

@@ -657,6 +657,7 @@ struct pfc_batch {
     TcWalk tcw[kLists][2];
     uint64_t next_id = 1;
     double work_per_iter = 0;            // candidate-steps per iteration (class 64 weighs 3); 0: the policy's
+    double tc_steps[kLists] = {};        // candidate-steps walked on the tensor cores, per class group
     int policy = PFC_BATCH_THROUGHPUT;
     uint64_t iterations = 0;
     // timing: kernel spans (CUDA events) and host phases (wall clock)
@@ -1340,6 +1341,7 @@ static void launch_tc_walks(pfc_batch *b, int l, int shape, const JobDev<typenam
             g.d_fin.p, (uint32_t)g.fin.size(), jobs, h);
         b->ctx->launches++;
     }
+    for (const auto &e : g.plan) b->tc_steps[l] += e.first * e.second.ncand;   // (steps over all chains)
     b->used[si] = true;
 }
 
@@ -1766,6 +1768,12 @@ extern "C" int pfc_batch_release(pfc_batch *b, uint64_t id) {
     auto it = b->all.find(id);
     if (it == b->all.end() || it->second->state != kDone) return PFC_ERR_STATE;
     b->all.erase(it);
+    return PFC_OK;
+}
+
+extern "C" int pfc_batch_tc_walk_steps(pfc_batch *b, double steps[3]) {
+    if (!b || !steps) return PFC_ERR_ARG;
+    std::copy(b->tc_steps, b->tc_steps + pfc_batch::kLists, steps);
     return PFC_OK;
 }
 

@@ -81,7 +81,7 @@ def run_batched(ctx, searches, iteration_work=None, keep_hits=True):
                 raise PFCError(st.status, "batched search %d" % i)
             out[i] = Outcome(st.term_checksum, st.primecount, b.hits(jid) if keep_hits else None)
             b.release(jid)
-        return out, dt, b.timing()
+        return out, dt, dict(b.timing(), tc_walk_steps=b.tc_walk_steps())
 
 
 def run_plain(ctx, searches, keep_hits=True):
