@@ -99,8 +99,10 @@ int pfc_ctx_set_graphs(pfc_ctx *ctx, int on);
  * into up to 8 sub-ranges: the residue at each boundary b comes from a setup
  * program for (b-1)! (or (b-1)!/(b-1)#, or the primorial below the boundary's
  * prime), and one launch walks every (candidate, sub-range) pair.  Used only
- * when those programs cost under a sixth of the walk (a small nmin), in
- * pfc_segment and in a pfc_iterate call over the whole range.  No
+ * when those programs cost under a sixth of the walk (a small nmin; on the
+ * tensor-core walk when its modelled time is less) and the memory budget has
+ * room for them, in pfc_segment and in a pfc_iterate call over the whole
+ * range.  No
  * counterpart in the reference, which walks each prime's n range in order
  * (kernels/iterate.cl:59-198).  On by default; off (`on` = 0, or
  * PFCSIEVE_SPLIT=0 in the environment when the context is created) walks

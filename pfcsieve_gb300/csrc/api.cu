@@ -6,7 +6,8 @@
 //   class-64 candidates: p, s0, s1 (u64) and nnext (u32)   28 B / candidate
 //   hit list pfc_factor[hitcap] + 64-bit counter
 //   setup programs (896-bit words for class 32 and for class 64 below 2^64/3,
-//   u64 words above), prime flags of [nmin, nmax) (1 bit per n)
+//   u64 words above, or 896-bit ones where the tensor cores set up), their
+//   tiles, the walk's word tables, prime flags of [nmin, nmax) (1 bit per n)
 //   or the prime list of [nmin, nmax) for the primorial walk
 //   per-segment accumulators: counts[2], termsum, flags
 //
@@ -39,7 +40,7 @@ struct pfc_job {
 
     DevProg<WideWord> a32, b32;   // class 32 (896-bit words)
     DevProg<uint64_t> a64, b64;   // class 64 at or above 2^64/3 (64-bit words)
-    DevProg<WideWord> aw, bw;     // class 64 below 2^64/3 (896-bit words)
+    DevProg<WideWord> aw, bw;     // class 64 below 2^64/3, and above on the tensor cores (896-bit words)
     // the tensor-core setup: aw, bw in their paired form (TcProg), packed into
     // fp16 tiles on first use
     TcProg tcp[2];
@@ -672,7 +673,7 @@ static int tc_prepare(pfc_job *j) {
     CK(j->tct.alloc(c, std::max<size_t>((na + nb) * tb, 16), true));
     CK(j->tc_src.upload(c, src, true));
     CK(j->tc_groups.upload(c, groups, true));
-    // the words: the lazy class-64 copy of the programs, or the class-32 one (the same programs)
+    // the words: the class-64 copy of the programs, or the class-32 one (the same programs)
     const bool w64 = j->aw.view.ngroups || j->bw.view.ngroups;
     const WideWord *wa = w64 ? j->aw.words.p : j->a32.words.p, *wb = w64 ? j->bw.words.p : j->b32.words.p;
     c->launches += launch_tc_pack(wa, j->tc_src.p, (uint32_t)pa.src.size(), (uint32_t)na, j->tct.p, c->st);
@@ -1075,9 +1076,11 @@ static int split_prepare(pfc_job *j) {
     const uint64_t chains = (n32 + n64) * (fused ? 2 : 1);
     const uint64_t target = (uint64_t)c->sms * 3 * 256 * 2 * 2;   // two waves of CTAs, two chains a thread
     uint32_t S = (uint32_t)std::min<uint64_t>({(uint64_t)kMaxSplit, target / chains, len / kMinSplitLen});
-    // From 2^64/3 up to a wave of candidates splits wherever the per-step walk
-    // would (13,500 candidates x 19,900 n: 0.27 ms split, 0.22 plain, since
-    // the boundaries' programs there take 64-bit words).
+    // From 2^64/3 on, sets of up to a wave of candidates keep the per-step
+    // walk's plan, which the model would leave: the walk of 13,460 candidates x
+    // 19,900 n takes 0.245 ms split and 0.201 plain (per step 0.765 and 1.188).
+    // Kept because it is the one split whose boundaries' programs are 64-bit
+    // words, which the tests of split walks run.
     const bool keep = tc && narrow && S > 1 && held(n64) <= 128.0 * c->sms;
     if (tc) {
         // by the model, with a program for b estimated at the 2 b bits of b!'s
@@ -1287,7 +1290,7 @@ static int commit_segment(pfc_job *j) {
     if (s.counts[0] > j->c32.cap && j->c32.p.p) return PFC_ERR_CAND_OVERFLOW;
     if (s.counts[1] > j->c64.cap && j->c64.p.p) return PFC_ERR_CAND_OVERFLOW;
     if ((!j->c32.p.p && s.counts[0]) || (!j->c64.p.p && s.counts[1])) return PFC_ERR_CAND_OVERFLOW;
-    if (s.tc_err) return PFC_ERR_CUDA;   // a tensor-core setup wait gave up
+    if (s.tc_err) return PFC_ERR_CUDA;   // a tensor-core setup's or walk's wait gave up
     if (s.flags & 1u) return PFC_ERR_VALIDATION;
     j->termsum += s.termsum;
     j->primecount += (uint64_t)s.counts[0] + s.counts[1];

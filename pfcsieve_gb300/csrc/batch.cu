@@ -392,13 +392,13 @@ struct BatchJob {
     std::vector<WideWord> words32;     // class 32
     std::vector<uint32_t> cmult, qlist;
     std::vector<uint64_t> words64;   // class 64 at or above 2^64/3
-    std::vector<WideWord> wordsw;      // class 64 below 2^64/3
+    std::vector<WideWord> wordsw;      // class 64 below 2^64/3, or from there on set up on the tensor cores (tc_top)
     std::vector<SetupSeg> segs32, segs64;
     uint32_t nsetup32 = 0, nsetup64 = 0;
-    // class 32 and class 64 below 2^64/3 on the tensor cores: the wide
-    // programs' groups (first program's, then the second's) and their shapes
+    // setups on the tensor cores: the wide programs' groups (first program's,
+    // then the second's) and their shapes
     bool tc = false;
-    // per size class (0: class 32, 1: class 64 below 2^64/3)
+    // per size class (0: class 32, 1: class 64)
     bool tc_wait[2] = {false, false};    // its setup is still running (no window of the class yet)
     cudaEvent_t tc_ev0[2] = {}, tc_ev1[2] = {};   // around that setup (throughput policy)
     uint32_t tc_block[2] = {0, 0}, tc_blocks[2] = {0, 0};   // latency policy: next candidate block, blocks
@@ -922,7 +922,7 @@ int admit_prepared(pfc_batch *b) {
         c->h2d += sizeof(v32[f]) + sizeof(v64[f]);
     }
     CK(cudaStreamSynchronize(c->st));
-    // setups of class 32 and of class 64 below 2^64/3 on the tensor cores.
+    // setups on the tensor cores.
     // The search's timeline of the class starts at its walk, which joins the
     // iterations once the setup has finished (build_tasks).  Throughput
     // policy: one setup launch per fresh search and class on the setup

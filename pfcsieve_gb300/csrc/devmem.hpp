@@ -36,7 +36,7 @@ struct pfc_ctx {
     bool graphs = true;   // pfc_segment replays each job's segment body as a CUDA graph
     bool split = true;    // small candidate sets walk their n range in sub-ranges (split walks)
     int walk_tc = 1;      // walks test their steps on the tensor cores (1: where that pays, 2: wherever it can)
-    bool setup_tc = true; // lazy class-64 setup folds its table words on the tensor cores
+    bool setup_tc = true; // setups fold their table words on the tensor cores (programs of kTcMinWords* and more)
     // prime flags of [0, vbits_top] kept for pfc_verify_factors_device (one
     // bit per integer), rebuilt only when a call needs a larger range
     uint32_t *vbits = nullptr;
@@ -187,7 +187,7 @@ struct DevClass {
 struct SegStats {
     uint32_t counts[2];
     uint32_t flags;
-    uint32_t tc_err;     // set by the tensor-core setup when a wait gave up
+    uint32_t tc_err;     // set by a tensor-core setup (2) or walk (4) when a wait gave up
     unsigned long long termsum;
     unsigned long long hits;
 };

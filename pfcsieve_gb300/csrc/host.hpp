@@ -6,10 +6,11 @@
 
 namespace pfc {
 
-// 896-bit setup table word (class 64 below 2^64/3): a product of primes as
-// 32 little-endian limbs of 28 bits (each limb in the low bits of a u32),
-// read on the device with eight 16-byte loads.  The 28-bit radix lets the
-// device sum limb x residue products in 64-bit accumulators without carries.
+// 896-bit setup table word (class 32, class 64 below 2^64/3, every class on the
+// tensor cores): a product of primes as 32 little-endian limbs of 28 bits
+// (each limb in the low bits of a u32), read on the device with eight 16-byte
+// loads.  The 28-bit radix lets the device sum limb x residue products in
+// 64-bit accumulators without carries.
 constexpr int kWideLimbs = 32;
 constexpr int kWideRadixBits = 28;
 struct alignas(16) WideWord {

@@ -133,14 +133,15 @@ int launch_setup32(const ClassBuf<uint32_t> &c, const SetupArgs<WideWord> &a, cu
 int launch_setup64(const ClassBuf<uint64_t> &c, const SetupArgs<uint64_t> &a, cudaStream_t st);
 // class 64 below 2^64/3 with 896-bit table words
 int launch_setup64w(const ClassBuf<uint64_t> &c, const SetupArgs<WideWord> &a, cudaStream_t st);
-// the same with the table-word fold on the tensor cores (setup_tc.cu): each
-// program in its paired form (host.hpp TcProg: 1792-bit words, each the
-// product of one or two 896-bit words, src[i] = first word | pair << 31)
-// first packed once into fp16 byte tiles of tc_tile_words() words
-// (tc_tile_bytes() each; tile i holds paired words 128 i ..), then the setup
-// over those tiles with the paired programs' groups, final squarings and
-// corrections in `a`; a wait that gives up sets *err (the segment then fails
-// with PFC_ERR_CUDA)
+// The setup of any class with the table-word fold on the tensor cores
+// (setup_tc.cu): each program in its paired form (host.hpp TcProg: 1792-bit
+// words, each the product of one or two 896-bit words, merged first groups,
+// every group in lanes of its own through all tiles, kTcOne in lanes without a
+// word), packed into fp16 digit tiles of tc_tile_words() lanes (tc_tile_bytes()
+// each; src[128 t + l] is the word of lane l of tile t), then the setup over
+// those tiles with the paired programs' groups (of lanes), final squarings and
+// corrections in `a`; a wait that gives up sets bit 1 of *err (the segment then
+// fails with PFC_ERR_CUDA)
 struct TcTiles {
     const void *tiles;   // device, ntiles * tc_tile_bytes(), 16-byte aligned
     uint32_t ntiles;
@@ -149,13 +150,13 @@ size_t tc_tile_bytes();
 uint32_t tc_tile_words();
 int launch_tc_pack(const WideWord *words, const uint32_t *src, uint32_t nw, uint32_t ntiles, void *out,
                    cudaStream_t st);
-// (candidate blocks of 64: [block0, block0 + nblocks), nblocks 0 to the end)
+// class 64: candidate blocks of 32, [block0, block0 + nblocks), nblocks 0 to the
+// end (lazy: every candidate is below 2^64/3)
 uint32_t tc_setup_blocks(uint32_t cands);
-// (lazy: every candidate is below 2^64/3)
 int launch_setup64_tc(const ClassBuf<uint64_t> &c, const SetupArgs<WideWord> &a, const TcTiles &ta,
                       const TcTiles &tb, bool lazy, uint32_t *err, cudaStream_t st, uint32_t block0 = 0,
                       uint32_t nblocks = 0);
-// class 32 on the same tiles (the class-32 and lazy class-64 programs are the same)
+// class 32, blocks of 64, on the same tiles (the classes' 896-bit programs are the same)
 uint32_t tc_setup_blocks32(uint32_t cands);
 // Smallest programs (896-bit words, both programs of the search) set up on the
 // tensor cores: below them the kernel's fixed cost per CTA (the position

@@ -64,8 +64,9 @@
 // and packed minima).  Cycles per 32 candidates and step on an SM's quarter,
 // per-step kernels to this one: class 32 (4.8e5 candidates) 17.7 to 12.5 (words
 // of 47 digits), 19.6 to 13.4 (63); class 64 (1.2e5) 35.9 to 17.0 (63), 38.3 to
-// 17.9 (47), from 2^64/3 (3.0e5) 69.5 to 20.4.  At that rate about 70% of the
-// issue slots are used, the ALU 60% of the time, the tensor cores 30 to 36%.
+// 17.9 (47), from 2^64/3 (3.0e5) 69.5 to 20.4.  At that rate 66 to 68% of the
+// issue slots are used, the ALU 56 to 59% of the time, the fma-heavy pipe 43%
+// (class 32) and 58% (class 64), the tensor cores 32 and 40%.
 // (The testers' loop runs over whole units, unrolled, and a suspect's residue
 // is read only when there is one: a tile at a time took 13.4 cycles in class
 // 32, 11% more instructions.)  A CTA's fixed part, about 1,500 steps long, is planes
