@@ -185,9 +185,16 @@ extern "C" int pfc_ctx_create(int device, uint64_t mem_budget, pfc_ctx **out) {
     return PFC_OK;
 }
 
+static int job_release(pfc_job *j);
+
 extern "C" int pfc_ctx_destroy(pfc_ctx *c) {
     if (!c) return PFC_ERR_ARG;
     cudaSetDevice(c->device);
+    while (!c->jobs.empty()) {   // jobs that outlive the context keep nothing on it
+        pfc_job *j = c->jobs.back();
+        job_release(j);
+        j->ctx = nullptr;
+    }
     if (c->st) {
         dfree_bytes(c, c->d_pat, kPatEntries * sizeof(uint64_t));
         dfree_bytes(c, c->vbits, c->vbits_bytes);
@@ -591,7 +598,7 @@ extern "C" int pfc_job_submit(pfc_ctx *c, unsigned mode, uint32_t nmin, uint32_t
 
 extern "C" int pfc_job_destroy(pfc_job *j) {
     if (!j) return PFC_ERR_ARG;
-    job_release(j);
+    if (j->ctx) job_release(j);
     delete j;
     return PFC_OK;
 }
@@ -760,6 +767,7 @@ static int enqueue_setup(pfc_job *j) {
         const int rc = setup_prepare(j);
         if (rc) return rc;
     }
+    if (!j->tc_packed && (tc_setup_applies(j) || tc_setup32_applies(j))) return PFC_ERR_NOMEM;
     CK(cudaMemsetAsync(&j->stats.p->tc_err, 0, sizeof(uint32_t), c->st));   // of this segment's tensor-core kernels
     SetupArgs<WideWord> s32;
     s32.mode = j->mode;

@@ -118,3 +118,15 @@ def test_a_batch_gives_its_window_records_back(search):
     small = (1, 101, 9000, 10**9, 10**9 + 20000)
     want = batch([small, search], 0)[0]
     assert batch([small, search], least(lambda b: batch([search], b)))[0] == want
+
+
+def test_a_job_that_outlives_its_context():
+    """Closing the context gives its jobs' buffers back; the job is closed (or collected) after it."""
+    for _ in range(3):
+        c = pfc.Context(0)
+        jobs = [pfc.Job(c, *s) for s in (SEARCHES[4], SEARCHES[3])]
+        jobs[0].segment(*SEARCHES[4][3:])
+        c.close()
+        jobs[0].close()
+        del jobs
+    assert job(SEARCHES[4], 0)[0][0][1]
